@@ -127,21 +127,23 @@ def _lattices(case):
     return out
 
 
-def _generators():
-    """The Gell-Mann matrices over two, (8, 3, 3)."""
-    t = np.zeros((8, 3, 3), dtype=np.complex128)
-    for a, (i, j) in enumerate(((0, 1), (0, 2), (1, 2))):
-        re, im = ((0, 1), (3, 4), (5, 6))[a]
-        t[re, i, j] = t[re, j, i] = 0.5
-        t[im, i, j], t[im, j, i] = -0.5j, 0.5j
-    t[2] = np.diag([0.5, -0.5, 0.0])
-    t[7] = np.diag([1.0, 1.0, -2.0]) / (2.0 * math.sqrt(3.0))
-    return torch.from_numpy(t).to(DEV)
-
-
 def _herm(v):
-    """t^a v^a, (..., 3, 3)."""
-    return torch.einsum("...a,aij->...ij", v.to(torch.complex128), _generators())
+    """t^a v^a, (..., 3, 3), with the Gell-Mann matrices over two as t^a."""
+    c = 0.5 * v
+    s = c[..., 7] / math.sqrt(3.0)
+    z = torch.zeros_like(s)
+    a01, a02, a12 = (torch.complex(c[..., k], -c[..., k + 1]) for k in (0, 3, 5))
+    d = [torch.complex(x, z) for x in (c[..., 2] + s, s - c[..., 2], -2 * s)]
+    rows = ((d[0], a01, a02), (a01.conj(), d[1], a12), (a02.conj(), a12.conj(), d[2]))
+    return torch.stack([torch.stack(r, dim=-1) for r in rows], dim=-2)
+
+
+def _mul(*factors):
+    """The product of batches of 3x3 matrices, left to right."""
+    p = factors[0]
+    for f in factors[1:]:
+        p = sum(p[..., :, k, None] * f[..., None, k, :] for k in range(3))
+    return p
 
 
 def _expi(c, v):
@@ -154,7 +156,7 @@ def _expi(c, v):
     one = torch.eye(3, dtype=torch.complex128, device=DEV)
     x = one + q / terms
     for n in range(terms - 1, 0, -1):
-        x = one + (q @ x) / n
+        x = one + _mul(q, x) / n
     return x
 
 
@@ -360,7 +362,7 @@ def exact(case, seed):
                "gauss_profile": g2 / (N[0] * N[1]), "emt": _emt(f, a)}
         if case["precision"] == "fp32":
             u = _mat(f["U"][1:-1])
-            d = torch.linalg.matrix_norm(u @ u.mH - torch.eye(3, dtype=torch.complex128, device=DEV))
+            d = torch.linalg.matrix_norm(_mul(u, u.mH) - torch.eye(3, dtype=torch.complex128, device=DEV))
             out["unitarity"] = torch.stack([d.max(), (d.square().sum() / (3 * sites)).sqrt()])
         return out
     if kind == "gauge":
@@ -411,12 +413,16 @@ def _sum(p, q):
 
 def _retr(m):
     """Re tr(i t^a m), (..., 8)."""
-    return (1j * torch.einsum("aij,...ji->...a", _generators(), m)).real
+    off = [p for i, j in ((0, 1), (0, 2), (1, 2)) for p in (m[..., i, j].imag + m[..., j, i].imag,
+                                                            m[..., i, j].real - m[..., j, i].real)]
+    d = [m[..., i, i].imag for i in range(3)]
+    last = (d[0] + d[1] - 2 * d[2]) / math.sqrt(3.0)
+    return -0.5 * torch.stack(off[:2] + [d[0] - d[1]] + off[2:] + [last], dim=-1)
 
 
 def _rotate(v, e):
     """2 tr(t^a v (t.e) v^dagger)."""
-    return 2 * torch.einsum("aij,...ji->...a", _generators(), v @ _herm(e) @ v.mH).real
+    return 2 * (_retr(-1j * _mul(v, _herm(e), v.mH)))
 
 
 def _step(f, a):
@@ -436,10 +442,10 @@ def _step(f, a):
             if nu == mu:
                 continue
             m, n, b = _unit(mu), _unit(nu), _unit(nu, -1)
-            up = link(nu, m) @ link(mu, n).mH @ link(nu).mH
-            down = link(nu, _sum(m, b)).mH @ link(mu, b).mH @ link(nu, b)
+            up = _mul(link(nu, m), link(mu, n).mH, link(nu).mH)
+            down = _mul(link(nu, _sum(m, b)).mH, link(mu, b).mH, link(nu, b))
             staples = staples + (up + down) / a[nu] ** 2
-        e = f["E"][1:-1, ..., mu, :] - 2 * DT * a3 / a[mu] ** 2 * _retr(link(mu) @ staples)
+        e = f["E"][1:-1, ..., mu, :] - 2 * DT * a3 / a[mu] ** 2 * _retr(_mul(link(mu), staples))
         if mu == 2:
             e = e - DT / a[2] / math.sqrt(2.0) * (J["Jp"] - J["Jm"])[1:-1]
         E.append(e)
@@ -452,8 +458,8 @@ def _step(f, a):
     half, full = [], []
     for mu in range(3):
         x = _expi(-0.5 * DT * a[mu] ** 2 / a3, E[..., mu, :])
-        half.append(x @ link(mu))
-        full.append(x @ half[mu])
+        half.append(_mul(x, link(mu)))
+        full.append(_mul(x, half[mu]))
     cur = {}
     for k, sign in (("Jp", -1), ("Jm", 1)):
         s = stat[k + "Stat"]
@@ -470,8 +476,8 @@ def _energies(f, a):
     e = torch.stack([c[k] * f["E"][1:-1, ..., k, :].square().sum((1, 2, 3)) for k in range(3)], dim=-1)
     b = []
     for k, (i, j) in enumerate(((1, 2), (2, 0), (0, 1))):
-        p = _at(U[..., i, :, :]) @ _at(U[..., j, :, :], *_unit(i))
-        q = _at(U[..., j, :, :]) @ _at(U[..., i, :, :], *_unit(j))
+        p = _mul(_at(U[..., i, :, :]), _at(U[..., j, :, :], *_unit(i)))
+        q = _mul(_at(U[..., j, :, :]), _at(U[..., i, :, :], *_unit(j)))
         b.append(c[k] * 4 * (3 - (p * q.conj()).sum((-1, -2)).real).sum((1, 2)))
     return e, torch.stack(b, dim=-1)
 
@@ -510,10 +516,10 @@ def _emt(f, a):
         def u(axis, dm, dn):
             return _at(W[..., axis, :, :], *_sum(_unit(m, dm), _unit(n, dn)))
 
-        avg = 0.25 * (u(m, 0, 0) @ u(n, 1, 0) @ u(m, 0, 1).mH @ u(n, 0, 0).mH
-                      + u(n, 0, 0) @ u(m, -1, 1).mH @ u(n, -1, 0).mH @ u(m, -1, 0)
-                      + u(n, 0, -1).mH @ u(m, 0, -1) @ u(n, 1, -1) @ u(m, 0, 0).mH
-                      + u(m, -1, 0).mH @ u(n, -1, -1).mH @ u(m, -1, -1) @ u(n, 0, -1))
+        avg = 0.25 * (_mul(u(m, 0, 0), u(n, 1, 0), u(m, 0, 1).mH, u(n, 0, 0).mH)
+                      + _mul(u(n, 0, 0), u(m, -1, 1).mH, u(n, -1, 0).mH, u(m, -1, 0))
+                      + _mul(u(n, 0, -1).mH, u(m, 0, -1), u(n, 1, -1), u(m, 0, 0).mH)
+                      + _mul(u(m, -1, 0).mH, u(n, -1, -1).mH, u(m, -1, -1), u(n, 0, -1)))
         B.append(q[k] * 2 * _retr(avg))
         Bs.append(q[k] ** 2 * 4 * (3 - avg.diagonal(dim1=-2, dim2=-1).sum(-1).real))
     for mu in range(3):
@@ -539,7 +545,7 @@ def _old_links(f, a, precision):
     out = torch.empty_like(f["U"])
     for mu in range(3):
         x = _expi(0.5 * DT * a[mu] ** 2 / a3, f["E"][..., mu, :])
-        out[..., mu, :, :] = _mat(x @ _mat(f["U"][..., mu, :, :]))
+        out[..., mu, :, :] = _mat(_mul(x, _mat(f["U"][..., mu, :, :])))
     return out.to(torch.complex64).to(torch.complex128) if precision == "fp32" else out
 
 
@@ -562,7 +568,7 @@ def _coulomb(f, a, iters, project):
     weight = torch.where(p2 > 0, 1 / (volume * torch.where(p2 > 0, p2, 1.0)), 0.0 if project else 1.0)
 
     def transform():
-        return [_at(G) @ _at(U[..., mu, :, :]) @ _at(G, *_unit(mu)).mH for mu in range(3)]
+        return [_mul(_at(G), _at(U[..., mu, :, :]), _at(G, *_unit(mu)).mH) for mu in range(3)]
 
     rows = []
     for it in range(iters):
@@ -576,7 +582,7 @@ def _coulomb(f, a, iters, project):
         lf = w.diagonal(dim1=-2, dim2=-1).sum(-1).real
         upd = torch.fft.ifftn(weight * torch.fft.fftn(dev, dim=(0, 1, 2)), dim=(0, 1, 2), norm="forward").real
         x = _expi(-0.08, upd)
-        G[1:-1] = x.mH @ G[1:-1]
+        G[1:-1] = _mul(x.mH, G[1:-1])
         step = (3 - x.diagonal(dim1=-2, dim2=-1).sum(-1)).abs()
         bound = torch.tensor(6.0 * sum(c), dtype=torch.float64, device=DEV)
         rows.append(torch.stack([torch.full_like(bound, it), dev.abs().max(), (dev.square().sum() / (8 * volume)).sqrt(),
