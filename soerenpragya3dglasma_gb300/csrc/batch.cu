@@ -89,10 +89,11 @@ __global__ void __launch_bounds__(kThreads, Occupancy<T>::kLinksMinBlocks)
 template <typename T, typename I, int R, bool kStride>
 __global__ void __launch_bounds__(kThreads, PlaqOccupancy<T, T>::kMinBlocks)
     plaquette_batch_kernel(const __grid_constant__ EventTable<T> tab, const unsigned short* __restrict__ tile_ev) {
+  __shared__ __align__(8) int sh[kPlaqShared<T, T>];
   for (long long t = tab.t0 + blockIdx.x; t < tab.t1; t += gridDim.x) {
     const EventDesc<T>& d = tab.ev[tile_ev[t] - tab.ev0];
     const long long idx = (t - d.k1_begin) * kThreads + threadIdx.x;
-    if (idx < d.g.plane * (d.g.nz + 1)) plaquette_site<T, I, R, T>(d.g, d.f, d.C, d.ep, (I)idx);
+    if (idx < d.g.plane * (d.g.nz + 1)) plaquette_site<T, I, R, T>(d.g, d.f, d.C, d.ep, (I)idx, sh);
     if (!kStride) break;
   }
 }
@@ -228,6 +229,7 @@ int build_descriptors(glasma_batch* b, double dt) {
     e.ep.do_jstat = 1;
     e.ep.dry = 0;
     e.lp.cj = (T)(dt / h->g.a[2]);
+    set_gather_weights(h->g, dt, e.lp);
     e.lp.save_uold = 0;
     e.lp.do_j = 1;
     e.lp.do_second = 1;

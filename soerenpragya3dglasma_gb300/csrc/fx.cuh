@@ -1,0 +1,495 @@
+// fx.cuh -- SU(3) products of FP64 data on the integer pipe.
+//
+// GB300 runs 2 FP64 multiply-adds per clock and SM (measured 1.7-2.0), but 59 `mad.wide.s32` (32 x 32 + 64
+// bits), and the two pipes run side by side (measured: 8 mad.wide and one FP64 fma per iteration take the
+// fma's time alone).  Links are bounded by one, so a matrix product can run in 60-bit fixed point with
+// one exponent per matrix: three mad.wide per real multiply-add instead of one FP64 fma, about ten times the
+// rate, and an error of ~2^-58 of the matrices' size against FP64's ~2^-54.
+//
+// A number is q 2^(e-60), q a 64-bit integer kept in two halves, q = h 2^32 + 2 l with -2^30 <= l < 2^30, and
+// e the exponent of its matrix; |q| < 2^63, so a value may reach 8 2^e.  A product of two numbers is
+//   h h' 2^64 + (h l' + l h') 2^33   (l l' 2^2 dropped: < 2^-58 of 2^(e+e'))
+// summed in two 64-bit accumulators: six terms of |h h'| <= 2^58 and twelve of |h l'| <= 2^59 fit easily.
+// Sums of q are exact modulo 2^64, so an intermediate sum may wrap where the final one is in range.
+//
+// Links near the identity keep their relative accuracy: a link is held as A = U - 1 with the exponent of
+// its largest entry (link_near), and a product of links as w = ab - 1 = A + B + AB.  The plaquette's
+// anti-Hermitian part is then accurate to ~2^-57 of the links' departure from 1, as small as that may be,
+// where FP64's is to ~2^-53 of it.
+//
+// What the format cannot hold is found, not assumed away: a link entry above 1.03 (or not finite), a row of a
+// product of two links whose norm is not near one, and an accumulator out of range set Guard, and the caller
+// runs the FP64 arithmetic for that site instead.
+#pragma once
+
+#include "su3.cuh"
+
+namespace glasma {
+namespace fx {
+
+typedef long long ll;
+
+struct R {
+  int h, l;
+};
+struct C {
+  R re, im;
+};
+struct M {
+  C e[9];  // e[i + 3*j]
+};
+struct Acc {
+  ll hh, cr;
+};
+// extremes of what has to stay in range, in one comparison at the end
+struct Guard {
+  int hi, lo;
+  bool bad;
+};
+
+constexpr int kScale = 60;
+constexpr int kOneH = 1 << (kScale - 32);  // h of the value 1 at exponent 0
+
+__device__ __forceinline__ R split(ll q) {
+  const int lo = (int)q, hi = (int)(q >> 32);
+  R r;
+  r.h = hi - (lo >> 31);
+  r.l = lo >> 1;
+  return r;
+}
+__device__ __forceinline__ ll join(const R& r) { return ((ll)r.h << 32) + 2 * (ll)r.l; }
+
+__device__ __forceinline__ Acc acc_zero() {
+  Acc a;
+  a.hh = 0;
+  a.cr = 0;
+  return a;
+}
+// half a unit of the result, so that finish rounds
+__device__ __forceinline__ Acc acc_half() {
+  Acc a;
+  a.hh = 0;
+  a.cr = 1 << 26;
+  return a;
+}
+__device__ __forceinline__ void mad(Acc& s, const R& a, const R& b) {
+  s.hh += (ll)a.h * b.h;
+  s.cr += (ll)a.h * b.l;
+  s.cr += (ll)a.l * b.h;
+}
+__device__ __forceinline__ ll finish(const Acc& s) { return (s.hh << 4) + (s.cr >> 27); }
+__device__ __forceinline__ ll finish_diff(const Acc& p, const Acc& n) {
+  Acc s;
+  s.hh = p.hh - n.hh;
+  s.cr = p.cr - n.cr;
+  return finish(s);
+}
+// The accumulated value stays below 4: |hh| < 2^58, its high word below 2^26.
+__device__ __forceinline__ void watch(Guard& g, ll hh_re, ll hh_im) {
+  const int a = (int)(hh_re >> 32), b = (int)(hh_im >> 32);
+  g.hi = max(g.hi, max(a, b));
+  g.lo = min(g.lo, min(a, b));
+}
+__device__ __forceinline__ bool tripped(const Guard& g) { return g.bad || g.hi >= (1 << 26) || g.lo < -(1 << 26); }
+__device__ __forceinline__ Guard guard_init() {
+  Guard g;
+  g.hi = 0;
+  g.lo = 0;
+  g.bad = false;
+  return g;
+}
+
+// ---- doubles in and out -------------------------------------------------------------------------------
+// By integer operations on the bits: GB300's FP64 <-> 64-bit integer conversions run on the FP64 pipe, at the
+// rate of an fma (measured: with them the force kernel kept that pipe 67 % busy, two thirds of it converting).
+// shift(k): what the conversions take for a scale of 2^k
+__device__ __forceinline__ int shift(int k) { return 1083 - k; }
+// |v| 2^k, truncated; |v| 2^k < 2^62 (larger values give garbage, never a fault)
+__device__ __forceinline__ ll magnitude(double v, int sh) {
+  const int h = __double2hiint(v);
+  const unsigned long long m =
+      ((unsigned long long)((h & 0xfffff) | 0x100000) << 40) | ((unsigned long long)(unsigned)__double2loint(v) << 8);
+  ll q;
+  asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(sh - ((h >> 20) & 0x7ff)));  // clamps: zero beyond 63
+  return q;
+}
+__device__ __forceinline__ ll to_fixed(double v, int sh) {
+  const ll q = magnitude(v, sh), s = __double2hiint(v) >> 31;
+  return (q ^ s) - s;
+}
+__device__ __forceinline__ R to_fixed_split(double v, int sh) {
+  R r = split(magnitude(v, sh));
+  const int sg = (__double2hiint(v) >> 31) | 1;
+  r.h *= sg;
+  r.l *= sg;
+  return r;
+}
+// q 2^k, rounded to nearest (half up)
+__device__ __forceinline__ double from_fixed(ll q, int k) {
+  const ll s = q >> 63;
+  const unsigned long long m = (unsigned long long)((q ^ s) - s);
+  const int n = __clzll((ll)m);
+  const unsigned long long t = m << (n & 63);
+  const unsigned long long b = (t >> 11) + ((t >> 10) & 1) + ((unsigned long long)(unsigned)(1023 + 62 + k - n) << 52);
+  return m == 0 ? 0.0 : __longlong_as_double((ll)b | (q & (1LL << 63)));
+}
+// 2^k as a double, -1022 <= k <= 1023
+__device__ __forceinline__ double pow2(int k) { return __hiloint2double((k + 1023) << 20, 0); }
+constexpr int kMinExp = -400;  // smaller values are held at 2^-460
+// |v| < 2^exponent_of(largest |high word| of v)
+__device__ __forceinline__ int exponent_of(int habs) { return (habs >> 20) - 1022; }
+constexpr int kMaxEntryHi = 0x3FF07AE1;  // 1.03
+
+__device__ __forceinline__ int habs(double v) { return __double2hiint(v) & 0x7fffffff; }
+
+// A plain matrix with entries up to one (a link), exponent 0.
+template <typename I>
+__device__ __forceinline__ void link_plain(const cx<double>* __restrict__ U, I S, int mu, I s, M& m, Guard& g) {
+  const cx<double>* p = U + ((I)(mu * 9) * S + s);
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const cx<double> v = p[(I)k * S];
+    top = max(top, max(habs(v.re), habs(v.im)));
+    m.e[k].re = to_fixed_split(v.re, shift(kScale));
+    m.e[k].im = to_fixed_split(v.im, shift(kScale));
+  }
+  g.bad |= top > kMaxEntryHi;
+}
+
+// A = U - 1 with the exponent of its largest entry (at most 0).
+template <typename I>
+__device__ __forceinline__ void link_near(const cx<double>* __restrict__ U, I S, int mu, I s, M& m, int& e, Guard& g) {
+  const cx<double>* p = U + ((I)(mu * 9) * S + s);
+  cx<double> v[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) v[k] = p[(I)k * S];
+  int top = 0, topd = 0;
+  ll d[3], dor = 0;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    top = max(top, habs(v[k].im));
+    if (k % 4 == 0) {
+      topd = max(topd, habs(v[k].re));
+      const ll q = to_fixed(v[k].re, shift(kScale)) - (1LL << kScale);
+      d[k / 4] = q;
+      dor |= q ^ (q >> 63);
+    } else {
+      top = max(top, habs(v[k].re));
+    }
+  }
+  g.bad |= max(top, topd) > kMaxEntryHi;
+  const int ed = 64 - __clzll(dor) - kScale;  // |diagonal - 1| < 2^ed
+  int ee = max(max(exponent_of(top), ed), kMinExp);
+  ee = min(ee, 0);
+  e = ee;
+  const int kb = shift(kScale - ee);
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    m.e[k].im = to_fixed_split(v[k].im, kb);
+    m.e[k].re = k % 4 == 0 ? split(d[k / 4] << min(-ee, 63)) : to_fixed_split(v[k].re, kb);
+  }
+}
+
+// ---- products -------------------------------------------------------------------------------------------
+// (A B)_ij
+__device__ __forceinline__ void entry_nn(const M& A, int i, const M& B, int j, Acc& rr, Acc& ii, Acc& im) {
+  rr = im = acc_half();
+  ii = acc_zero();
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const C &a = A.e[i + 3 * k], &b = B.e[k + 3 * j];
+    mad(rr, a.re, b.re);
+    mad(ii, a.im, b.im);
+    mad(im, a.re, b.im);
+    mad(im, a.im, b.re);
+  }
+}
+
+// w = (1 + A)(1 + B) - 1, its exponent at most 0 and at least 3 above A's and B's (below the cap), so |w| < 2^e / 2
+// there; at the cap |w| <= 2.
+__device__ __forceinline__ void near_product(const M& A, int ea, const M& B, int eb, M& W, int& ew, Guard& g) {
+  ew = min(max(ea, eb) + 3, 0);
+  const int kk = min(ew - ea - eb, 63), ka = min(ew - ea, 63), kb = min(ew - eb, 63);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      Acc rr, ii, im;
+      entry_nn(A, i, B, j, rr, ii, im);
+      const C &a = A.e[i + 3 * j], &b = B.e[i + 3 * j];
+      W.e[i + 3 * j].re = split((finish_diff(rr, ii) >> kk) + (join(a.re) >> ka) + (join(b.re) >> kb));
+      W.e[i + 3 * j].im = split((finish(im) >> kk) + (join(a.im) >> ka) + (join(b.im) >> kb));
+    }
+  if (ew == 0) {  // entries near or above 1/8: the rows of 1 + w must have norm one (to 10 %)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      ll n = 0;
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const int x = W.e[i + 3 * j].re.h + (i == j ? kOneH : 0), y = W.e[i + 3 * j].im.h;
+        n += (ll)x * x + (ll)y * y;
+      }
+      const int t = (int)(n >> 32);  // 2^56 is one: 2^24 here
+      g.bad |= n < 0 || t < (int)(0.81 * (1 << 24)) || t > (int)(1.21 * (1 << 24));
+    }
+  }
+}
+
+// The anti-Hermitian part of a matrix P: y_ij = Im(P_ij + P_ji), x_ij = Re(P_ij - P_ji) for (ij) = 01, 02, 12 and
+// d_i = Im P_ii.  al = ReTr(i t P) is -1/2 of (y01, x01, d0 - d1, y02, x02, y12, x12, (d0 + d1 - 2 d2) / sqrt 3).
+struct Anti {
+  ll y[3], x[3], d[3];
+  int e;
+};
+// component k of -2 al 2^(60-e), the last without its 1/sqrt(3)
+__device__ __forceinline__ ll component(const Anti& p, int k) {
+  switch (k) {
+    case 0: return p.y[0];
+    case 1: return p.x[0];
+    case 2: return p.d[0] - p.d[1];
+    case 3: return p.y[1];
+    case 4: return p.x[1];
+    case 5: return p.y[2];
+    case 6: return p.x[2];
+    default: return p.d[0] + p.d[1] - 2 * p.d[2];
+  }
+}
+
+// P = (1 + w)(1 + v)^dagger of two near products
+__device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, int ev, Anti& o) {
+  const int ep = max(ew, ev);
+  const int k = min(ep - ew - ev, 63), kw = min(ep - ew, 63), kv = min(ep - ev, 63);
+  o.e = ep;
+  constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    const int i = pi[n], j = pj[n];
+    Acc yp = acc_half(), yn = acc_zero(), xp = acc_half(), xn = acc_zero();
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+      const C &wi = W.e[i + 3 * t], &wj = W.e[j + 3 * t], &vi = V.e[i + 3 * t], &vj = V.e[j + 3 * t];
+      mad(yp, wi.im, vj.re);
+      mad(yp, wj.im, vi.re);
+      mad(yn, wi.re, vj.im);
+      mad(yn, wj.re, vi.im);
+      mad(xp, wi.re, vj.re);
+      mad(xp, wi.im, vj.im);
+      mad(xn, wj.re, vi.re);
+      mad(xn, wj.im, vi.im);
+    }
+    const ll yw = join(W.e[i + 3 * j].im) + join(W.e[j + 3 * i].im), yv = join(V.e[i + 3 * j].im) + join(V.e[j + 3 * i].im);
+    const ll xw = join(W.e[i + 3 * j].re) - join(W.e[j + 3 * i].re), xv = join(V.e[j + 3 * i].re) - join(V.e[i + 3 * j].re);
+    o.y[n] = (finish_diff(yp, yn) >> k) + (yw >> kw) - (yv >> kv);
+    o.x[n] = (finish_diff(xp, xn) >> k) + (xw >> kw) + (xv >> kv);
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    Acc p = acc_half(), q = acc_zero();
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+      const C &w = W.e[i + 3 * t], &v = V.e[i + 3 * t];
+      mad(p, w.im, v.re);
+      mad(q, w.re, v.im);
+    }
+    o.d[i] = (finish_diff(p, q) >> k) + (join(W.e[4 * i].im) >> kw) - (join(V.e[4 * i].im) >> kv);
+  }
+}
+
+// M = H(p) + i H(q) with H_ij = y_ij - i x_ij, H_ji its conjugate (i < j), H_ii = 2 d_i: H(p) is -4 t.al up to a
+// multiple of 1, which a rotation leaves alone.  Exponent e; the two exponents may differ.
+__device__ __forceinline__ void herm_pair(const Anti& p, const Anti& q, M& m, int& e, ll& tr_re, ll& tr_im) {
+  const int em = max(p.e, q.e) + 1;
+  const int kp = min(em - p.e, 63), kq = min(em - q.e, 63);
+  e = em;
+  constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    const int i = pi[n], j = pj[n];
+    const ll y1 = p.y[n] >> kp, x1 = p.x[n] >> kp, y2 = q.y[n] >> kq, x2 = q.x[n] >> kq;
+    m.e[i + 3 * j].re = split(y1 + x2);
+    m.e[i + 3 * j].im = split(y2 - x1);
+    m.e[j + 3 * i].re = split(y1 - x2);
+    m.e[j + 3 * i].im = split(y2 + x1);
+  }
+  tr_re = tr_im = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const ll a = p.d[i] >> (kp - 1), b = q.d[i] >> (kq - 1);
+    m.e[4 * i].re = split(a);
+    m.e[4 * i].im = split(b);
+    tr_re += a;
+    tr_im += b;
+  }
+}
+
+// The Hermitian and anti-Hermitian parts of C = V^dagger M V (kInv) or V M V^dagger, as split_herm_pair gives them
+// (the last of each without its 1/sqrt(3)); V plain, in units of M.  tr: the trace of M (C_22 follows from it).
+template <bool kInv>
+__device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll tr_re, ll tr_im, ll (&o1)[8], ll (&o2)[8],
+                                            Guard& g) {
+  ll cr[9], ci[9];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    C t[3];  // row i of V^dagger M, or of V M
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      Acc a = acc_half(), b = acc_half(), c = acc_zero();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const C& m = Mm.e[k + 3 * j];
+        if constexpr (kInv) {  // conj(v) m
+          const C& v = V.e[k + 3 * i];
+          mad(a, v.re, m.re);
+          mad(a, v.im, m.im);
+          mad(b, v.re, m.im);
+          mad(c, v.im, m.re);
+        } else {  // v m
+          const C& v = V.e[i + 3 * k];
+          mad(b, v.re, m.re);
+          mad(c, v.im, m.im);
+          mad(a, v.re, m.im);
+          mad(a, v.im, m.re);
+        }
+      }
+      const ll dh = b.hh - c.hh;
+      watch(g, a.hh, dh);
+      const R sum = split(finish(a)), dif = split(finish_diff(b, c));
+      t[j].re = kInv ? sum : dif;
+      t[j].im = kInv ? dif : sum;
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      if (i == 2 && j == 2) continue;
+      Acc a = acc_half(), b = acc_half(), c = acc_zero();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if constexpr (kInv) {  // t v
+          const C& v = V.e[k + 3 * j];
+          mad(b, t[k].re, v.re);
+          mad(c, t[k].im, v.im);
+          mad(a, t[k].re, v.im);
+          mad(a, t[k].im, v.re);
+        } else {  // t conj(v)
+          const C& v = V.e[j + 3 * k];
+          mad(a, t[k].re, v.re);
+          mad(a, t[k].im, v.im);
+          mad(b, t[k].im, v.re);
+          mad(c, t[k].re, v.im);
+        }
+      }
+      watch(g, a.hh, b.hh - c.hh);
+      const ll sum = finish(a), dif = finish_diff(b, c);
+      cr[i + 3 * j] = kInv ? dif : sum;
+      ci[i + 3 * j] = kInv ? sum : dif;
+    }
+  }
+  o1[0] = cr[3] + cr[1];
+  o1[1] = ci[1] - ci[3];
+  o1[2] = cr[0] - cr[4];
+  o1[3] = cr[6] + cr[2];
+  o1[4] = ci[2] - ci[6];
+  o1[5] = cr[7] + cr[5];
+  o1[6] = ci[5] - ci[7];
+  o1[7] = 3 * (cr[0] + cr[4]) - 2 * tr_re;
+  o2[0] = ci[3] + ci[1];
+  o2[1] = cr[3] - cr[1];
+  o2[2] = ci[0] - ci[4];
+  o2[3] = ci[6] + ci[2];
+  o2[4] = cr[6] - cr[2];
+  o2[5] = ci[7] + ci[5];
+  o2[6] = cr[7] - cr[5];
+  o2[7] = 3 * (ci[0] + ci[4]) - 2 * tr_im;
+}
+
+// M = 2 (t.p + i t.q) from two FP64 algebra vectors, exponent two above their largest component's.
+__device__ __forceinline__ void herm_pair(const Alg<double>& p, const Alg<double>& q, M& m, int& e, ll& tr_re, ll& tr_im,
+                                          Guard& g) {
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) top = max(top, max(habs(p.a[k]), habs(q.a[k])));
+  g.bad |= top >= 0x43100000;  // 2^50 or more, or not finite
+  const int em = max(exponent_of(min(top, 0x43100000)), kMinExp) + 2;
+  e = em;
+  const int kb = shift(kScale - em);
+  const ll s1 = to_fixed(p.a[7] * Consts<double>::inv_sqrt3(), kb), s2 = to_fixed(q.a[7] * Consts<double>::inv_sqrt3(), kb);
+  constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2}, py[3] = {0, 3, 5};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    const int i = pi[n], j = pj[n];
+    const ll y1 = to_fixed(p.a[py[n]], kb), x1 = to_fixed(p.a[py[n] + 1], kb);
+    const ll y2 = to_fixed(q.a[py[n]], kb), x2 = to_fixed(q.a[py[n] + 1], kb);
+    m.e[i + 3 * j].re = split(y1 + x2);
+    m.e[i + 3 * j].im = split(y2 - x1);
+    m.e[j + 3 * i].re = split(y1 - x2);
+    m.e[j + 3 * i].im = split(y2 + x1);
+  }
+  const ll c1 = to_fixed(p.a[2], kb), c2 = to_fixed(q.a[2], kb);
+  m.e[0].re = split(c1 + s1);
+  m.e[0].im = split(c2 + s2);
+  m.e[4].re = split(s1 - c1);
+  m.e[4].im = split(s2 - c2);
+  m.e[8].re = split(-2 * s1);
+  m.e[8].im = split(-2 * s2);
+  tr_re = tr_im = 0;
+}
+
+// +-2^k o, the last component over sqrt 3
+__device__ __forceinline__ void to_alg(const ll (&o)[8], int k, double sign, Alg<double>& out) {
+#pragma unroll
+  for (int n = 0; n < 7; n++) out.a[n] = sign < 0 ? -from_fixed(o[n], k) : from_fixed(o[n], k);
+  out.a[7] = from_fixed(o[7], k) * (sign * Consts<double>::inv_sqrt3());
+}
+
+// Two adjoint actions by one plain matrix, as inv_adj_mul2 / adj_mul2: out_k = V^d (t.e_k) V or V (t.e_k) V^d.
+template <bool kInv>
+__device__ __forceinline__ void adj_pair(const M& V, const Alg<double>& e1, const Alg<double>& e2, Alg<double>& out1,
+                                         Alg<double>& out2, Guard& g) {
+  M m;
+  int e;
+  ll tr_re, tr_im, o1[8], o2[8];
+  herm_pair(e1, e2, m, e, tr_re, tr_im, g);
+  rotate_pair<kInv>(V, m, tr_re, tr_im, o1, o2, g);
+  to_alg(o1, e - kScale - 1, 1.0, out1);
+  to_alg(o2, e - kScale - 1, 1.0, out2);
+}
+
+
+// A matrix of doubles with the exponent of its largest entry; kLink: exponent 0 and entries up to one (1.03).
+template <bool kLink>
+__device__ __forceinline__ void from_mat(const Mat<double>& u, M& m, int& e, Guard& g) {
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 9; k++) top = max(top, max(habs(u.e[k].re), habs(u.e[k].im)));
+  g.bad |= kLink ? top > kMaxEntryHi : top >= 0x43100000;
+  e = kLink ? 0 : max(exponent_of(min(top, 0x43100000)), kMinExp);
+  const int kb = shift(kScale - e);
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    m.e[k].re = to_fixed_split(u.e[k].re, kb);
+    m.e[k].im = to_fixed_split(u.e[k].im, kb);
+  }
+}
+
+// out = u + A u for A = X - 1 (any size up to one) and a link u: the product in fixed point with A's exponent, the
+// sum in FP64, so the result is rounded once.  False where the format does not hold the operands.
+__device__ __forceinline__ bool add_product(const Mat<double>& A, const Mat<double>& u, Mat<double>& out) {
+  Guard g = guard_init();
+  M a, b;
+  int ea, eb;
+  from_mat<false>(A, a, ea, g);
+  from_mat<true>(u, b, eb, g);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      Acc rr, ii, im;
+      entry_nn(a, i, b, j, rr, ii, im);
+      out.e[i + 3 * j].re = u.e[i + 3 * j].re + from_fixed(finish_diff(rr, ii), ea - kScale);
+      out.e[i + 3 * j].im = u.e[i + 3 * j].im + from_fixed(finish(im), ea - kScale);
+    }
+  return !g.bad;
+}
+
+}  // namespace fx
+}  // namespace glasma

@@ -65,9 +65,10 @@ template <typename T, typename I, int R, typename TC>
 __global__ void __launch_bounds__(kThreads, PlaqOccupancy<T, TC>::kMinBlocks)
     plaquette_kernel(const __grid_constant__ Geometry g, const __grid_constant__ FieldPtrs<T> f, T* __restrict__ C,
                      const __grid_constant__ EParams<T> p) {
+  __shared__ __align__(8) int sh[kPlaqShared<T, TC>];
   const I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
   if (idx >= (I)(g.plane * (g.nz + 1))) return;
-  plaquette_site<T, I, R, TC>(g, f, C, p, idx);
+  plaquette_site<T, I, R, TC>(g, f, C, p, idx, sh);
 }
 
 template <typename T, typename I, int R>
@@ -253,6 +254,7 @@ LParams<T> make_lparams(const Geometry& g, double dt, bool save_uold, bool do_j,
   const double a3 = g.a[0] * g.a[1] * g.a[2];
   for (int mu = 0; mu < 3; mu++) p.cU[mu] = (T)(-(0.5 * dt) * g.a[mu] * g.a[mu] / a3);
   p.cj = (T)(dt / g.a[2]);
+  set_gather_weights(g, dt, p);
   p.save_uold = save_uold ? 1 : 0;
   p.do_j = do_j ? 1 : 0;
   p.do_second = do_second ? 1 : 0;

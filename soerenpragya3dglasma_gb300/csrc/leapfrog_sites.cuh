@@ -2,6 +2,7 @@
 // launches (leapfrog.cu) and the batched multi-event launches (batch.cu).
 #pragma once
 
+#include "fx.cuh"
 #include "lattice.cuh"
 
 namespace glasma {
@@ -13,20 +14,43 @@ constexpr int kThreads = 128;
 // of two); the double-float force kernel keeps its out-of-line single actions (ddf.cuh).
 template <typename TC>
 constexpr bool kPairRotations = !std::is_same<TC, ddf>::value;
-// The pairs of the current transport (Jp and Jm rotated by one link) only in FP64, where the FP64 pipe
-// bounds the kernels: at the FP32 link kernels' 64-register cap the paired form spills.
+// The pairs of the current transport (Jp and Jm rotated by one link) only in FP64: at the FP32 link kernels'
+// 64-register cap the paired form spills.
 template <typename T>
 constexpr bool kPairCurrents = std::is_same<T, double>::value;
 
-// out_p = V (t.ep) V^d, out_m = V (t.em) V^d (adj = true) or the V^d . V forms, paired where kPairCurrents
+// What the integer pipe's fixed-point products hand back (fx.cuh), out of line.
+template <bool adj>
+__device__ __noinline__ void rotate_pair_fp64(const Mat<double>& V, const Alg<double>& ep, const Alg<double>& em,
+                                              Alg<double>& out_p, Alg<double>& out_m) {
+  if constexpr (adj)
+    adj_mul2(V, ep, em, out_p, out_m);
+  else
+    inv_adj_mul2(V, ep, em, out_p, out_m);
+}
+static __device__ __noinline__ void near_identity_fp64(const Mat<double>& Xm1, const Mat<double>& u, Mat<double>& out) {
+  mul_near_identity(Xm1, u, out);
+}
+
+// out_p = V (t.ep) V^d, out_m = V (t.em) V^d (adj = true) or the V^d . V forms, paired where kPairCurrents, in FP64 on
+// the integer pipe
 template <typename T, bool adj>
 __device__ __forceinline__ void rotate_currents(const Mat<T>& V, const Alg<T>& ep, const Alg<T>& em, Alg<T>& out_p,
                                                 Alg<T>& out_m) {
   if constexpr (kPairCurrents<T>) {
-    if constexpr (adj)
-      adj_mul2(V, ep, em, out_p, out_m);
-    else
-      inv_adj_mul2(V, ep, em, out_p, out_m);
+    fx::Guard g = fx::guard_init();
+    fx::M v;
+    int e;
+    fx::from_mat<true>(V, v, e, g);
+    fx::adj_pair<!adj>(v, ep, em, out_p, out_m, g);
+    if (fx::tripped(g)) {
+      const Mat<double> Vc = V;
+      const Alg<double> a = ep, b = em;
+      Alg<double> oa, ob;
+      rotate_pair_fp64<adj>(Vc, a, b, oa, ob);
+      out_p = oa;
+      out_m = ob;
+    }
   } else {
     if constexpr (adj) {
       adj_mul(V, ep, out_p);
@@ -35,6 +59,21 @@ __device__ __forceinline__ void rotate_currents(const Mat<T>& V, const Alg<T>& e
       inv_adj_mul(V, ep, out_p);
       inv_adj_mul(V, em, out_m);
     }
+  }
+}
+
+// out = X u from X - 1: FP64 on the integer pipe, FP32 as mul_near_identity
+template <typename T>
+__device__ __forceinline__ void link_apply(const Mat<T>& Xm1, const Mat<T>& u, Mat<T>& out) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (!fx::add_product(Xm1, u, out)) {
+      const Mat<double> a = Xm1, b = u;
+      Mat<double> o;
+      near_identity_fp64(a, b, o);
+      out = o;
+    }
+  } else {
+    mul_near_identity(Xm1, u, out);
   }
 }
 
@@ -59,6 +98,9 @@ __device__ __forceinline__ void rotate_currents(const Mat<T>& V, const Alg<T>& e
 #ifndef GLASMA_DDF_PLAQ_MIN_BLOCKS
 #define GLASMA_DDF_PLAQ_MIN_BLOCKS 3
 #endif
+#ifndef GLASMA_FX_PLAQ_MIN_BLOCKS
+#define GLASMA_FX_PLAQ_MIN_BLOCKS 3
+#endif
 template <typename T>
 struct Occupancy;
 template <>
@@ -66,7 +108,7 @@ struct Occupancy<double> {
   static constexpr int kMinBlocks = GLASMA_FP64_MIN_BLOCKS;       // electric-field kernel
   static constexpr int kLinksMinBlocks = GLASMA_FP64_MIN_BLOCKS;  // link/J kernel
   static constexpr int kFusedMinBlocks = GLASMA_FP64_MIN_BLOCKS;  // one-pass step kernel
-  static constexpr int kPlaqMinBlocks = GLASMA_FP64_MIN_BLOCKS;   // plaquette-method force kernel
+  static constexpr int kPlaqMinBlocks = GLASMA_FX_PLAQ_MIN_BLOCKS;  // plaquette-method force kernel
 };
 template <>
 struct Occupancy<float> {
@@ -252,9 +294,10 @@ __device__ __forceinline__ void efield_site(const Geometry& g, const FieldPtrs<T
 // each, three shared) and three final products: ~18 instead of ~24 matrix products per site.
 // K1' (plaquette_site) runs one thread per plaquette owner y, slices -1 .. Nz-1 (the ghost slice owns
 // the plaquettes whose lower-staple terms reach slice 0): it adds the first two terms and the current
-// source to E at y and stores the last two, already weighted, in a contribution buffer at y.  K2'
-// (links_site with kGather) adds the two contributions each link receives, from y = x-q and x-p, to
-// E before it exponentiates it.  Contribution slots C[(slot*8 + a)*S + y]:
+// source to E at y and stores the rotated vectors of the last two, without their weights, in a contribution
+// buffer at y.  K2' (links_site with kGather) adds the two each link receives, from y = x-q and x-p, times
+// their weights (LParams wa, wb: an fma where a weighted contribution would take an add) to E before it
+// exponentiates it.  Contribution slots C[(slot*8 + a)*S + y]:
 enum ContribSlot {
   kC01p = 0,  // plane (0,1), to link 1 at y+x
   kC01q = 1,  // plane (0,1), to link 0 at y+y
@@ -286,8 +329,8 @@ __device__ __forceinline__ void plaquette_alg(const Mat<T>& a, const Mat<T>& b, 
 // arithmetic type: T itself, or ddf for FP64 fields (double-float arithmetic on the FP32 pipe, the
 // fields converted on load and store).
 template <typename T, typename I, int R, typename TC = T>
-__device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtrs<T>& f, T* __restrict__ C,
-                                               const EParams<T>& p, I idx) {
+__device__ __forceinline__ void plaquette_site_direct(const Geometry& g, const FieldPtrs<T>& f, T* __restrict__ C,
+                                                      const EParams<T>& p, I idx) {
   const I S = (I)g.S, plane = (I)g.plane;
   const I s = idx;
   const int zz = (int)(idx / plane);
@@ -332,8 +375,6 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
     plaquette_alg(u1, b, c, u2, al12);
     if (below_top) {
       inv_adj_mul2(u2, al, al12, out, out2);
-      scale_alg(-w02p, out);  // to link 0 at y+z
-      scale_alg(-w12p, out2);  // to link 1 at y+z
       if (!p.dry) {
         store_alg_c(C, S, kC02q * 8, s, out);
         store_alg_c(C, S, kC12q * 8, s, out2);
@@ -348,15 +389,11 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
       F2.a[k] -= w12q * al12.a[k];
     }
     inv_adj_mul2(u1, al01, al12, out, out2);
-    scale_alg(-w01p, out);  // to link 0 at y+y
-    scale_alg(w12q, out2);  // to link 2 at y+y
     if (!p.dry) {
       store_alg_c(C, S, kC01q * 8, s, out);
       store_alg_c(C, S, kC12p * 8, s, out2);
     }
     inv_adj_mul2(u0, al01, al, out, out2);
-    scale_alg(w01q, out);  // to link 1 at y+x
-    scale_alg(w02q, out2);  // to link 2 at y+x
     if (!p.dry) {
       store_alg_c(C, S, kC01p * 8, s, out);
       store_alg_c(C, S, kC02p * 8, s, out2);
@@ -373,10 +410,8 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
         F1.a[k] = -w01q * al.a[k];
       }
       inv_adj_mul(u1, al, out);  // to link 0 at y+y
-      scale_alg(-w01p, out);
       if (!p.dry) store_alg_c(C, S, kC01q * 8, s, out);
       inv_adj_mul(u0, al, out);  // to link 1 at y+x
-      scale_alg(w01q, out);
       if (!p.dry) store_alg_c(C, S, kC01p * 8, s, out);
     }
     // plane (0,2): a = U_0(y), b = U_2(y+x), c = U_0(y+z), d = U_2(y)
@@ -385,7 +420,6 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
     plaquette_alg(u0, b, c, u2, al);
     if (below_top) {
       inv_adj_mul(u2, al, out);  // to link 0 at y+z
-      scale_alg(-w02p, out);
       if (!p.dry) store_alg_c(C, S, kC02q * 8, s, out);
     }
     if (interior) {
@@ -395,7 +429,6 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
         F2.a[k] = -w02q * al.a[k];
       }
       inv_adj_mul(u0, al, out);  // to link 2 at y+x
-      scale_alg(w02q, out);
       if (!p.dry) store_alg_c(C, S, kC02p * 8, s, out);
     }
     // plane (1,2): a = U_1(y), b = U_2(y+y), c = U_1(y+z), d = U_2(y)
@@ -404,7 +437,6 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
     plaquette_alg(u1, b, c, u2, al);
     if (below_top) {
       inv_adj_mul(u2, al, out);  // to link 1 at y+z
-      scale_alg(-w12p, out);
       if (!p.dry) store_alg_c(C, S, kC12q * 8, s, out);
     }
     if (!interior) return;
@@ -414,7 +446,6 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
       F2.a[k] -= w12q * al.a[k];
     }
     inv_adj_mul(u1, al, out);  // to link 2 at y+y
-    scale_alg(w12q, out);
     if (!p.dry) store_alg_c(C, S, kC12p * 8, s, out);
   }
   // E += the forces of the plaquettes owned here (+ the current source on E_z); K2' adds the rest
@@ -474,6 +505,175 @@ __device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtr
   }
 }
 
+// plaquette_site for FP64 fields with the products on the integer pipe (fx.cuh).  Bound by FP64, the direct form
+// runs ~2000 FP64 operations per site; here they are ~5,000 mad.wide and as many integer operations, with ~200
+// FP64 ones beside them (the sums into E, the scaling of the contributions).  The plaquettes in a loop and the
+// four rotation pairs in a loop, so that the code stays inside the instruction cache (a straight-line body of
+// ~12,000 instructions does not); the three anti-Hermitian parts wait in shared memory for their rotations.
+// False, with neither E nor JStat written, where the fixed-point format does not hold the site's values.
+constexpr int kFxShared = 3 * 18 * kThreads + 3 * kThreads;  // ints of shared memory per block
+
+template <typename I>
+__device__ __forceinline__ bool plaquette_site_fx(const Geometry& g, const FieldPtrs<double>& f, double* __restrict__ C,
+                                                  const EParams<double>& p, I idx, int* __restrict__ sh) {
+  using fx::ll;
+  const I S = (I)g.S, plane = (I)g.plane;
+  const I s = idx;
+  const int zz = (int)(idx / plane);
+  const int z = zz - 1;
+  const int r = (int)(idx - (I)zz * plane);
+  const int y = r / g.nx, x = r - y * g.nx;
+  const bool interior = z >= 0;
+  const bool below_top = z < g.nz - 1;
+  const I sxp = nb<I>(g, x, y, z, 1, 0, 0), syp = nb<I>(g, x, y, z, 0, 1, 0), szp = s + plane;
+  ll* const slot = reinterpret_cast<ll*>(sh) + threadIdx.x;  // number w of plane n: slot[(n * 9 + w) * kThreads]
+  int* const slot_e = sh + 3 * 18 * kThreads + threadIdx.x;
+  auto put = [&](int n, const fx::Anti& a) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      slot[(n * 9 + k) * kThreads] = a.y[k];
+      slot[(n * 9 + 3 + k) * kThreads] = a.x[k];
+      slot[(n * 9 + 6 + k) * kThreads] = a.d[k];
+    }
+    slot_e[n * kThreads] = a.e;
+  };
+  auto get = [&](int n, fx::Anti& a) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      a.y[k] = slot[(n * 9 + k) * kThreads];
+      a.x[k] = slot[(n * 9 + 3 + k) * kThreads];
+      a.d[k] = slot[(n * 9 + 6 + k) * kThreads];
+    }
+    a.e = slot_e[n * kThreads];
+  };
+  fx::Guard guard = fx::guard_init();
+  // planes 0: (0,1), 1: (0,2), 2: (1,2); the ghost slice -1 owns only those with z
+#pragma unroll 1
+  for (int n = interior ? 0 : 1; n < 3; n++) {
+    const int mp = n == 2 ? 1 : 0, mq = n == 0 ? 1 : 2;
+    const I sp = n == 2 ? syp : sxp, sq = n == 0 ? syp : szp;
+    fx::M a, b, w, v;
+    int ea, eb, ew, ev;
+    fx::link_near(f.U, S, mp, s, a, ea, guard);
+    fx::link_near(f.U, S, mq, sp, b, eb, guard);
+    fx::near_product(a, ea, b, eb, w, ew, guard);
+    fx::link_near(f.U, S, mq, s, a, ea, guard);
+    fx::link_near(f.U, S, mp, sq, b, eb, guard);
+    fx::near_product(a, ea, b, eb, v, ev, guard);
+    fx::Anti al;
+    fx::plaquette_parts(w, ew, v, ev, al);
+    put(n, al);
+  }
+  // rotations: 0 by u2 (al02, al12), 1 by u1 (al01, al12), 2 by u0 (al01, al02), 3 the currents below by U_2(y-z)
+  const double w01p = p.gc[0] * p.cnu[1], w01q = p.gc[1] * p.cnu[0];
+  const double w02p = p.gc[0] * p.cnu[2], w02q = p.gc[2] * p.cnu[0];
+  const double w12p = p.gc[1] * p.cnu[2], w12q = p.gc[2] * p.cnu[1];
+  Alg<double> down, downm;
+#pragma unroll 1
+  for (int n = below_top ? 0 : 1; n < (interior ? 4 : 1); n++) {
+    fx::M v, m;
+    int e;
+    ll tr_re, tr_im, o1[8], o2[8];
+    fx::link_plain(f.U, S, n == 3 ? 2 : 2 - n, n == 3 ? s - plane : s, v, guard);
+    if (n < 3) {
+      fx::Anti a1, a2;
+      get(n == 0 ? 1 : 0, a1);
+      get(n == 2 ? 1 : 2, a2);
+      fx::herm_pair(a1, a2, m, e, tr_re, tr_im);
+    } else {
+      Alg<double> jp, jm;
+      load_alg(f.Jp, S, 0, s - plane, jp);
+      load_alg(f.Jm, S, 0, s - plane, jm);
+      fx::herm_pair(jp, jm, m, e, tr_re, tr_im, guard);
+    }
+    fx::rotate_pair<true>(v, m, tr_re, tr_im, o1, o2, guard);
+    if (n < 3) {
+      const int k1 = n == 0 ? kC02q : (n == 1 ? kC01q : kC01p), k2 = n == 0 ? kC12q : (n == 1 ? kC12p : kC02p);
+      Alg<double> out, out2;
+      fx::to_alg(o1, e - fx::kScale - 2, -1.0, out);
+      fx::to_alg(o2, e - fx::kScale - 2, -1.0, out2);
+      if (!p.dry) {
+        store_alg(C, S, k1 * 8, s, out);
+        store_alg(C, S, k2 * 8, s, out2);
+      }
+    } else {
+      fx::to_alg(o1, e - fx::kScale - 1, 1.0, down);
+      fx::to_alg(o2, e - fx::kScale - 1, 1.0, downm);
+    }
+  }
+  if (fx::tripped(guard)) return false;
+  if (!interior) return true;
+  // E += the forces of the plaquettes owned here (+ the current source on E_z)
+#pragma unroll 1
+  for (int mu = 0; mu < 3; mu++) {
+    // link 0: +w01p al01 + w02p al02; link 1: -w01q al01 + w12p al12; link 2: -w02q al02 - w12q al12
+    const int n1 = mu == 2 ? 1 : 0, n2 = mu == 0 ? 1 : 2;
+    fx::Anti a1, a2;
+    get(n1, a1);
+    get(n2, a2);
+    const double c1 = -0.5 * (mu == 0 ? w01p : (mu == 1 ? -w01q : -w02q));
+    const double c2 = -0.5 * (mu == 0 ? w02p : (mu == 1 ? w12p : -w12q));
+    Alg<double> e, F;
+    load_alg(f.E, S, mu * 8, s, e);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const double q = k == 7 ? Consts<double>::inv_sqrt3() : 1.0;
+      F.a[k] = fma(fx::from_fixed(fx::component(a2, k), a2.e - fx::kScale), c2 * q,
+                   fx::from_fixed(fx::component(a1, k), a1.e - fx::kScale) * (c1 * q));
+    }
+    if (mu == 2) {
+      Alg<double> jp, jm;
+      load_alg(f.Jp, S, 0, s, jp);
+      load_alg(f.Jm, S, 0, s, jm);
+#pragma unroll
+      for (int k = 0; k < 8; k++) F.a[k] += p.jz * (jp.a[k] - jm.a[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) e.a[k] += F.a[k];
+    if (!p.dry) store_alg(f.E, S, mu * 8, s, e);
+  }
+  // UpdateJStat, as K1
+  const bool lo = (z == 0), hi = (z == g.nz - 1);
+  const I sg = lo ? s - plane : (hi ? s + plane : (I)-1);
+  Alg<double> jc, st;
+  load_alg(f.Jp, S, 0, s, jc);
+  load_alg(f.JpStat, S, 0, s, st);
+  axpy_diff(st, -p.cj, jc, down);
+  if (!p.dry) {
+    store_alg(f.JpStat, S, 0, s, st);
+    if (sg >= 0) store_alg(f.JpStat, S, 0, sg, st);
+  }
+  load_alg(f.Jm, S, 0, s, jc);
+  load_alg(f.JmStat, S, 0, s, st);
+  axpy_diff(st, p.cj, jc, downm);
+  if (!p.dry) {
+    store_alg(f.JmStat, S, 0, s, st);
+    if (sg >= 0) store_alg(f.JmStat, S, 0, sg, st);
+  }
+  return true;
+}
+
+// Out of line: the sites that the fixed-point form hands back.
+template <typename I>
+__device__ __noinline__ void plaquette_site_fp64(const Geometry& g, const FieldPtrs<double>& f, double* C,
+                                                 const EParams<double>& p, I idx) {
+  plaquette_site_direct<double, I, 3>(g, f, C, p, idx);
+}
+
+// Ints of shared memory the force kernel of type T, TC needs per block.
+template <typename T, typename TC>
+constexpr int kPlaqShared = (std::is_same<T, double>::value && std::is_same<TC, double>::value) ? kFxShared : 2;
+
+template <typename T, typename I, int R, typename TC = T>
+__device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtrs<T>& f, T* __restrict__ C,
+                                               const EParams<T>& p, I idx, int* sh) {
+  if constexpr (std::is_same<T, double>::value && std::is_same<TC, double>::value) {
+    if (!plaquette_site_fx<I>(g, f, C, p, idx, sh)) plaquette_site_fp64<I>(g, f, C, p, idx);
+  } else {
+    plaquette_site_direct<T, I, R, TC>(g, f, C, p, idx);
+  }
+}
+
 // Blocks per SM of the force kernel: by storage type, and for FP64 fields computed in double-float.
 template <typename T, typename TC>
 struct PlaqOccupancy {
@@ -513,8 +713,29 @@ template <typename T>
 struct LParams {
   T cU[3];  // -(h) a_mu^2 / a^3 for the half step h
   T cj;     // dt/a_z
+  T wa[3], wb[3];  // plaquette method: weights of the two contributions link mu gathers
   int save_uold, do_j, do_second;
 };
+
+// Weights of the contributions: gc_p c_q and gc_q c_p with gc_mu = gamma c_mu, gamma = -2 dt a^3, c_mu = 1 / a_mu^2,
+// formed in the fields' precision.  Link 0 gathers (0,1) from x-y and (0,2) from x-z, link 1 (0,1) from x-x and (1,2)
+// from x-z, link 2 (0,2) from x-x and (1,2) from x-y.
+template <typename T>
+inline void set_gather_weights(const Geometry& g, double dt, LParams<T>& p) {
+  const double gamma = -2.0 * dt * (g.a[0] * g.a[1] * g.a[2]);
+  T gc[3], c[3];
+  for (int mu = 0; mu < 3; mu++) {
+    const double ce = 1.0 / (g.a[mu] * g.a[mu]);
+    gc[mu] = (T)(gamma * ce);
+    c[mu] = (T)ce;
+  }
+  p.wa[0] = -(gc[0] * c[1]);
+  p.wb[0] = -(gc[0] * c[2]);
+  p.wa[1] = gc[1] * c[0];
+  p.wb[1] = -(gc[1] * c[2]);
+  p.wa[2] = gc[2] * c[0];
+  p.wb[2] = gc[2] * c[1];
+}
 
 // K2's per-site body: links to t+dt (two applications of one exp), UOld, J transport.  kGather (the
 // plaquette method): first E_mu += the two contributions link mu receives from the plaquette owners
@@ -549,7 +770,7 @@ __device__ __forceinline__ void links_site(const Geometry& g, const FieldPtrs<T>
       load_alg(C, S, c1 * 8, s1, a1);
       load_alg(C, S, c2 * 8, s2, a2);
 #pragma unroll
-      for (int k = 0; k < 8; k++) e.a[k] += a1.a[k] + a2.a[k];
+      for (int k = 0; k < 8; k++) e.a[k] += fma(pick3(p.wa, mu), a1.a[k], pick3(p.wb, mu) * a2.a[k]);
       store_alg(f.E, S, mu * 8, s, e);
       if (sg >= 0) store_alg(f.E, S, mu * 8, sg, e);
     }

@@ -463,23 +463,27 @@ __device__ __forceinline__ void expi_impl(T c, const Alg<T>& al, Mat<T>& X) {
   for (int a = 0; a < 8; a++) sc.a[a] = c * al.a[a];
   Mat<T> Q, Q2;
   herm_from_alg(sc, Q);
-  // Q^2 is Hermitian: its upper triangle and real diagonal, the rest by conjugation
-  mul_nn_herm(Q, Q, Q2);
-  Q2.e[1] = mk<T>(Q2.e[3].re, -Q2.e[3].im);
-  Q2.e[2] = mk<T>(Q2.e[6].re, -Q2.e[6].im);
-  Q2.e[5] = mk<T>(Q2.e[7].re, -Q2.e[7].im);
-  Q2.e[0].im = Q2.e[4].im = Q2.e[8].im = T(0);
+  // Q^2 of a traceless Hermitian Q: the off-diagonal entries as -Q_kk Q_ij + Q_ik Q_kj, the diagonal from the
+  // moduli, the lower triangle by conjugation
+  const T q0 = Q.e[0].re, q1 = Q.e[4].re, q2 = Q.e[8].re;
+  const cx<T> a01 = Q.e[3], a02 = Q.e[6], a12 = Q.e[7];
+  const T m01 = fma(a01.re, a01.re, a01.im * a01.im), m02 = fma(a02.re, a02.re, a02.im * a02.im),
+          m12 = fma(a12.re, a12.re, a12.im * a12.im);
+  Q2.e[3] = mk<T>(fma(-q2, a01.re, fma(a02.re, a12.re, a02.im * a12.im)),   // Q02 conj(Q12)
+                  fma(-q2, a01.im, fma(a02.im, a12.re, -(a02.re * a12.im))));
+  Q2.e[6] = mk<T>(fma(-q1, a02.re, fma(a01.re, a12.re, -(a01.im * a12.im))),  // Q01 Q12
+                  fma(-q1, a02.im, fma(a01.re, a12.im, a01.im * a12.re)));
+  Q2.e[7] = mk<T>(fma(-q0, a12.re, fma(a01.re, a02.re, a01.im * a02.im)),   // conj(Q01) Q02
+                  fma(-q0, a12.im, fma(a01.re, a02.im, -(a01.im * a02.re))));
+  Q2.e[0] = mk<T>(fma(q0, q0, m01 + m02), T(0));
+  Q2.e[4] = mk<T>(fma(q1, q1, m01 + m12), T(0));
+  Q2.e[8] = mk<T>(fma(q2, q2, m02 + m12), T(0));
   const T c1 = T(0.5) * (Q2.e[0].re + Q2.e[4].re + Q2.e[8].re);
-  // det Q = Q00 (Q11 Q22 - |Q12|^2) - ... ; real for Hermitian Q.  Expanded in the
-  // Gell-Mann components for brevity: det Q = tr(Q^3)/3.
-  T c0 = (Q2.e[0].re * Q.e[0].re + Q2.e[4].re * Q.e[4].re + Q2.e[8].re * Q.e[8].re);
-  // tr(Q2 Q) = sum_ij Q2_ij Q_ji; add off-diagonal terms (both triangles)
-  c0 += T(2) * (Q2.e[3].re * Q.e[1].re - Q2.e[3].im * Q.e[1].im);  // (0,1)*(1,0) + (1,0)*(0,1)
-  c0 += T(2) * (Q2.e[6].re * Q.e[2].re - Q2.e[6].im * Q.e[2].im);  // (0,2)*(2,0) + (2,0)*(0,2)
-  c0 += T(2) * (Q2.e[7].re * Q.e[5].re - Q2.e[7].im * Q.e[5].im);  // (1,2)*(2,1) + (2,1)*(1,2)
-  c0 *= T(1) / T(3);
+  // det Q = q0 q1 q2 + 2 Re(Q01 Q12 conj(Q02)) - q0 |Q12|^2 - q1 |Q02|^2 - q2 |Q01|^2, real
+  const T t01 = fma(a01.re, a12.re, -(a01.im * a12.im)), t12 = fma(a01.re, a12.im, a01.im * a12.re);
+  const T c0 = fma(q0, fma(q1, q2, -m12), fma(T(2), fma(t01, a02.re, t12 * a02.im), -fma(q1, m02, q2 * m01)));
   cx<T> f0, f1, f2;
-  if (sizeof(T) == 8 && !kMinusOne && c1 >= Trig<T>::taylor_c1() && c1 < T(0.5)) {
+  if (sizeof(T) == 8 && c1 >= Trig<T>::taylor_c1() && c1 < T(0.5)) {
     // FP64 without transcendental functions (they cost ~60 % of this exponential on GB300's FP64 pipe):
     // exp(iQ) = sum_n i^n Q^n / n!, and by Cayley-Hamilton (Q^3 = c1 Q + c0) Q^n / n! = a_n + b_n Q + d_n
     // Q^2 with a_{n+1} = c0 d_n / (n+1), b_{n+1} = (a_n + c1 d_n) / (n+1), d_{n+1} = b_n / (n+1).  The
@@ -490,7 +494,7 @@ __device__ __forceinline__ void expi_impl(T c, const Alg<T>& al, Mat<T>& X) {
     // beyond c1 = 0.5 the closed form below.
     const int nterms = c1 < T(1e-4) ? 7 : (c1 < T(1e-3) ? 8 : (c1 < T(0.02) ? 11 : 17));
     T a = T(1), b = T(0), d = T(0);
-    T f0r = T(1), f0i = T(0), f1r = T(0), f1i = T(0), f2r = T(0), f2i = T(0);
+    T f0r = T(kMinusOne ? 0 : 1), f0i = T(0), f1r = T(0), f1i = T(0), f2r = T(0), f2i = T(0);
 #pragma unroll
     for (int n = 1; n <= 17; n++) {
       if (n > nterms) break;
@@ -578,19 +582,22 @@ __device__ __forceinline__ void expi_impl(T c, const Alg<T>& al, Mat<T>& X) {
     }
     if (kMinusOne) f0.re -= T(1);
   }
+  // f1 Q + f2 Q^2, entries (i,j) and (j,i) from the same products: with r = f1r Q.re + f2r Q2.re, s = f1i Q.im +
+  // f2i Q2.im, t = f1r Q.im + f2r Q2.im, u = f1i Q.re + f2i Q2.re at (i,j) they are (r - s, u + t) and (r + s, u - t)
+  constexpr int up[3] = {3, 6, 7}, low[3] = {1, 2, 5};
 #pragma unroll
-  for (int k = 0; k < 9; k++) {
-    cx<T> v = mk<T>(T(0), T(0));
-    cfma(v, f1, Q.e[k]);
-    cfma(v, f2, Q2.e[k]);
-    X.e[k] = v;
+  for (int n = 0; n < 3; n++) {
+    const cx<T> q = Q.e[up[n]], p = Q2.e[up[n]];
+    const T r = fma(f1.re, q.re, f2.re * p.re), sI = fma(f1.im, q.im, f2.im * p.im);
+    const T t = fma(f1.re, q.im, f2.re * p.im), u = fma(f1.im, q.re, f2.im * p.re);
+    X.e[up[n]] = mk<T>(r - sI, u + t);
+    X.e[low[n]] = mk<T>(r + sI, u - t);
   }
-  X.e[0].re += f0.re;
-  X.e[0].im += f0.im;
-  X.e[4].re += f0.re;
-  X.e[4].im += f0.im;
-  X.e[8].re += f0.re;
-  X.e[8].im += f0.im;
+#pragma unroll
+  for (int k = 0; k < 9; k += 4) {
+    X.e[k].re = fma(f1.re, Q.e[k].re, f2.re * Q2.e[k].re) + f0.re;
+    X.e[k].im = fma(f1.im, Q.e[k].re, f2.im * Q2.e[k].re) + f0.im;
+  }
 }
 template <typename T>
 __device__ __forceinline__ void expi(T c, const Alg<T>& al, Mat<T>& X) {
@@ -639,20 +646,10 @@ __device__ __forceinline__ void mul_near_identity(const Mat<T>& Xm1, const Mat<T
     out.e[k].im += u.e[k].im;
   }
 }
-// The link update's exponential and its application: FP32 keeps X - 1 (expi_m1), FP64 forms X.
+// The link update's exponential, as X - 1.
 template <typename T>
-__device__ __forceinline__ void link_exp(T c, const Alg<T>& al, Mat<T>& X) {
-  if (sizeof(T) == 4)
-    expi_m1(c, al, X);
-  else
-    expi(c, al, X);
-}
-template <typename T>
-__device__ __forceinline__ void link_apply(const Mat<T>& X, const Mat<T>& u, Mat<T>& out) {
-  if (sizeof(T) == 4)
-    mul_near_identity(X, u, out);
-  else
-    mul_nn(X, u, out);
+__device__ __forceinline__ void link_exp(T c, const Alg<T>& al, Mat<T>& Xm1) {
+  expi_m1(c, al, Xm1);
 }
 
 // ||V V^dagger - 1||_F  (S/SUNc/SU3/GroupOperations.cpp:337-349)
