@@ -89,11 +89,10 @@ __global__ void __launch_bounds__(kThreads, Occupancy<T>::kLinksMinBlocks)
 template <typename T, typename I, int R, bool kStride>
 __global__ void __launch_bounds__(kThreads, PlaqOccupancy<T, T>::kMinBlocks)
     plaquette_batch_kernel(const __grid_constant__ EventTable<T> tab, const unsigned short* __restrict__ tile_ev) {
-  __shared__ __align__(8) int sh[kPlaqShared<T, T>];
+  __shared__ __align__(8) int sh[kPlaqShared<T, T, 1>];
   for (long long t = tab.t0 + blockIdx.x; t < tab.t1; t += gridDim.x) {
     const EventDesc<T>& d = tab.ev[tile_ev[t] - tab.ev0];
-    const long long idx = (t - d.k1_begin) * kThreads + threadIdx.x;
-    if (idx < d.g.plane * (d.g.nz + 1)) plaquette_site<T, I, R, T>(d.g, d.f, d.C, d.ep, (I)idx, sh);
+    plaquette_block<T, I, R, T>(d.g, d.f, d.C, d.ep, t - d.k1_begin, d.g.plane * (d.g.nz + 1), sh);
     if (!kStride) break;
   }
 }

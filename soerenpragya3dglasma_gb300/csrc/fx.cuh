@@ -133,6 +133,14 @@ __device__ __forceinline__ double from_fixed(ll q, int k) {
   const unsigned long long b = (t >> 11) + ((t >> 10) & 1) + ((unsigned long long)(unsigned)(1023 + 62 + k - n) << 52);
   return m == 0 ? 0.0 : __longlong_as_double((ll)b | (q & (1LL << 63)));
 }
+// The same by two FP64 additions (q in two pieces placed into the low bits of 2^84 and 2^52) where that pipe has room:
+// 9 operations instead of 24.
+__device__ __forceinline__ double from_fixed_fp64(ll q, int k) {
+  const double hi = __hiloint2double(0x45300000, (int)(q >> 32) ^ (int)0x80000000);
+  const double lo = __hiloint2double(0x43300000, (int)q);
+  const double v = (hi - 19342822341709703277445120.0) + lo;  // 2^84 + 2^63 + 2^52
+  return q == 0 ? 0.0 : __hiloint2double(__double2hiint(v) + (int)((unsigned)k << 20), __double2loint(v));
+}
 // 2^k as a double, -1022 <= k <= 1023
 __device__ __forceinline__ double pow2(int k) { return __hiloint2double((k + 1023) << 20, 0); }
 constexpr int kMinExp = -400;  // smaller values are held at 2^-460
@@ -192,15 +200,20 @@ __device__ __forceinline__ void link_near(const cx<double>* __restrict__ U, I S,
 }
 
 // ---- products -------------------------------------------------------------------------------------------
-// (A B)_ij
-__device__ __forceinline__ void entry_nn(const M& A, int i, const M& B, int j, Acc& rr, Acc& ii, Acc& im) {
-  rr = im = acc_half();
-  ii = acc_zero();
+__device__ __forceinline__ R neg(const R& a) {
+  R r;
+  r.h = -a.h;
+  r.l = -a.l;
+  return r;
+}
+// (A B)_ij; nB: -Im of B's entries
+__device__ __forceinline__ void entry_nn(const M& A, int i, const M& B, const R (&nB)[9], int j, Acc& re, Acc& im) {
+  re = im = acc_half();
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     const C &a = A.e[i + 3 * k], &b = B.e[k + 3 * j];
-    mad(rr, a.re, b.re);
-    mad(ii, a.im, b.im);
+    mad(re, a.re, b.re);
+    mad(re, a.im, nB[k + 3 * j]);
     mad(im, a.re, b.im);
     mad(im, a.im, b.re);
   }
@@ -211,14 +224,17 @@ __device__ __forceinline__ void entry_nn(const M& A, int i, const M& B, int j, A
 __device__ __forceinline__ void near_product(const M& A, int ea, const M& B, int eb, M& W, int& ew, Guard& g) {
   ew = min(max(ea, eb) + 3, 0);
   const int kk = min(ew - ea - eb, 63), ka = min(ew - ea, 63), kb = min(ew - eb, 63);
+  R nB[9];
+#pragma unroll
+  for (int n = 0; n < 9; n++) nB[n] = neg(B.e[n].im);
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      Acc rr, ii, im;
-      entry_nn(A, i, B, j, rr, ii, im);
+      Acc re, im;
+      entry_nn(A, i, B, nB, j, re, im);
       const C &a = A.e[i + 3 * j], &b = B.e[i + 3 * j];
-      W.e[i + 3 * j].re = split((finish_diff(rr, ii) >> kk) + (join(a.re) >> ka) + (join(b.re) >> kb));
+      W.e[i + 3 * j].re = split((finish(re) >> kk) + (join(a.re) >> ka) + (join(b.re) >> kb));
       W.e[i + 3 * j].im = split((finish(im) >> kk) + (join(a.im) >> ka) + (join(b.im) >> kb));
     }
   if (ew == 0) {  // entries near or above 1/8: the rows of 1 + w must have norm one (to 10 %)
@@ -329,59 +345,43 @@ template <bool kInv>
 __device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll tr_re, ll tr_im, ll (&o1)[8], ll (&o2)[8],
                                             Guard& g) {
   ll cr[9], ci[9];
+  R nV[9];
+#pragma unroll
+  for (int n = 0; n < 9; n++) nV[n] = neg(V.e[n].im);
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     C t[3];  // row i of V^dagger M, or of V M
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      Acc a = acc_half(), b = acc_half(), c = acc_zero();
+      Acc re = acc_half(), im = acc_half();
 #pragma unroll
       for (int k = 0; k < 3; k++) {
         const C& m = Mm.e[k + 3 * j];
-        if constexpr (kInv) {  // conj(v) m
-          const C& v = V.e[k + 3 * i];
-          mad(a, v.re, m.re);
-          mad(a, v.im, m.im);
-          mad(b, v.re, m.im);
-          mad(c, v.im, m.re);
-        } else {  // v m
-          const C& v = V.e[i + 3 * k];
-          mad(b, v.re, m.re);
-          mad(c, v.im, m.im);
-          mad(a, v.re, m.im);
-          mad(a, v.im, m.re);
-        }
+        const int n = kInv ? k + 3 * i : i + 3 * k;  // conj(v) m or v m
+        mad(re, V.e[n].re, m.re);
+        mad(re, kInv ? V.e[n].im : nV[n], m.im);
+        mad(im, V.e[n].re, m.im);
+        mad(im, kInv ? nV[n] : V.e[n].im, m.re);
       }
-      const ll dh = b.hh - c.hh;
-      watch(g, a.hh, dh);
-      const R sum = split(finish(a)), dif = split(finish_diff(b, c));
-      t[j].re = kInv ? sum : dif;
-      t[j].im = kInv ? dif : sum;
+      watch(g, re.hh, im.hh);
+      t[j].re = split(finish(re));
+      t[j].im = split(finish(im));
     }
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       if (i == 2 && j == 2) continue;
-      Acc a = acc_half(), b = acc_half(), c = acc_zero();
+      Acc re = acc_half(), im = acc_half();
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        if constexpr (kInv) {  // t v
-          const C& v = V.e[k + 3 * j];
-          mad(b, t[k].re, v.re);
-          mad(c, t[k].im, v.im);
-          mad(a, t[k].re, v.im);
-          mad(a, t[k].im, v.re);
-        } else {  // t conj(v)
-          const C& v = V.e[j + 3 * k];
-          mad(a, t[k].re, v.re);
-          mad(a, t[k].im, v.im);
-          mad(b, t[k].im, v.re);
-          mad(c, t[k].re, v.im);
-        }
+        const int n = kInv ? k + 3 * j : j + 3 * k;  // t v or t conj(v)
+        mad(re, t[k].re, V.e[n].re);
+        mad(re, t[k].im, kInv ? nV[n] : V.e[n].im);
+        mad(im, t[k].im, V.e[n].re);
+        mad(im, t[k].re, kInv ? V.e[n].im : nV[n]);
       }
-      watch(g, a.hh, b.hh - c.hh);
-      const ll sum = finish(a), dif = finish_diff(b, c);
-      cr[i + 3 * j] = kInv ? dif : sum;
-      ci[i + 3 * j] = kInv ? sum : dif;
+      watch(g, re.hh, im.hh);
+      cr[i + 3 * j] = finish(re);
+      ci[i + 3 * j] = finish(im);
     }
   }
   o1[0] = cr[3] + cr[1];
@@ -434,11 +434,14 @@ __device__ __forceinline__ void herm_pair(const Alg<double>& p, const Alg<double
   tr_re = tr_im = 0;
 }
 
-// +-2^k o, the last component over sqrt 3
+// +-2^k o, the last component over sqrt 3; kFp64: by the FP64 pipe
+template <bool kFp64 = false>
 __device__ __forceinline__ void to_alg(const ll (&o)[8], int k, double sign, Alg<double>& out) {
 #pragma unroll
-  for (int n = 0; n < 7; n++) out.a[n] = sign < 0 ? -from_fixed(o[n], k) : from_fixed(o[n], k);
-  out.a[7] = from_fixed(o[7], k) * (sign * Consts<double>::inv_sqrt3());
+  for (int n = 0; n < 8; n++) {
+    const double v = kFp64 ? from_fixed_fp64(o[n], k) : from_fixed(o[n], k);
+    out.a[n] = n == 7 ? v * (sign * Consts<double>::inv_sqrt3()) : (sign < 0 ? -v : v);
+  }
 }
 
 // Two adjoint actions by one plain matrix, as inv_adj_mul2 / adj_mul2: out_k = V^d (t.e_k) V or V (t.e_k) V^d.
@@ -471,21 +474,178 @@ __device__ __forceinline__ void from_mat(const Mat<double>& u, M& m, int& e, Gua
   }
 }
 
-// out = u + A u for A = X - 1 (any size up to one) and a link u: the product in fixed point with A's exponent, the
-// sum in FP64, so the result is rounded once.  False where the format does not hold the operands.
-__device__ __forceinline__ bool add_product(const Mat<double>& A, const Mat<double>& u, Mat<double>& out) {
+// ---- the link update's exponential -----------------------------------------------------------------------
+// f0 - 1, f1, f2 of exp(iQ) = f0 + f1 Q + f2 Q^2 for c1 = tr Q^2 / 2 >= 0.02 (expi_impl's tiers), out of line.
+static __device__ __noinline__ void exp_coefficients(double c0, double c1, double (&f)[6]) {
+  cx<double> f0, f1, f2;
+  exp_coeff<double, true>(c0, c1, f0, f1, f2);
+  f[0] = f0.re;
+  f[1] = f0.im;
+  f[2] = f1.re;
+  f[3] = f1.im;
+  f[4] = f2.re;
+  f[5] = f2.im;
+}
+
+// X - 1 = exp(i c t.al) - 1 in fixed point, exponent e.  False when |c al| has a component of one or more.
+// With B = 2 Q (entries of c al without the factors 1/2) in units of 2^em, em one above the largest component's
+// exponent: Q^2 = B^2 / 4, c1 = tr B^2 / 8, det Q = det B / 8 from 28 products; c0 and c1 leave as doubles, and below
+// c1 = 0.02 (c al up to ~0.1 in every component) f0 - 1, f1, f2 are polynomials in them, exp's power series reduced by
+// Q^3 = c1 Q + c0 and cut after Q^11 / 11! (the next term is below 7e-19): 34 FP64 operations, where the
+// matrix form of this exponential takes ~150.
+__device__ __forceinline__ bool near_exp(double c, const Alg<double>& al, M& X, int& e) {
+  Alg<double> q;
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    q.a[k] = c * al.a[k];
+    top = max(top, habs(q.a[k]));
+  }
+  if (top >= 0x3ff00000) return false;  // also NaN and infinity
+  const int em = max(exponent_of(top), kMinExp) + 1;
+  const int sh = shift(kScale - em);
+  const ll s8 = to_fixed(q.a[7] * Consts<double>::inv_sqrt3(), sh), q2 = to_fixed(q.a[2], sh);
+  R b[3];  // diagonal of B
+  C o[3];  // B_01, B_02, B_12
+  b[0] = split(q2 + s8);
+  b[1] = split(s8 - q2);
+  b[2] = split(-2 * s8);
+  constexpr int comp[3] = {0, 3, 5};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    o[n].re = to_fixed_split(q.a[comp[n]], sh);
+    o[n].im = to_fixed_split(-q.a[comp[n] + 1], sh);
+  }
+  // moduli, products of two off-diagonal entries
+  ll mod[3];
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    Acc a = acc_half();
+    mad(a, o[n].re, o[n].re);
+    mad(a, o[n].im, o[n].im);
+    mod[n] = finish(a);
+  }
+  auto product = [&](const C& u, const C& v, int conj_of, ll& re, ll& im) {  // conj_of: 0 none, 1 of u, 2 of v
+    Acc a = acc_half(), z = acc_half(), y = acc_zero();
+    if (conj_of == 0) {  // (ur vr - ui vi, ur vi + ui vr)
+      mad(z, u.re, v.re);
+      mad(y, u.im, v.im);
+      mad(a, u.re, v.im);
+      mad(a, u.im, v.re);
+      re = finish_diff(z, y);
+      im = finish(a);
+    } else {  // (ur vr + ui vi, +-(ur vi - ui vr))
+      mad(a, u.re, v.re);
+      mad(a, u.im, v.im);
+      mad(z, conj_of == 1 ? u.re : u.im, conj_of == 1 ? v.im : v.re);
+      mad(y, conj_of == 1 ? u.im : u.re, conj_of == 1 ? v.re : v.im);
+      re = finish(a);
+      im = finish_diff(z, y);
+    }
+  };
+  auto times = [&](const R& u, const R& v) {
+    Acc a = acc_half();
+    mad(a, u, v);
+    return finish(a);
+  };
+  ll pr[3], pi[3];
+  product(o[1], o[2], 2, pr[0], pi[0]);  // B02 conj(B12)
+  product(o[0], o[2], 0, pr[1], pi[1]);  // B01 B12
+  product(o[0], o[1], 1, pr[2], pi[2]);  // conj(B01) B02
+  ll det = 0;
+  {
+    C t;
+    t.re = split(pr[1]);
+    t.im = split(pi[1]);
+    const R n = split(times(b[1], b[2]) - mod[2]);
+    Acc a = acc_half(), d = acc_zero();
+    mad(a, t.re, o[1].re);
+    mad(a, t.im, o[1].im);
+    det = 2 * finish(a);
+    a = acc_half();
+    mad(a, b[0], n);
+    mad(d, b[1], split(mod[1]));
+    mad(d, b[2], split(mod[0]));
+    det += finish_diff(a, d);
+  }
+  const ll d0 = times(b[0], b[0]) + mod[0] + mod[1], d1 = times(b[1], b[1]) + mod[0] + mod[2],
+           d2 = times(b[2], b[2]) + mod[1] + mod[2];
+  const double c1 = from_fixed(d0 + d1 + d2, 2 * em - kScale - 3), c0 = from_fixed(det, 3 * em - kScale - 3);
+  double f[6];
+  if (c1 < 0.02) {
+    const double z = c0 * c0;
+    f[0] = z * fma(c1, fma(c1, -1.0 / 1209600, 1.0 / 20160), -1.0 / 720);
+    f[1] = c0 * fma(z, 1.0 / 362880, fma(c1, fma(c1, fma(c1, fma(c1, -1.0 / 39916800, 1.0 / 362880), -1.0 / 5040), 1.0 / 120), -1.0 / 6));
+    f[2] = c0 * fma(z, -1.0 / 3628800, fma(c1, fma(c1, fma(c1, -1.0 / 907200, 1.0 / 13440), -1.0 / 360), 1.0 / 24));
+    f[3] = fma(z, fma(c1, fma(c1, -1.0 / 6652800, 1.0 / 120960), -1.0 / 5040),
+               fma(c1, fma(c1, fma(c1, fma(c1, fma(c1, -1.0 / 39916800, 1.0 / 362880), -1.0 / 5040), 1.0 / 120), -1.0 / 6), 1.0));
+    f[4] = fma(z, fma(c1, -1.0 / 1209600, 1.0 / 40320),
+               fma(c1, fma(c1, fma(c1, fma(c1, -1.0 / 3628800, 1.0 / 40320), -1.0 / 720), 1.0 / 24), -0.5));
+    f[5] = c0 * fma(z, -1.0 / 39916800, fma(c1, fma(c1, fma(c1, -1.0 / 9979200, 1.0 / 120960), -1.0 / 2520), 1.0 / 120));
+  } else {
+    exp_coefficients(c0, c1, f);
+  }
+  // X - 1 = f0 - 1 + (f1 B + 2^(em-1) (f2 / 2^(em-1)) B^2 / 2) / 2 in units of 2^(em-1): B^2 moved to B's units
+  e = em - 1;
+  const int down = min(1 - em, 63);
+  C g1, g2;
+  g1.re = to_fixed_split(f[2], shift(kScale));
+  g1.im = to_fixed_split(f[3], shift(kScale));
+  g2.re = to_fixed_split(f[4], shift(kScale));
+  g2.im = to_fixed_split(f[5], shift(kScale));
+  constexpr int up[3] = {3, 6, 7}, low[3] = {1, 2, 5}, opp[3] = {2, 1, 0};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    C w;  // (B^2)_ij = -B_kk B_ij + B_ik B_kj
+    w.re = split((pr[n] - times(b[opp[n]], o[n].re)) >> down);
+    w.im = split((pi[n] - times(b[opp[n]], o[n].im)) >> down);
+    Acc r = acc_half(), s = acc_half(), t = acc_half(), u = acc_half();
+    mad(r, g1.re, o[n].re);
+    mad(r, g2.re, w.re);
+    mad(s, g1.im, o[n].im);
+    mad(s, g2.im, w.im);
+    mad(t, g1.re, o[n].im);
+    mad(t, g2.re, w.im);
+    mad(u, g1.im, o[n].re);
+    mad(u, g2.im, w.re);
+    const ll rr = finish(r), ss = finish(s), tt = finish(t), uu = finish(u);
+    X.e[up[n]].re = split(rr - ss);
+    X.e[up[n]].im = split(uu + tt);
+    X.e[low[n]].re = split(rr + ss);
+    X.e[low[n]].im = split(uu - tt);
+  }
+  const ll f0r = to_fixed(f[0], shift(kScale - e)), f0i = to_fixed(f[1], shift(kScale - e));
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    const R w = split((n == 0 ? d0 : (n == 1 ? d1 : d2)) >> down);
+    Acc r = acc_half(), u = acc_half();
+    mad(r, g1.re, b[n]);
+    mad(r, g2.re, w);
+    mad(u, g1.im, b[n]);
+    mad(u, g2.im, w);
+    X.e[4 * n].re = split(finish(r) + f0r);
+    X.e[4 * n].im = split(finish(u) + f0i);
+  }
+  return true;
+}
+
+// out = u + A u for A = X - 1 in fixed point and a link u: the product with A's exponent, the sum in FP64, so the
+// result is rounded once.  False where the format does not hold u.
+__device__ __forceinline__ bool add_product(const M& a, int ea, const Mat<double>& u, Mat<double>& out) {
   Guard g = guard_init();
-  M a, b;
-  int ea, eb;
-  from_mat<false>(A, a, ea, g);
+  M b;
+  int eb;
   from_mat<true>(u, b, eb, g);
+  R nb[9];
+#pragma unroll
+  for (int n = 0; n < 9; n++) nb[n] = neg(b.e[n].im);
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      Acc rr, ii, im;
-      entry_nn(a, i, b, j, rr, ii, im);
-      out.e[i + 3 * j].re = u.e[i + 3 * j].re + from_fixed(finish_diff(rr, ii), ea - kScale);
+      Acc re, im;
+      entry_nn(a, i, b, nb, j, re, im);
+      out.e[i + 3 * j].re = u.e[i + 3 * j].re + from_fixed(finish(re), ea - kScale);
       out.e[i + 3 * j].im = u.e[i + 3 * j].im + from_fixed(finish(im), ea - kScale);
     }
   return !g.bad;

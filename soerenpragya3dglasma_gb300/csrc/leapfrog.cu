@@ -61,23 +61,27 @@ __global__ void __launch_bounds__(kThreads, Occupancy<T>::kFusedMinBlocks)
 
 // The plaquette method (leapfrog_sites.cuh): K1' over the plaquette owners of slices -1 .. Nz-1,
 // K2' gathering the contributions into E before the link update.
-template <typename T, typename I, int R, typename TC>
+template <typename T, typename I, int R, typename TC, int kRoles = 1>
 __global__ void __launch_bounds__(kThreads, PlaqOccupancy<T, TC>::kMinBlocks)
     plaquette_kernel(const __grid_constant__ Geometry g, const __grid_constant__ FieldPtrs<T> f, T* __restrict__ C,
                      const __grid_constant__ EParams<T> p) {
-  __shared__ __align__(8) int sh[kPlaqShared<T, TC>];
-  const I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
-  if (idx >= (I)(g.plane * (g.nz + 1))) return;
-  plaquette_site<T, I, R, TC>(g, f, C, p, idx, sh);
+  __shared__ __align__(8) int sh[kPlaqShared<T, TC, kRoles>];
+  plaquette_block<T, I, R, TC, kRoles>(g, f, C, p, blockIdx.x, g.plane * (g.nz + 1), sh);
 }
 
-template <typename T, typename I, int R>
+// kSplit: three blocks per chunk of sites, one per link direction (a site's three links share nothing), the z links,
+// which have twice the work, first.
+template <typename T, typename I, int R, bool kSplit>
 __global__ void __launch_bounds__(kThreads, Occupancy<T>::kLinksMinBlocks)
     links_gather_kernel(const __grid_constant__ Geometry g, const __grid_constant__ FieldPtrs<T> f,
                         const T* __restrict__ C, const __grid_constant__ LParams<T> p) {
-  const I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
+  const unsigned chunk = kSplit ? blockIdx.x / 3u : blockIdx.x;
+  const I idx = (I)chunk * (I)kThreads + (I)threadIdx.x;
   if (idx >= (I)g.vol) return;
-  links_site<T, I, R, true>(g, f, p, idx, C);
+  if constexpr (kSplit)
+    link_site<T, I, R, true>(g, f, p, idx, 2 - (int)(blockIdx.x - 3u * chunk), C);
+  else
+    links_site<T, I, R, true>(g, f, p, idx, C);
 }
 
 template <typename T, typename I>
@@ -356,20 +360,37 @@ void launch_links_rows(const Geometry& g, FieldPtrs<T> f, const LParams<T>& p, c
     links_j_kernel<T, long long, R><<<grid_for(g.vol, kThreads), kThreads, 0, stream>>>(g, f, p);
 }
 
+// Small lattices: a site over four warps in the FP64 force kernel, its links over three blocks in the link kernel, as
+// long as all those blocks are resident at once (152 SMs).  Beyond that the split costs more than it hides (the warps'
+// code no longer stays in the instruction cache).  us per launch, together | split:
+//   force FP64   8x8x16 52 | 21   16x16x32 52 | 26   16x16x64 53 | 50   24x24x64 69 | 80
+//   links FP64   8x8x16 39 | 29   16x16x32 41 | 32   16x16x64 43 | 46   24x24x64 57 | 86
+//   links FP32   8x8x16 13 | 11   16x16x64 14 | 13   24x24x64 16 | 14   32x32x64 19 | 21
+constexpr long long kSms = 152;
+constexpr long long kRoleSites = kSms * PlaqOccupancy<double, double>::kMinBlocks * kFxSites<4>;
+template <typename T>
+constexpr long long kSplitSites = kSms * Occupancy<T>::kLinksMinBlocks * kThreads / 3;
+
 template <typename T, typename I, int R>
 void launch_plaquette_rows(const Geometry& g, FieldPtrs<T> f, T* C, const EParams<T>& pe, const LParams<T>& pl,
                            cudaStream_t stream, cudaEvent_t between, bool double_float) {
-  const unsigned grid = grid_for(g.plane * (g.nz + 1), kThreads);
+  const long long owners = g.plane * (g.nz + 1);
+  const unsigned grid = grid_for(owners, kThreads);
   if constexpr (sizeof(T) == 8) {
     if (double_float)
       plaquette_kernel<T, I, R, ddf><<<grid, kThreads, 0, stream>>>(g, f, C, pe);
+    else if (owners <= kRoleSites)
+      plaquette_kernel<T, I, R, T, 4><<<grid_for(owners, kFxSites<4>), kThreads, 0, stream>>>(g, f, C, pe);
     else
       plaquette_kernel<T, I, R, T><<<grid, kThreads, 0, stream>>>(g, f, C, pe);
   } else {
     plaquette_kernel<T, I, R, T><<<grid, kThreads, 0, stream>>>(g, f, C, pe);
   }
   if (between) cudaEventRecord(between, stream);
-  links_gather_kernel<T, I, R><<<grid_for(g.vol, kThreads), kThreads, 0, stream>>>(g, f, C, pl);
+  if (g.vol <= kSplitSites<T>)
+    links_gather_kernel<T, I, R, true><<<3 * grid_for(g.vol, kThreads), kThreads, 0, stream>>>(g, f, C, pl);
+  else
+    links_gather_kernel<T, I, R, false><<<grid_for(g.vol, kThreads), kThreads, 0, stream>>>(g, f, C, pl);
 }
 
 template <typename T>

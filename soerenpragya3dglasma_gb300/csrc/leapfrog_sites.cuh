@@ -28,8 +28,11 @@ __device__ __noinline__ void rotate_pair_fp64(const Mat<double>& V, const Alg<do
   else
     inv_adj_mul2(V, ep, em, out_p, out_m);
 }
-static __device__ __noinline__ void near_identity_fp64(const Mat<double>& Xm1, const Mat<double>& u, Mat<double>& out) {
-  mul_near_identity(Xm1, u, out);
+static __device__ __noinline__ void link_step_fp64(double c, const Alg<double>& e, const Mat<double>& u,
+                                                  Mat<double>& out) {
+  Mat<double> X;
+  link_exp(c, e, X);
+  mul_near_identity(X, u, out);
 }
 
 // out_p = V (t.ep) V^d, out_m = V (t.em) V^d (adj = true) or the V^d . V forms, paired where kPairCurrents, in FP64 on
@@ -62,24 +65,43 @@ __device__ __forceinline__ void rotate_currents(const Mat<T>& V, const Alg<T>& e
   }
 }
 
-// out = X u from X - 1: FP64 on the integer pipe, FP32 as mul_near_identity
+// The link update u -> exp(i c t.e) u: the exponential formed once, applied once or twice.  FP32 as mul_near_identity,
+// FP64 in fixed point on the integer pipe (fx.cuh), or in FP64 where that does not hold the numbers.
 template <typename T>
-__device__ __forceinline__ void link_apply(const Mat<T>& Xm1, const Mat<T>& u, Mat<T>& out) {
-  if constexpr (std::is_same<T, double>::value) {
-    if (!fx::add_product(Xm1, u, out)) {
-      const Mat<double> a = Xm1, b = u;
-      Mat<double> o;
-      near_identity_fp64(a, b, o);
-      out = o;
-    }
-  } else {
-    mul_near_identity(Xm1, u, out);
+struct LinkStep {
+  Mat<T> X;
+  __device__ __forceinline__ void set(T c, const Alg<T>& e) { link_exp(c, e, X); }
+  __device__ __forceinline__ void apply(const Mat<T>& u, Mat<T>& out) const { mul_near_identity(X, u, out); }
+};
+template <>
+struct LinkStep<double> {
+  fx::M X;
+  int ex;
+  bool ok;
+  double c;
+  Alg<double> e;
+  __device__ __forceinline__ void set(double c_, const Alg<double>& e_) {
+    c = c_;
+    e = e_;
+    ex = 0;
+    ok = fx::near_exp(c, e, X, ex);
   }
-}
+  __device__ __forceinline__ void apply(const Mat<double>& u, Mat<double>& out) const {
+    Mat<double> o;
+    if (!ok || !fx::add_product(X, ex, u, o)) {
+      const Mat<double> b = u;
+      const Alg<double> a = e;
+      link_step_fp64(c, a, b, o);
+    }
+    out = o;
+  }
+};
 
 // Blocks per SM the register allocation must leave room for (the register cap is 64K / (128 * n)),
 // chosen by measurement on GB300; overridable at build time for tuning sweeps.
-// (GB300 sweep, 128x128x512: FP32 K1 fastest at 5 blocks/SM, K2 at 8; FP64 is FP64-ALU bound.)
+// (GB300 sweep, 128x128x512: FP32 K1 fastest at 5 blocks/SM, K2 at 8; the staple kernels in FP64 are FP64-ALU bound.
+// The fixed-point kernels: force 10.7 ms at 3 blocks/SM, 12.3 at 2, 11.9 at 4; links 11.4 ms at 2 and at 3, 14 at 4, and
+// on 32x32x64 0.106 ms at 2, 0.130 at 3.)
 #ifndef GLASMA_FP64_MIN_BLOCKS
 #define GLASMA_FP64_MIN_BLOCKS 2
 #endif
@@ -98,6 +120,9 @@ __device__ __forceinline__ void link_apply(const Mat<T>& Xm1, const Mat<T>& u, M
 #ifndef GLASMA_DDF_PLAQ_MIN_BLOCKS
 #define GLASMA_DDF_PLAQ_MIN_BLOCKS 3
 #endif
+#ifndef GLASMA_FX_LINKS_MIN_BLOCKS
+#define GLASMA_FX_LINKS_MIN_BLOCKS 2
+#endif
 #ifndef GLASMA_FX_PLAQ_MIN_BLOCKS
 #define GLASMA_FX_PLAQ_MIN_BLOCKS 3
 #endif
@@ -106,7 +131,7 @@ struct Occupancy;
 template <>
 struct Occupancy<double> {
   static constexpr int kMinBlocks = GLASMA_FP64_MIN_BLOCKS;       // electric-field kernel
-  static constexpr int kLinksMinBlocks = GLASMA_FP64_MIN_BLOCKS;  // link/J kernel
+  static constexpr int kLinksMinBlocks = GLASMA_FX_LINKS_MIN_BLOCKS;  // link/J kernel
   static constexpr int kFusedMinBlocks = GLASMA_FP64_MIN_BLOCKS;  // one-pass step kernel
   static constexpr int kPlaqMinBlocks = GLASMA_FX_PLAQ_MIN_BLOCKS;  // plaquette-method force kernel
 };
@@ -506,17 +531,30 @@ __device__ __forceinline__ void plaquette_site_direct(const Geometry& g, const F
 }
 
 // plaquette_site for FP64 fields with the products on the integer pipe (fx.cuh).  Bound by FP64, the direct form
-// runs ~2000 FP64 operations per site; here they are ~5,000 mad.wide and as many integer operations, with ~200
-// FP64 ones beside them (the sums into E, the scaling of the contributions).  The plaquettes in a loop and the
-// four rotation pairs in a loop, so that the code stays inside the instruction cache (a straight-line body of
-// ~12,000 instructions does not); the three anti-Hermitian parts wait in shared memory for their rotations.
-// False, with neither E nor JStat written, where the fixed-point format does not hold the site's values.
-constexpr int kFxShared = 3 * 18 * kThreads + 3 * kThreads;  // ints of shared memory per block
-
+// runs ~2000 FP64 operations per site; here they are ~5,000 mad.wide and ~15,000 other integer operations, with ~300
+// FP64 ones beside them (the sums into E, conversions).  One copy of the plaquette and of the rotation in the code, so
+// that it stays inside the instruction cache; the three anti-Hermitian parts wait in shared memory for their rotations.
+// kRoles = 1: a thread does its site's three plaquettes and four rotation pairs in turn.  kRoles = 4: a block of four
+// warps does 32 sites, warp r plaquette r, rotation r and the sum into E_r (warp 3 the currents' rotation and JStat):
+// a third of the serial chain and four times the blocks, for lattices that do not fill the GPU (launch_plaquette_rows).
+// The arithmetic is the same either way.  Sites that the fixed-point format does not hold go through the FP64 form.
 template <typename I>
-__device__ __forceinline__ bool plaquette_site_fx(const Geometry& g, const FieldPtrs<double>& f, double* __restrict__ C,
-                                                  const EParams<double>& p, I idx, int* __restrict__ sh) {
+static __device__ __noinline__ void plaquette_site_fp64(const Geometry& g, const FieldPtrs<double>& f, double* C,
+                                                 const EParams<double>& p, I idx) {
+  plaquette_site_direct<double, I, 3>(g, f, C, p, idx);
+}
+
+template <int kRoles>
+constexpr int kFxSites = kThreads / kRoles;  // sites per block
+template <int kRoles>
+constexpr int kFxShared = (3 * 18 + 3 + (kRoles > 1 ? kRoles : 0)) * kFxSites<kRoles>;  // ints of shared memory per block
+
+template <typename I, int kRoles>
+__device__ __forceinline__ void plaquette_site_fx(const Geometry& g, const FieldPtrs<double>& f, double* __restrict__ C,
+                                                  const EParams<double>& p, I idx, bool active, int role,
+                                                  int* __restrict__ sh) {
   using fx::ll;
+  constexpr int kSites = kFxSites<kRoles>;
   const I S = (I)g.S, plane = (I)g.plane;
   const I s = idx;
   const int zz = (int)(idx / plane);
@@ -525,33 +563,34 @@ __device__ __forceinline__ bool plaquette_site_fx(const Geometry& g, const Field
   const int y = r / g.nx, x = r - y * g.nx;
   const bool interior = z >= 0;
   const bool below_top = z < g.nz - 1;
-  const I sxp = nb<I>(g, x, y, z, 1, 0, 0), syp = nb<I>(g, x, y, z, 0, 1, 0), szp = s + plane;
-  ll* const slot = reinterpret_cast<ll*>(sh) + threadIdx.x;  // number w of plane n: slot[(n * 9 + w) * kThreads]
-  int* const slot_e = sh + 3 * 18 * kThreads + threadIdx.x;
+  const int site = kRoles == 1 ? threadIdx.x : threadIdx.x % kSites;
+  ll* const slot = reinterpret_cast<ll*>(sh) + site;  // number w of plane n: slot[(n * 9 + w) * kSites]
+  int* const slot_e = sh + 3 * 18 * kSites + site;
+  int* const flag = slot_e + 3 * kSites;  // kRoles > 1: role r's guard
   auto put = [&](int n, const fx::Anti& a) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      slot[(n * 9 + k) * kThreads] = a.y[k];
-      slot[(n * 9 + 3 + k) * kThreads] = a.x[k];
-      slot[(n * 9 + 6 + k) * kThreads] = a.d[k];
+      slot[(n * 9 + k) * kSites] = a.y[k];
+      slot[(n * 9 + 3 + k) * kSites] = a.x[k];
+      slot[(n * 9 + 6 + k) * kSites] = a.d[k];
     }
-    slot_e[n * kThreads] = a.e;
+    slot_e[n * kSites] = a.e;
   };
   auto get = [&](int n, fx::Anti& a) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      a.y[k] = slot[(n * 9 + k) * kThreads];
-      a.x[k] = slot[(n * 9 + 3 + k) * kThreads];
-      a.d[k] = slot[(n * 9 + 6 + k) * kThreads];
+      a.y[k] = slot[(n * 9 + k) * kSites];
+      a.x[k] = slot[(n * 9 + 3 + k) * kSites];
+      a.d[k] = slot[(n * 9 + 6 + k) * kSites];
     }
-    a.e = slot_e[n * kThreads];
+    a.e = slot_e[n * kSites];
   };
   fx::Guard guard = fx::guard_init();
   // planes 0: (0,1), 1: (0,2), 2: (1,2); the ghost slice -1 owns only those with z
-#pragma unroll 1
-  for (int n = interior ? 0 : 1; n < 3; n++) {
+  auto plaquette = [&](int n) {
     const int mp = n == 2 ? 1 : 0, mq = n == 0 ? 1 : 2;
-    const I sp = n == 2 ? syp : sxp, sq = n == 0 ? syp : szp;
+    const I sp = n == 2 ? nb<I>(g, x, y, z, 0, 1, 0) : nb<I>(g, x, y, z, 1, 0, 0);
+    const I sq = n == 0 ? nb<I>(g, x, y, z, 0, 1, 0) : s + plane;
     fx::M a, b, w, v;
     int ea, eb, ew, ev;
     fx::link_near(f.U, S, mp, s, a, ea, guard);
@@ -563,14 +602,10 @@ __device__ __forceinline__ bool plaquette_site_fx(const Geometry& g, const Field
     fx::Anti al;
     fx::plaquette_parts(w, ew, v, ev, al);
     put(n, al);
-  }
+  };
   // rotations: 0 by u2 (al02, al12), 1 by u1 (al01, al12), 2 by u0 (al01, al02), 3 the currents below by U_2(y-z)
-  const double w01p = p.gc[0] * p.cnu[1], w01q = p.gc[1] * p.cnu[0];
-  const double w02p = p.gc[0] * p.cnu[2], w02q = p.gc[2] * p.cnu[0];
-  const double w12p = p.gc[1] * p.cnu[2], w12q = p.gc[2] * p.cnu[1];
   Alg<double> down, downm;
-#pragma unroll 1
-  for (int n = below_top ? 0 : 1; n < (interior ? 4 : 1); n++) {
+  auto rotation = [&](int n) {
     fx::M v, m;
     int e;
     ll tr_re, tr_im, o1[8], o2[8];
@@ -590,37 +625,46 @@ __device__ __forceinline__ bool plaquette_site_fx(const Geometry& g, const Field
     if (n < 3) {
       const int k1 = n == 0 ? kC02q : (n == 1 ? kC01q : kC01p), k2 = n == 0 ? kC12q : (n == 1 ? kC12p : kC02p);
       Alg<double> out, out2;
-      fx::to_alg(o1, e - fx::kScale - 2, -1.0, out);
-      fx::to_alg(o2, e - fx::kScale - 2, -1.0, out2);
+      fx::to_alg<true>(o1, e - fx::kScale - 2, -1.0, out);
+      fx::to_alg<true>(o2, e - fx::kScale - 2, -1.0, out2);
       if (!p.dry) {
         store_alg(C, S, k1 * 8, s, out);
         store_alg(C, S, k2 * 8, s, out2);
       }
     } else {
-      fx::to_alg(o1, e - fx::kScale - 1, 1.0, down);
-      fx::to_alg(o2, e - fx::kScale - 1, 1.0, downm);
+      fx::to_alg<true>(o1, e - fx::kScale - 1, 1.0, down);
+      fx::to_alg<true>(o2, e - fx::kScale - 1, 1.0, downm);
     }
-  }
-  if (fx::tripped(guard)) return false;
-  if (!interior) return true;
-  // E += the forces of the plaquettes owned here (+ the current source on E_z)
-#pragma unroll 1
-  for (int mu = 0; mu < 3; mu++) {
-    // link 0: +w01p al01 + w02p al02; link 1: -w01q al01 + w12p al12; link 2: -w02q al02 - w12q al12
-    const int n1 = mu == 2 ? 1 : 0, n2 = mu == 0 ? 1 : 2;
-    fx::Anti a1, a2;
-    get(n1, a1);
-    get(n2, a2);
-    const double c1 = -0.5 * (mu == 0 ? w01p : (mu == 1 ? -w01q : -w02q));
-    const double c2 = -0.5 * (mu == 0 ? w02p : (mu == 1 ? w12p : -w12q));
-    Alg<double> e, F;
-    load_alg(f.E, S, mu * 8, s, e);
+  };
+  // -2 al of plane n as doubles; with one role they then wait in the place of the fixed-point form, for two links
+  auto convert = [&](int n, Alg<double>& v) {
+    fx::Anti a;
+    get(n, a);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const double q = k == 7 ? Consts<double>::inv_sqrt3() : 1.0;
-      F.a[k] = fma(fx::from_fixed(fx::component(a2, k), a2.e - fx::kScale), c2 * q,
-                   fx::from_fixed(fx::component(a1, k), a1.e - fx::kScale) * (c1 * q));
+    for (int k = 0; k < 8; k++) v.a[k] = fx::from_fixed_fp64(fx::component(a, k), a.e - fx::kScale);
+    v.a[7] *= Consts<double>::inv_sqrt3();
+  };
+  auto alg = [&](int n, Alg<double>& v) {
+    if constexpr (kRoles == 1) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) v.a[k] = __longlong_as_double(slot[(n * 9 + k) * kSites]);
+    } else {
+      convert(n, v);
     }
+  };
+  // E_mu += the forces of the plaquettes owned here (+ the current source on E_z)
+  auto efield = [&](int mu) {
+    // link 0: +w01p al01 + w02p al02; link 1: -w01q al01 + w12p al12; link 2: -w02q al02 - w12q al12
+    // (w_pq p = gc_p c_q, q = gc_q c_p)
+    const int n1 = mu == 2 ? 1 : 0, n2 = mu == 0 ? 1 : 2;
+    const double c1 = -0.5 * (mu == 0 ? p.gc[0] * p.cnu[1] : (mu == 1 ? -(p.gc[1] * p.cnu[0]) : -(p.gc[2] * p.cnu[0])));
+    const double c2 = -0.5 * (mu == 0 ? p.gc[0] * p.cnu[2] : (mu == 1 ? p.gc[1] * p.cnu[2] : -(p.gc[2] * p.cnu[1])));
+    Alg<double> e, F, v1, v2;
+    load_alg(f.E, S, mu * 8, s, e);
+    alg(n1, v1);
+    alg(n2, v2);
+#pragma unroll
+    for (int k = 0; k < 8; k++) F.a[k] = fma(v2.a[k], c2, v1.a[k] * c1);
     if (mu == 2) {
       Alg<double> jp, jm;
       load_alg(f.Jp, S, 0, s, jp);
@@ -631,46 +675,85 @@ __device__ __forceinline__ bool plaquette_site_fx(const Geometry& g, const Field
 #pragma unroll
     for (int k = 0; k < 8; k++) e.a[k] += F.a[k];
     if (!p.dry) store_alg(f.E, S, mu * 8, s, e);
+  };
+  auto jstat = [&]() {  // UpdateJStat, as K1
+    const bool lo = (z == 0), hi = (z == g.nz - 1);
+    const I sg = lo ? s - plane : (hi ? s + plane : (I)-1);
+    Alg<double> jc, st;
+    load_alg(f.Jp, S, 0, s, jc);
+    load_alg(f.JpStat, S, 0, s, st);
+    axpy_diff(st, -p.cj, jc, down);
+    if (!p.dry) {
+      store_alg(f.JpStat, S, 0, s, st);
+      if (sg >= 0) store_alg(f.JpStat, S, 0, sg, st);
+    }
+    load_alg(f.Jm, S, 0, s, jc);
+    load_alg(f.JmStat, S, 0, s, st);
+    axpy_diff(st, p.cj, jc, downm);
+    if (!p.dry) {
+      store_alg(f.JmStat, S, 0, s, st);
+      if (sg >= 0) store_alg(f.JmStat, S, 0, sg, st);
+    }
+  };
+  // Neither E nor JStat is written before every guard of the site is known.
+  if constexpr (kRoles == 1) {
+    if (!active) return;
+#pragma unroll 1
+    for (int n = interior ? 0 : 1; n < 3; n++) plaquette(n);
+#pragma unroll 1
+    for (int n = below_top ? 0 : 1; n < (interior ? 4 : 1); n++) rotation(n);
+    if (fx::tripped(guard)) {
+      plaquette_site_fp64<I>(g, f, C, p, idx);
+      return;
+    }
+    if (!interior) return;
+#pragma unroll 1
+    for (int n = 0; n < 3; n++) {
+      Alg<double> v;
+      convert(n, v);
+#pragma unroll
+      for (int k = 0; k < 8; k++) slot[(n * 9 + k) * kSites] = __double_as_longlong(v.a[k]);
+    }
+#pragma unroll 1
+    for (int mu = 0; mu < 3; mu++) efield(mu);
+    jstat();
+  } else {
+    if (active && role < 3 && (interior || role > 0)) plaquette(role);
+    __syncthreads();
+    // role 3's rotation reads no plaquette; it waits here only so that the rotation is in the code once
+    if (active && (role == 0 ? below_top : interior)) rotation(role);
+    flag[role * kSites] = active && fx::tripped(guard);
+    __syncthreads();
+    if (!active) return;
+    if (flag[0] | flag[kSites] | flag[2 * kSites] | flag[3 * kSites]) {
+      if (role == 0) plaquette_site_fp64<I>(g, f, C, p, idx);
+      return;
+    }
+    if (!interior) return;
+    if (role < 3)
+      efield(role);
+    else
+      jstat();
   }
-  // UpdateJStat, as K1
-  const bool lo = (z == 0), hi = (z == g.nz - 1);
-  const I sg = lo ? s - plane : (hi ? s + plane : (I)-1);
-  Alg<double> jc, st;
-  load_alg(f.Jp, S, 0, s, jc);
-  load_alg(f.JpStat, S, 0, s, st);
-  axpy_diff(st, -p.cj, jc, down);
-  if (!p.dry) {
-    store_alg(f.JpStat, S, 0, s, st);
-    if (sg >= 0) store_alg(f.JpStat, S, 0, sg, st);
-  }
-  load_alg(f.Jm, S, 0, s, jc);
-  load_alg(f.JmStat, S, 0, s, st);
-  axpy_diff(st, p.cj, jc, downm);
-  if (!p.dry) {
-    store_alg(f.JmStat, S, 0, s, st);
-    if (sg >= 0) store_alg(f.JmStat, S, 0, sg, st);
-  }
-  return true;
-}
-
-// Out of line: the sites that the fixed-point form hands back.
-template <typename I>
-__device__ __noinline__ void plaquette_site_fp64(const Geometry& g, const FieldPtrs<double>& f, double* C,
-                                                 const EParams<double>& p, I idx) {
-  plaquette_site_direct<double, I, 3>(g, f, C, p, idx);
 }
 
 // Ints of shared memory the force kernel of type T, TC needs per block.
-template <typename T, typename TC>
-constexpr int kPlaqShared = (std::is_same<T, double>::value && std::is_same<TC, double>::value) ? kFxShared : 2;
+template <typename T, typename TC, int kRoles>
+constexpr int kPlaqShared = (std::is_same<T, double>::value && std::is_same<TC, double>::value) ? kFxShared<kRoles> : 2;
 
-template <typename T, typename I, int R, typename TC = T>
-__device__ __forceinline__ void plaquette_site(const Geometry& g, const FieldPtrs<T>& f, T* __restrict__ C,
-                                               const EParams<T>& p, I idx, int* sh) {
+// One block of the force kernel over n owner sites, block b.
+template <typename T, typename I, int R, typename TC, int kRoles = 1>
+__device__ __forceinline__ void plaquette_block(const Geometry& g, const FieldPtrs<T>& f, T* __restrict__ C,
+                                                const EParams<T>& p, long long b, long long n, int* sh) {
   if constexpr (std::is_same<T, double>::value && std::is_same<TC, double>::value) {
-    if (!plaquette_site_fx<I>(g, f, C, p, idx, sh)) plaquette_site_fp64<I>(g, f, C, p, idx);
+    constexpr int kSites = kFxSites<kRoles>;
+    const long long idx = b * kSites + threadIdx.x % kSites;
+    // the roles move on by one from block to block, so that no scheduler gets the lighter one every time
+    const int role = kRoles == 1 ? 0 : (int)((threadIdx.x / kSites + b) % kRoles);
+    plaquette_site_fx<I, kRoles>(g, f, C, p, (I)(idx < n ? idx : 0), idx < n, role, sh);
   } else {
-    plaquette_site_direct<T, I, R, TC>(g, f, C, p, idx);
+    const long long idx = b * kThreads + threadIdx.x;
+    if (idx < n) plaquette_site_direct<T, I, R, TC>(g, f, C, p, (I)idx);
   }
 }
 
@@ -737,12 +820,42 @@ inline void set_gather_weights(const Geometry& g, double dt, LParams<T>& p) {
   p.wb[2] = gc[2] * c[1];
 }
 
-// K2's per-site body: links to t+dt (two applications of one exp), UOld, J transport.  kGather (the
-// plaquette method): first E_mu += the two contributions link mu receives from the plaquette owners
+// UpdateJ at s with the z link uh of t + dt/2.
+template <typename T, typename I>
+__device__ __forceinline__ void transport_currents(const FieldPtrs<T>& f, const LParams<T>& p, I S, I s, I szp, I sg,
+                                                   const Mat<T>& uh) {
+  Alg<T> up, um, st, j;
+  load_alg(f.JpStat, S, 0, szp, st);
+  if constexpr (kPairCurrents<T>) {
+    load_alg(f.JmStat, S, 0, szp, j);
+    rotate_currents<T, true>(uh, st, j, up, um);
+  } else {
+    adj_mul(uh, st, up);
+  }
+  load_alg(f.JpStat, S, 0, s, st);
+  load_alg(f.Jp, S, 0, s, j);
+  axpy_diff(j, -p.cj, up, st);
+  store_alg(f.Jp, S, 0, s, j);
+  if (sg >= 0) store_alg(f.Jp, S, 0, sg, j);
+  if constexpr (kPairCurrents<T>) {
+    up = um;
+  } else {
+    load_alg(f.JmStat, S, 0, szp, st);
+    adj_mul(uh, st, up);
+  }
+  load_alg(f.JmStat, S, 0, s, st);
+  load_alg(f.Jm, S, 0, s, j);
+  axpy_diff(j, p.cj, up, st);
+  store_alg(f.Jm, S, 0, s, j);
+  if (sg >= 0) store_alg(f.Jm, S, 0, sg, j);
+}
+
+// K2's body for link mu of one site: the link to t+dt (two applications of one exp), UOld, J transport (mu = 2).
+// kGather (the plaquette method): first E_mu += the two contributions link mu receives from the plaquette owners
 // x-nu (see plaquette_site), stored with its ghost copy.
 template <typename T, typename I, int R = 3, bool kGather = false>
-__device__ __forceinline__ void links_site(const Geometry& g, const FieldPtrs<T>& f, const LParams<T>& p, I idx,
-                                           const T* __restrict__ C = nullptr) {
+__device__ __forceinline__ void link_site(const Geometry& g, const FieldPtrs<T>& f, const LParams<T>& p, I idx,
+                                           const int mu, const T* __restrict__ C = nullptr) {
   const I S = (I)g.S, plane = (I)g.plane;
   const I s = idx + plane;
   const int z = (int)(idx / plane);
@@ -755,77 +868,82 @@ __device__ __forceinline__ void links_site(const Geometry& g, const FieldPtrs<T>
     sxm = nb<I>(g, x, y, z, -1, 0, 0);
     sym = nb<I>(g, x, y, z, 0, -1, 0);
   }
-#pragma unroll 1
-  for (int mu = 0; mu < 3; mu++) {
-    Alg<T> e;
-    load_alg(f.E, S, mu * 8, s, e);
-    if constexpr (kGather) {
-      // link 0: from (0,1) at x-y and (0,2) at x-z; link 1: (0,1) at x-x, (1,2) at x-z;
-      // link 2: (0,2) at x-x, (1,2) at x-y
-      const I s1 = mu == 0 ? sym : sxm;
-      const I s2 = mu == 2 ? sym : s - plane;
-      const int c1 = mu == 0 ? kC01q : (mu == 1 ? kC01p : kC02p);
-      const int c2 = mu == 0 ? kC02q : (mu == 1 ? kC12q : kC12p);
-      Alg<T> a1, a2;
-      load_alg(C, S, c1 * 8, s1, a1);
-      load_alg(C, S, c2 * 8, s2, a2);
+  Alg<T> e;
+  load_alg(f.E, S, mu * 8, s, e);
+  if constexpr (kGather) {
+    // link 0: from (0,1) at x-y and (0,2) at x-z; link 1: (0,1) at x-x, (1,2) at x-z;
+    // link 2: (0,2) at x-x, (1,2) at x-y
+    const I s1 = mu == 0 ? sym : sxm;
+    const I s2 = mu == 2 ? sym : s - plane;
+    const int c1 = mu == 0 ? kC01q : (mu == 1 ? kC01p : kC02p);
+    const int c2 = mu == 0 ? kC02q : (mu == 1 ? kC12q : kC12p);
+    Alg<T> a1, a2;
+    load_alg(C, S, c1 * 8, s1, a1);
+    load_alg(C, S, c2 * 8, s2, a2);
 #pragma unroll
-      for (int k = 0; k < 8; k++) e.a[k] += fma(pick3(p.wa, mu), a1.a[k], pick3(p.wb, mu) * a2.a[k]);
-      store_alg(f.E, S, mu * 8, s, e);
-      if (sg >= 0) store_alg(f.E, S, mu * 8, sg, e);
-    }
-    Mat<T> X, u, uh;
-    load_link_r<R>(f.U, S, mu, s, u);
-    // Without a use for U(t+dt/2) (UOld, the z-link J transport), the two half steps are one:
-    // exp(i c t.E)^2 = exp(2i c t.E), one matmul less (equal up to rounding).
-    if (p.do_second && !p.save_uold && !(mu == 2 && p.do_j)) {
-      link_exp(T(2) * pick3(p.cU, mu), e, X);
-      link_apply(X, u, uh);
-      store_link_r<R>(f.U, S, mu, s, uh);
-      if (sg >= 0) store_link_r<R>(f.U, S, mu, sg, uh);
-      continue;
-    }
-    link_exp(pick3(p.cU, mu), e, X);
-    link_apply(X, u, uh);
-    if (p.save_uold) {
-      store_link(f.UOld, S, mu, s, uh);
-      if (sg >= 0) store_link(f.UOld, S, mu, sg, uh);
-    }
-    if (mu == 2 && p.do_j) {
-      Alg<T> up, um, st, j;
-      const I szp = s + plane;
-      load_alg(f.JpStat, S, 0, szp, st);
-      if constexpr (kPairCurrents<T>) {
-        load_alg(f.JmStat, S, 0, szp, j);
-        rotate_currents<T, true>(uh, st, j, up, um);
-      } else {
-        adj_mul(uh, st, up);
-      }
-      load_alg(f.JpStat, S, 0, s, st);
-      load_alg(f.Jp, S, 0, s, j);
-      axpy_diff(j, -p.cj, up, st);
-      store_alg(f.Jp, S, 0, s, j);
-      if (sg >= 0) store_alg(f.Jp, S, 0, sg, j);
-      if constexpr (kPairCurrents<T>) {
-        up = um;
-      } else {
-        load_alg(f.JmStat, S, 0, szp, st);
-        adj_mul(uh, st, up);
-      }
-      load_alg(f.JmStat, S, 0, s, st);
-      load_alg(f.Jm, S, 0, s, j);
-      axpy_diff(j, p.cj, up, st);
-      store_alg(f.Jm, S, 0, s, j);
-      if (sg >= 0) store_alg(f.Jm, S, 0, sg, j);
-    }
-    if (p.do_second) {
-      link_apply(X, uh, u);
-    } else {
-      u = uh;
-    }
-    store_link_r<R>(f.U, S, mu, s, u);
-    if (sg >= 0) store_link_r<R>(f.U, S, mu, sg, u);
+    for (int k = 0; k < 8; k++) e.a[k] += fma(pick3(p.wa, mu), a1.a[k], pick3(p.wb, mu) * a2.a[k]);
+    store_alg(f.E, S, mu * 8, s, e);
+    if (sg >= 0) store_alg(f.E, S, mu * 8, sg, e);
   }
+  if constexpr (std::is_same<T, double>::value) {
+    // One copy of the product and of the current transport in the code, run once or twice per link: written out
+    // (three products, two exponentials) the fixed-point body overflowed the instruction cache (5.6 fetch stalls
+    // per issue, 14.3 ms at 128x128x512).
+    const bool doubled = p.do_second && !p.save_uold && !(mu == 2 && p.do_j);
+    LinkStep<double> X;
+    X.set(doubled ? 2.0 * pick3(p.cU, mu) : pick3(p.cU, mu), e);
+    Mat<double> u;
+    load_link(f.U, S, mu, s, u);
+    const int napply = (doubled || !p.do_second) ? 1 : 2;
+#pragma unroll 1
+    for (int ap = 0; ap < napply; ap++) {
+      X.apply(u, u);
+      if (ap == 0 && !doubled) {
+        if (p.save_uold) {
+          store_link(f.UOld, S, mu, s, u);
+          if (sg >= 0) store_link(f.UOld, S, mu, sg, u);
+        }
+        if (mu == 2 && p.do_j) transport_currents<double, I>(f, p, S, s, s + plane, sg, u);
+      }
+    }
+    store_link(f.U, S, mu, s, u);
+    if (sg >= 0) store_link(f.U, S, mu, sg, u);
+    return;
+  }
+  LinkStep<T> X;
+  Mat<T> u, uh;
+  load_link_r<R>(f.U, S, mu, s, u);
+  // Without a use for U(t+dt/2) (UOld, the z-link J transport), the two half steps are one:
+  // exp(i c t.E)^2 = exp(2i c t.E), one matmul less (equal up to rounding).
+  if (p.do_second && !p.save_uold && !(mu == 2 && p.do_j)) {
+    X.set(T(2) * pick3(p.cU, mu), e);
+    X.apply(u, uh);
+    store_link_r<R>(f.U, S, mu, s, uh);
+    if (sg >= 0) store_link_r<R>(f.U, S, mu, sg, uh);
+    return;
+  }
+  X.set(pick3(p.cU, mu), e);
+  X.apply(u, uh);
+  if (p.save_uold) {
+    store_link(f.UOld, S, mu, s, uh);
+    if (sg >= 0) store_link(f.UOld, S, mu, sg, uh);
+  }
+  if (mu == 2 && p.do_j) transport_currents<T, I>(f, p, S, s, s + plane, sg, uh);
+  if (p.do_second) {
+    X.apply(uh, u);
+  } else {
+    u = uh;
+  }
+  store_link_r<R>(f.U, S, mu, s, u);
+  if (sg >= 0) store_link_r<R>(f.U, S, mu, sg, u);
+}
+
+// K2 over the three links of a site in turn.
+template <typename T, typename I, int R = 3, bool kGather = false>
+__device__ __forceinline__ void links_site(const Geometry& g, const FieldPtrs<T>& f, const LParams<T>& p, I idx,
+                                           const T* __restrict__ C = nullptr) {
+#pragma unroll 1
+  for (int mu = 0; mu < 3; mu++) link_site<T, I, R, kGather>(g, f, p, idx, mu, C);
 }
 
 // ---- the whole step in one pass -------------------------------------------------------------------
@@ -943,23 +1061,24 @@ __device__ __forceinline__ void fused_site(const Geometry& g, const FieldPtrs<T>
       store_alg(in.E, S, mu * 8, s, e);
       if (sg >= 0) store_alg(in.E, S, mu * 8, sg, e);
     }
-    Mat<T> X, uh;
+    LinkStep<T> X;
+    Mat<T> uh;
     if (!pl.save_uold && mu != 2) {  // one exp at twice the angle, as in links_site
-      link_exp(T(2) * pick3(pl.cU, mu), e, X);
-      link_apply(X, u, w);
+      X.set(T(2) * pick3(pl.cU, mu), e);
+      X.apply(u, w);
       if (!dry) {
         store_link_r<R>(out.U, S, mu, s, w);
         if (sg >= 0) store_link_r<R>(out.U, S, mu, sg, w);
       }
       continue;
     }
-    link_exp(pick3(pl.cU, mu), e, X);
-    link_apply(X, u, uh);
+    X.set(pick3(pl.cU, mu), e);
+    X.apply(u, uh);
     if (pl.save_uold && !dry) {
       store_link(in.UOld, S, mu, s, uh);
       if (sg >= 0) store_link(in.UOld, S, mu, sg, uh);
     }
-    link_apply(X, uh, w);
+    X.apply(uh, w);
     if (!dry) {
       store_link_r<R>(out.U, S, mu, s, w);
       if (sg >= 0) store_link_r<R>(out.U, S, mu, sg, w);

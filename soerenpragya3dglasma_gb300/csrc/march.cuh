@@ -327,13 +327,14 @@ __global__ void __launch_bounds__(kMarchThreads, MarchOccupancy<T>::kMinBlocks)
         // the links: one exponential at twice the angle where U(t+dt/2) has no use, else two half steps
         // with SaveOldLink and UpdateJ between them
         const bool doubled = pl.do_second && !pl.save_uold && !(mu == 2 && pl.do_j);
-        Mat<T> X, u, w;
+        LinkStep<T> X;
+        Mat<T> u, w;
         load_link_r<R>(in.U, S, mu, s, u);
-        link_exp(doubled ? T(2) * pick3(pl.cU, mu) : pick3(pl.cU, mu), e, X);
+        X.set(doubled ? T(2) * pick3(pl.cU, mu) : pick3(pl.cU, mu), e);
         const int napply = (doubled || !pl.do_second) ? 1 : 2;
 #pragma unroll 1
         for (int ap = 0; ap < napply; ap++) {
-          link_apply(X, u, w);
+          X.apply(u, w);
           u = w;
           if (ap == 0 && !doubled) {
             if (pl.save_uold) {

@@ -454,35 +454,9 @@ struct Trig<float> {
   static __device__ __forceinline__ float taylor_c1() { return 1e-3f; }
 };
 
-// X = exp(i c t^a al^a), Cayley-Hamilton form exp(iQ) = f0 + f1 Q + f2 Q^2.  kMinusOne: X - 1
-// instead, with f0 - 1 formed directly (expi_m1 below).
-template <typename T, bool kMinusOne = false>
-__device__ __forceinline__ void expi_impl(T c, const Alg<T>& al, Mat<T>& X) {
-  Alg<T> sc;
-#pragma unroll
-  for (int a = 0; a < 8; a++) sc.a[a] = c * al.a[a];
-  Mat<T> Q, Q2;
-  herm_from_alg(sc, Q);
-  // Q^2 of a traceless Hermitian Q: the off-diagonal entries as -Q_kk Q_ij + Q_ik Q_kj, the diagonal from the
-  // moduli, the lower triangle by conjugation
-  const T q0 = Q.e[0].re, q1 = Q.e[4].re, q2 = Q.e[8].re;
-  const cx<T> a01 = Q.e[3], a02 = Q.e[6], a12 = Q.e[7];
-  const T m01 = fma(a01.re, a01.re, a01.im * a01.im), m02 = fma(a02.re, a02.re, a02.im * a02.im),
-          m12 = fma(a12.re, a12.re, a12.im * a12.im);
-  Q2.e[3] = mk<T>(fma(-q2, a01.re, fma(a02.re, a12.re, a02.im * a12.im)),   // Q02 conj(Q12)
-                  fma(-q2, a01.im, fma(a02.im, a12.re, -(a02.re * a12.im))));
-  Q2.e[6] = mk<T>(fma(-q1, a02.re, fma(a01.re, a12.re, -(a01.im * a12.im))),  // Q01 Q12
-                  fma(-q1, a02.im, fma(a01.re, a12.im, a01.im * a12.re)));
-  Q2.e[7] = mk<T>(fma(-q0, a12.re, fma(a01.re, a02.re, a01.im * a02.im)),   // conj(Q01) Q02
-                  fma(-q0, a12.im, fma(a01.re, a02.im, -(a01.im * a02.re))));
-  Q2.e[0] = mk<T>(fma(q0, q0, m01 + m02), T(0));
-  Q2.e[4] = mk<T>(fma(q1, q1, m01 + m12), T(0));
-  Q2.e[8] = mk<T>(fma(q2, q2, m02 + m12), T(0));
-  const T c1 = T(0.5) * (Q2.e[0].re + Q2.e[4].re + Q2.e[8].re);
-  // det Q = q0 q1 q2 + 2 Re(Q01 Q12 conj(Q02)) - q0 |Q12|^2 - q1 |Q02|^2 - q2 |Q01|^2, real
-  const T t01 = fma(a01.re, a12.re, -(a01.im * a12.im)), t12 = fma(a01.re, a12.im, a01.im * a12.re);
-  const T c0 = fma(q0, fma(q1, q2, -m12), fma(T(2), fma(t01, a02.re, t12 * a02.im), -fma(q1, m02, q2 * m01)));
-  cx<T> f0, f1, f2;
+// The coefficients of exp(iQ) = f0 + f1 Q + f2 Q^2 from c0 = det Q, c1 = tr Q^2 / 2; kMinusOne: f0 - 1 in f0's place.
+template <typename T, bool kMinusOne>
+__device__ __forceinline__ void exp_coeff(T c0, T c1, cx<T>& f0, cx<T>& f1, cx<T>& f2) {
   if (sizeof(T) == 8 && c1 >= Trig<T>::taylor_c1() && c1 < T(0.5)) {
     // FP64 without transcendental functions (they cost ~60 % of this exponential on GB300's FP64 pipe):
     // exp(iQ) = sum_n i^n Q^n / n!, and by Cayley-Hamilton (Q^3 = c1 Q + c0) Q^n / n! = a_n + b_n Q + d_n
@@ -582,6 +556,38 @@ __device__ __forceinline__ void expi_impl(T c, const Alg<T>& al, Mat<T>& X) {
     }
     if (kMinusOne) f0.re -= T(1);
   }
+}
+
+// X = exp(i c t^a al^a), Cayley-Hamilton form exp(iQ) = f0 + f1 Q + f2 Q^2.  kMinusOne: X - 1
+// instead, with f0 - 1 formed directly (expi_m1 below).
+template <typename T, bool kMinusOne = false>
+__device__ __forceinline__ void expi_impl(T c, const Alg<T>& al, Mat<T>& X) {
+  Alg<T> sc;
+#pragma unroll
+  for (int a = 0; a < 8; a++) sc.a[a] = c * al.a[a];
+  Mat<T> Q, Q2;
+  herm_from_alg(sc, Q);
+  // Q^2 of a traceless Hermitian Q: the off-diagonal entries as -Q_kk Q_ij + Q_ik Q_kj, the diagonal from the
+  // moduli, the lower triangle by conjugation
+  const T q0 = Q.e[0].re, q1 = Q.e[4].re, q2 = Q.e[8].re;
+  const cx<T> a01 = Q.e[3], a02 = Q.e[6], a12 = Q.e[7];
+  const T m01 = fma(a01.re, a01.re, a01.im * a01.im), m02 = fma(a02.re, a02.re, a02.im * a02.im),
+          m12 = fma(a12.re, a12.re, a12.im * a12.im);
+  Q2.e[3] = mk<T>(fma(-q2, a01.re, fma(a02.re, a12.re, a02.im * a12.im)),   // Q02 conj(Q12)
+                  fma(-q2, a01.im, fma(a02.im, a12.re, -(a02.re * a12.im))));
+  Q2.e[6] = mk<T>(fma(-q1, a02.re, fma(a01.re, a12.re, -(a01.im * a12.im))),  // Q01 Q12
+                  fma(-q1, a02.im, fma(a01.re, a12.im, a01.im * a12.re)));
+  Q2.e[7] = mk<T>(fma(-q0, a12.re, fma(a01.re, a02.re, a01.im * a02.im)),   // conj(Q01) Q02
+                  fma(-q0, a12.im, fma(a01.re, a02.im, -(a01.im * a02.re))));
+  Q2.e[0] = mk<T>(fma(q0, q0, m01 + m02), T(0));
+  Q2.e[4] = mk<T>(fma(q1, q1, m01 + m12), T(0));
+  Q2.e[8] = mk<T>(fma(q2, q2, m02 + m12), T(0));
+  const T c1 = T(0.5) * (Q2.e[0].re + Q2.e[4].re + Q2.e[8].re);
+  // det Q = q0 q1 q2 + 2 Re(Q01 Q12 conj(Q02)) - q0 |Q12|^2 - q1 |Q02|^2 - q2 |Q01|^2, real
+  const T t01 = fma(a01.re, a12.re, -(a01.im * a12.im)), t12 = fma(a01.re, a12.im, a01.im * a12.re);
+  const T c0 = fma(q0, fma(q1, q2, -m12), fma(T(2), fma(t01, a02.re, t12 * a02.im), -fma(q1, m02, q2 * m01)));
+  cx<T> f0, f1, f2;
+  exp_coeff<T, kMinusOne>(c0, c1, f0, f1, f2);
   // f1 Q + f2 Q^2, entries (i,j) and (j,i) from the same products: with r = f1r Q.re + f2r Q2.re, s = f1i Q.im +
   // f2i Q2.im, t = f1r Q.im + f2r Q2.im, u = f1i Q.re + f2i Q2.re at (i,j) they are (r - s, u + t) and (r + s, u - t)
   constexpr int up[3] = {3, 6, 7}, low[3] = {1, 2, 5};
