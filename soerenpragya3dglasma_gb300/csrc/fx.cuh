@@ -105,21 +105,32 @@ __device__ __forceinline__ Guard guard_init() {
 // shift(k): what the conversions take for a scale of 2^k
 __device__ __forceinline__ int shift(int k) { return 1083 - k; }
 // |v| 2^k, truncated; |v| 2^k < 2^62 (larger values give garbage, never a fault)
+__device__ __forceinline__ ll shifted(unsigned long long m, int by) {
+  ll q;
+  asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(by));  // clamps: zero beyond 63
+  return q;
+}
 __device__ __forceinline__ ll magnitude(double v, int sh) {
   const int h = __double2hiint(v);
   const unsigned long long m =
       ((unsigned long long)((h & 0xfffff) | 0x100000) << 40) | ((unsigned long long)(unsigned)__double2loint(v) << 8);
-  ll q;
-  asm("shr.u64 %0, %1, %2;" : "=l"(q) : "l"(m), "r"(sh - ((h >> 20) & 0x7ff)));  // clamps: zero beyond 63
-  return q;
+  return shifted(m, sh - ((h >> 20) & 0x7ff));
 }
-__device__ __forceinline__ ll to_fixed(double v, int sh) {
-  const ll q = magnitude(v, sh), s = __double2hiint(v) >> 31;
+__device__ __forceinline__ ll magnitude(float v, int sh) {
+  const int h = __float_as_int(v);
+  return shifted((unsigned long long)((h & 0x7fffff) | 0x800000) << 37, sh - 896 - ((h >> 23) & 0xff));
+}
+__device__ __forceinline__ int sign_word(double v) { return __double2hiint(v) >> 31; }
+__device__ __forceinline__ int sign_word(float v) { return __float_as_int(v) >> 31; }
+template <typename T>
+__device__ __forceinline__ ll to_fixed(T v, int sh) {
+  const ll q = magnitude(v, sh), s = sign_word(v);
   return (q ^ s) - s;
 }
-__device__ __forceinline__ R to_fixed_split(double v, int sh) {
+template <typename T>
+__device__ __forceinline__ R to_fixed_split(T v, int sh) {
   R r = split(magnitude(v, sh));
-  const int sg = (__double2hiint(v) >> 31) | 1;
+  const int sg = sign_word(v) | 1;
   r.h *= sg;
   r.l *= sg;
   return r;
@@ -148,16 +159,18 @@ constexpr int kMinExp = -400;  // smaller values are held at 2^-460
 __device__ __forceinline__ int exponent_of(int habs) { return (habs >> 20) - 1022; }
 constexpr int kMaxEntryHi = 0x3FF07AE1;  // 1.03
 
+// the high word of |v| as a double
 __device__ __forceinline__ int habs(double v) { return __double2hiint(v) & 0x7fffffff; }
+__device__ __forceinline__ int habs(float v) { return ((__float_as_int(v) & 0x7fffffff) >> 3) + (896 << 20); }
 
 // A plain matrix with entries up to one (a link), exponent 0.
-template <typename I>
-__device__ __forceinline__ void link_plain(const cx<double>* __restrict__ U, I S, int mu, I s, M& m, Guard& g) {
-  const cx<double>* p = U + ((I)(mu * 9) * S + s);
+template <typename T, typename I>
+__device__ __forceinline__ void link_plain(const cx<T>* __restrict__ U, I S, int mu, I s, M& m, Guard& g) {
+  const cx<T>* p = U + ((I)(mu * 9) * S + s);
   int top = 0;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const cx<double> v = p[(I)k * S];
+    const cx<T> v = p[(I)k * S];
     top = max(top, max(habs(v.re), habs(v.im)));
     m.e[k].re = to_fixed_split(v.re, shift(kScale));
     m.e[k].im = to_fixed_split(v.im, shift(kScale));
@@ -165,13 +178,20 @@ __device__ __forceinline__ void link_plain(const cx<double>* __restrict__ U, I S
   g.bad |= top > kMaxEntryHi;
 }
 
-// A = U - 1 with the exponent of its largest entry (at most 0).
-template <typename I>
-__device__ __forceinline__ void link_near(const cx<double>* __restrict__ U, I S, int mu, I s, M& m, int& e, Guard& g) {
-  const cx<double>* p = U + ((I)(mu * 9) * S + s);
-  cx<double> v[9];
+// A = U - 1 (dag: U^dagger - 1) with the exponent of its largest entry (at most 0).
+template <typename T, typename I>
+__device__ __forceinline__ void link_near(const cx<T>* __restrict__ U, I S, int mu, I s, M& m, int& e, Guard& g,
+                                          bool dag = false) {
+  const cx<T>* p = U + ((I)(mu * 9) * S + s);
+  cx<T> v[9];
 #pragma unroll
-  for (int k = 0; k < 9; k++) v[k] = p[(I)k * S];
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      cx<T> x = p[(I)(dag ? j + 3 * i : i + 3 * j) * S];
+      if (dag) x.im = -x.im;
+      v[i + 3 * j] = x;
+    }
   int top = 0, topd = 0;
   ll d[3], dor = 0;
 #pragma unroll
@@ -312,6 +332,19 @@ __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, 
   }
 }
 
+// -Re tr(P - 1) 2^(60-e), e = max(ew, ev), of the same P: 3 - Re tr P without its cancellation
+__device__ __forceinline__ ll plaquette_trace(const M& W, int ew, const M& V, int ev) {
+  const int ep = max(ew, ev);
+  Acc a = acc_half();
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    mad(a, W.e[k].re, V.e[k].re);
+    mad(a, W.e[k].im, V.e[k].im);
+  }
+  const ll w = join(W.e[0].re) + join(W.e[4].re) + join(W.e[8].re), v = join(V.e[0].re) + join(V.e[4].re) + join(V.e[8].re);
+  return -((finish(a) >> min(ep - ew - ev, 63)) + (w >> min(ep - ew, 63)) + (v >> min(ep - ev, 63)));
+}
+
 // M = H(p) + i H(q) with H_ij = y_ij - i x_ij, H_ji its conjugate (i < j), H_ii = 2 d_i: H(p) is -4 t.al up to a
 // multiple of 1, which a rotation leaves alone.  Exponent e; the two exponents may differ.
 __device__ __forceinline__ void herm_pair(const Anti& p, const Anti& q, M& m, int& e, ll& tr_re, ll& tr_im) {
@@ -400,6 +433,87 @@ __device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll tr_re, l
   o2[5] = ci[7] + ci[5];
   o2[6] = cr[7] - cr[5];
   o2[7] = 3 * (ci[0] + ci[4]) - 2 * tr_im;
+}
+
+// C = V^dagger H V for Hermitian H, as alg_from_herm reads it (the last component without its 1/sqrt(3), all doubled as
+// in rotate_pair): the upper triangle of C and its diagonal.  (C_22 is formed, not taken from the trace: that is zero
+// only as far as V is unitary, which on links built as long products shows at 1e-15.)
+__device__ __forceinline__ void rotate_one(const M& V, const M& H, ll (&o)[8], Guard& g) {
+  ll cr[9], ci[9];
+  R nV[9];
+#pragma unroll
+  for (int n = 0; n < 9; n++) nV[n] = neg(V.e[n].im);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    C t[3];  // row i of V^dagger H; H_jj is real
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      Acc re = acc_half(), im = acc_half();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const C& m = H.e[k + 3 * j];
+        const int n = k + 3 * i;
+        mad(re, V.e[n].re, m.re);
+        mad(im, nV[n], m.re);
+        if (k != j) {
+          mad(re, V.e[n].im, m.im);
+          mad(im, V.e[n].re, m.im);
+        }
+      }
+      watch(g, re.hh, im.hh);
+      t[j].re = split(finish(re));
+      t[j].im = split(finish(im));
+    }
+#pragma unroll
+    for (int j = i; j < 3; j++) {
+      Acc re = acc_half(), im = acc_half();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const int n = k + 3 * j;
+        mad(re, t[k].re, V.e[n].re);
+        mad(re, t[k].im, nV[n]);
+        if (j != i) {
+          mad(im, t[k].im, V.e[n].re);
+          mad(im, t[k].re, V.e[n].im);
+        }
+      }
+      watch(g, re.hh, im.hh);
+      cr[i + 3 * j] = finish(re);
+      ci[i + 3 * j] = finish(im);
+    }
+  }
+  o[0] = 2 * cr[3];
+  o[1] = -2 * ci[3];
+  o[2] = cr[0] - cr[4];
+  o[3] = 2 * cr[6];
+  o[4] = -2 * ci[6];
+  o[5] = 2 * cr[7];
+  o[6] = -2 * ci[7];
+  o[7] = cr[0] + cr[4] - 2 * cr[8];
+}
+// 2 t.p
+template <typename T>
+__device__ __forceinline__ void herm_one(const Alg<T>& p, M& m, int& e, Guard& g) {
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) top = max(top, habs(p.a[k]));
+  g.bad |= top >= 0x43100000;  // 2^50 or more, or not finite
+  const int em = max(exponent_of(min(top, 0x43100000)), kMinExp) + 2;
+  e = em;
+  const int sh = shift(kScale - em);
+  // a_8 / sqrt 3 in FP64: exact in the format to 2^-60 whatever T is
+  const ll s8 = to_fixed((double)p.a[7] * Consts<double>::inv_sqrt3(), sh), c = to_fixed(p.a[2], sh);
+  constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2}, py[3] = {0, 3, 5};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    const int u = pi[n] + 3 * pj[n], l = pj[n] + 3 * pi[n];
+    m.e[u].re = m.e[l].re = to_fixed_split(p.a[py[n]], sh);
+    m.e[l].im = to_fixed_split(p.a[py[n] + 1], sh);
+    m.e[u].im = neg(m.e[l].im);
+  }
+  m.e[0].re = split(c + s8);
+  m.e[4].re = split(s8 - c);
+  m.e[8].re = split(-2 * s8);
 }
 
 // M = 2 (t.p + i t.q) from two FP64 algebra vectors, exponent two above their largest component's.

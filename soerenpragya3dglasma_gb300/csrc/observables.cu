@@ -23,6 +23,7 @@
 // norm terms are summed in FP64 per link (each link's n counted for the plaquettes it belongs to).
 #include <type_traits>
 
+#include "fx.cuh"
 #include "lattice.cuh"
 
 namespace glasma {
@@ -194,8 +195,111 @@ __device__ __forceinline__ double link_norm_dev(const cx<float>* __restrict__ U,
   return n;
 }
 
+// Site arithmetic of the FP64 sums on the integer pipe (fx.cuh): the magnetic terms are -Re tr(P - 1) from products of
+// links held as U - 1 (nothing cancels against 3), the electric ones rotations.  What the fixed-point format does not
+// hold goes through the FP64 forms, out of line.
+constexpr int kFxThreads = 128;
+constexpr int kFxMinBlocks = 3;     // 168 registers
+constexpr int kFxBlocks = 912;      // grid-stride sums: two waves of 152 x 3
+
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) bulk_kernel(Geometry g, FieldPtrs<T> f, double* partials) {
+__device__ __noinline__ double retr_plaq_fp64(const cx<T>* U, long long S, int p, int q, long long s, long long sp,
+                                              long long sq) {
+  Mat<double> a, b, c, d;
+  load_link_d(U, S, p, s, a);
+  load_link_d(U, S, q, sp, b);
+  load_link_d(U, S, p, sq, c);
+  load_link_d(U, S, q, s, d);
+  return 3.0 - retr_plaq(a, b, c, d);
+}
+// 3 - Re tr of the plaquette (p, q) at s
+template <typename T>
+__device__ __forceinline__ double plaquette_defect(const cx<T>* __restrict__ U, long long S, int p, int q, long long s,
+                                                   long long sp, long long sq) {
+  fx::Guard guard = fx::guard_init();
+  fx::M a, b, w, v;
+  int ea, eb, ew, ev;
+  fx::link_near(U, S, p, s, a, ea, guard);
+  fx::link_near(U, S, q, sp, b, eb, guard);
+  fx::near_product(a, ea, b, eb, w, ew, guard);
+  fx::link_near(U, S, q, s, a, ea, guard);
+  fx::link_near(U, S, p, sq, b, eb, guard);
+  fx::near_product(a, ea, b, eb, v, ev, guard);
+  if (fx::tripped(guard)) return retr_plaq_fp64(U, S, p, q, s, sp, sq);
+  return fx::from_fixed(fx::plaquette_trace(w, ew, v, ev), max(ew, ev) - fx::kScale);
+}
+template <typename T>
+__device__ __noinline__ void inv_adj_fp64(const cx<T>* U, const T* F, long long S, int mu, long long s, Alg<double>& out) {
+  Mat<double> u;
+  Alg<double> e;
+  load_link_d(U, S, mu, s, u);
+  load_alg_d(F, S, mu * 8, s, e);
+  inv_adj_mul(u, e, out);
+}
+// U_mu^d(s) E_mu(s) U_mu(s)
+template <typename T>
+__device__ __forceinline__ void transported(const cx<T>* __restrict__ U, const T* __restrict__ E, long long S, int mu,
+                                            long long s, const Alg<T>& e, Alg<double>& out) {
+  fx::Guard guard = fx::guard_init();
+  fx::M u, h;
+  int eh;
+  fx::ll o[8];
+  fx::link_plain(U, S, mu, s, u, guard);
+  fx::herm_one(e, h, eh, guard);
+  fx::rotate_one(u, h, o, guard);
+  fx::to_alg(o, eh - fx::kScale - 1, 1.0, out);
+  if (fx::tripped(guard)) {
+    Alg<double> t;
+    inv_adj_fp64(U, E, S, mu, s, t);
+    out = t;
+  }
+}
+
+__global__ void __launch_bounds__(kFxThreads, kFxMinBlocks) bulk_fp64_kernel(Geometry g, FieldPtrs<double> f,
+                                                                             double* partials) {
+  double v[7] = {0, 0, 0, 0, 0, 0, 0};
+  const bool is_max[7] = {false, false, false, false, false, false, false};
+  const long long S = g.S;
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < g.vol;
+       idx += (long long)gridDim.x * blockDim.x) {
+    int x, y, z;
+    decode_vol(g, idx, x, y, z);
+    const long long s = idx + g.plane;
+#pragma unroll 1
+    for (int n = 0; n < 3; n++) {  // planes (x,y), (x,z), (y,z)
+      const int p = n == 2 ? 1 : 0, q = n == 0 ? 1 : 2;
+      const long long sx = nbs(g, x, y, z, 1, 0, 0), sy = nbs(g, x, y, z, 0, 1, 0), sz = s + g.plane;
+      const double m = 4.0 * plaquette_defect(f.U, S, p, q, s, n == 2 ? sy : sx, n == 0 ? sy : sz);
+      if (n == 0)
+        v[2] += m;
+      else if (n == 1)
+        v[1] += m;
+      else
+        v[0] += m;
+    }
+    for (int mu = 0; mu < 3; mu++) {
+      Alg<double> e;
+      load_alg_d(f.E, S, mu * 8, s, e);
+      double q = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; k++) q += e.a[k] * e.a[k];
+      v[3 + mu] += q;
+      if (mu == 2) {
+        Alg<double> jp, jm;
+        load_alg_d(f.Jp, S, 0, s, jp);
+        load_alg_d(f.Jm, S, 0, s, jm);
+        double w = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) w += e.a[k] * (jp.a[k] - jm.a[k]);
+        v[6] += w * 0.70710678118654752440084436210484903928483593768847;
+      }
+    }
+  }
+  block_reduce_store<7>(v, is_max, partials + (long long)blockIdx.x * 7);
+}
+
+// The energies of an FP32 lattice (magnetic terms by the identity above).
+__global__ void __launch_bounds__(kRedThreads) bulk_kernel(Geometry g, FieldPtrs<float> f, double* partials) {
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
   const bool is_max[7] = {false, false, false, false, false, false, false};
   const long long S = g.S;
@@ -205,41 +309,19 @@ __global__ void __launch_bounds__(kRedThreads) bulk_kernel(Geometry g, FieldPtrs
     decode_vol(g, idx, x, y, z);
     const long long s = idx + g.plane;
     const long long sxp = nbs(g, x, y, z, 1, 0, 0), syp = nbs(g, x, y, z, 0, 1, 0), szp = s + g.plane;
-    if constexpr (std::is_same<T, float>::value) {
-      // 4 (3 - ReTr P) = 2 ||A - B||^2 - 2 (n(a) + n(b) + n(c) + n(d)).  Summed over the lattice, a
-      // plane with two periodic directions counts each of its links twice; in the planes with z
-      // (open), the transverse link counts once at slice 0 and once more on the top ghost slice.
-      const double nx = link_norm_dev(f.U, S, 0, s), ny = link_norm_dev(f.U, S, 1, s), nz = link_norm_dev(f.U, S, 2, s);
-      const double wz = (z == 0) ? 1.0 : 2.0;
-      double gx = 0.0, gy = 0.0;
-      if (z == g.nz - 1) {
-        gx = link_norm_dev(f.U, S, 0, szp);
-        gy = link_norm_dev(f.U, S, 1, szp);
-      }
-      v[2] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 0, 1, s, sxp, syp) - 2.0 * (2.0 * nx + 2.0 * ny);
-      v[0] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 1, 2, s, syp, szp) - 2.0 * (2.0 * nz + wz * ny + gy);
-      v[1] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 2, 0, s, szp, sxp) - 2.0 * (2.0 * nz + wz * nx + gx);
-    } else {
-      Mat<double> a, b, c, d;
-      // Uxy = U_x(x) U_y(x+x) U_x^d(x+y) U_y^d(x)
-      load_link_d(f.U, S, 0, s, a);
-      load_link_d(f.U, S, 1, sxp, b);
-      load_link_d(f.U, S, 0, syp, c);
-      load_link_d(f.U, S, 1, s, d);
-      v[2] += 4.0 * (3.0 - retr_plaq(a, b, c, d));
-      // Uyz = U_y(x) U_z(x+y) U_y^d(x+z) U_z^d(x)
-      load_link_d(f.U, S, 1, s, a);
-      load_link_d(f.U, S, 2, syp, b);
-      load_link_d(f.U, S, 1, szp, c);
-      load_link_d(f.U, S, 2, s, d);
-      v[0] += 4.0 * (3.0 - retr_plaq(a, b, c, d));
-      // Uzx = U_z(x) U_x(x+z) U_z^d(x+x) U_x^d(x)
-      load_link_d(f.U, S, 2, s, a);
-      load_link_d(f.U, S, 0, szp, b);
-      load_link_d(f.U, S, 2, sxp, c);
-      load_link_d(f.U, S, 0, s, d);
-      v[1] += 4.0 * (3.0 - retr_plaq(a, b, c, d));
+    // 4 (3 - ReTr P) = 2 ||A - B||^2 - 2 (n(a) + n(b) + n(c) + n(d)).  Summed over the lattice, a
+    // plane with two periodic directions counts each of its links twice; in the planes with z
+    // (open), the transverse link counts once at slice 0 and once more on the top ghost slice.
+    const double nx = link_norm_dev(f.U, S, 0, s), ny = link_norm_dev(f.U, S, 1, s), nz = link_norm_dev(f.U, S, 2, s);
+    const double wz = (z == 0) ? 1.0 : 2.0;
+    double gx = 0.0, gy = 0.0;
+    if (z == g.nz - 1) {
+      gx = link_norm_dev(f.U, S, 0, szp);
+      gy = link_norm_dev(f.U, S, 1, szp);
     }
+    v[2] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 0, 1, s, sxp, syp) - 2.0 * (2.0 * nx + 2.0 * ny);
+    v[0] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 1, 2, s, syp, szp) - 2.0 * (2.0 * nz + wz * ny + gy);
+    v[1] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 2, 0, s, szp, sxp) - 2.0 * (2.0 * nz + wz * nx + gx);
     for (int mu = 0; mu < 3; mu++) {
       Alg<double> e;
       load_alg_d(f.E, S, mu * 8, s, e);
@@ -263,7 +345,7 @@ __global__ void __launch_bounds__(kRedThreads) bulk_kernel(Geometry g, FieldPtrs
 
 // Gauss law, per slice: grid (kZChunks, nz).  Partials per (z, chunk): {sum G^2, max |G|}.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) gauss_kernel(Geometry g, FieldPtrs<T> f, double norm, double* partials) {
+__global__ void __launch_bounds__(kFxThreads, kFxMinBlocks) gauss_kernel(Geometry g, FieldPtrs<T> f, double norm, double* partials) {
   double v[2] = {0.0, 0.0};
   const bool is_max[2] = {false, true};
   const int z = blockIdx.y;
@@ -272,15 +354,16 @@ __global__ void __launch_bounds__(kRedThreads) gauss_kernel(Geometry g, FieldPtr
     int x, y;
     decode_plane(g, r, x, y);
     const long long s = site_index(g, x, y, z);
-    Mat<double> u;
-    Alg<double> e, down, tot;
+    Alg<double> tot;
 #pragma unroll
     for (int a = 0; a < 8; a++) tot.a[a] = 0.0;
-    const long long nbr[3] = {nbs(g, x, y, z, -1, 0, 0), nbs(g, x, y, z, 0, -1, 0), s - g.plane};
+#pragma unroll 1
     for (int mu = 0; mu < 3; mu++) {
-      load_link_d(f.U, S, mu, nbr[mu], u);
-      load_alg_d(f.E, S, mu * 8, nbr[mu], e);
-      inv_adj_mul(u, e, down);
+      const long long sb = mu == 0 ? nbs(g, x, y, z, -1, 0, 0) : (mu == 1 ? nbs(g, x, y, z, 0, -1, 0) : s - g.plane);
+      Alg<T> em;
+      Alg<double> e, down;
+      load_alg<T, long long>(f.E, S, mu * 8, sb, em);
+      transported(f.U, f.E, S, mu, sb, em, down);
       load_alg_d(f.E, S, mu * 8, s, e);
 #pragma unroll
       for (int a = 0; a < 8; a++) tot.a[a] += (e.a[a] - down.a[a]);
@@ -372,9 +455,71 @@ __device__ void clover(const Geometry& g, const cx<T>* U, int x, int y, int z, i
   for (int k = 0; k < 9; k++) { avg.e[k].re *= 0.25; avg.e[k].im *= 0.25; }
 }
 
+// The clover average in fixed point, one leaf at a time: leaf = W V^d with W, V products of two links or daggers,
+//   U_mu(x) U_nu(x+mu)         | U_nu(x) U_mu(x+nu)
+//   U_nu(x) U_mu^d(x-mu+nu)    | U_mu^d(x-mu) U_nu(x-mu)
+//   U_nu^d(x-nu) U_mu(x-nu)    | U_mu(x) U_nu^d(x-nu+mu)
+//   U_mu^d(x-mu) U_nu^d(x-mu-nu) | U_nu^d(x-nu) U_mu^d(x-mu-nu)
+// B = 2 ReTr(i t avg), defect = 4 (3 - Re tr avg).  The leaves' own links are multiplied, no U U^d = 1 is used (FP32
+// links satisfy it to 1e-7 only).
+template <typename T>
+__device__ __noinline__ void clover_fp64(const Geometry& g, const cx<T>* U, int x, int y, int z, int mu, int nu,
+                                         Alg<double>& B, double& defect) {
+  Mat<double> avg;
+  clover(g, U, x, y, z, mu, nu, avg);
+  retr_itg(avg, 2.0, B);
+  defect = 4.0 * (3.0 - avg.e[0].re - avg.e[4].re - avg.e[8].re);
+}
+template <typename T>
+__device__ __forceinline__ void clover_fx(const Geometry& g, const cx<T>* __restrict__ U, int x, int y, int z, int mu,
+                                          int nu, Alg<double>& B, double& defect) {
+  const long long S = g.S;
+  auto at = [&](int m, int n) {
+    const int d0 = (mu == 0 ? m : 0) + (nu == 0 ? n : 0), d1 = (mu == 1 ? m : 0) + (nu == 1 ? n : 0),
+              d2 = (mu == 2 ? m : 0) + (nu == 2 ? n : 0);
+    return nbs(g, x, y, z, d0, d1, d2);
+  };
+  fx::Guard guard = fx::guard_init();
+#pragma unroll
+  for (int k = 0; k < 8; k++) B.a[k] = 0.0;
+  defect = 0.0;
+#pragma unroll 1
+  for (int l = 0; l < 4; l++) {
+    const bool swap = l == 1 || l == 2;            // the first link of W is U_nu
+    const int lm = (l & 1) ? -1 : 0, ln = l >= 2 ? -1 : 0;  // the leaf's lower corner: x + lm mu + ln nu
+    fx::M a, b, w, v;
+    int ea, eb, ew, ev;
+    // W: first link
+    fx::link_near(U, S, swap ? nu : mu, l == 0 || l == 1 ? at(0, 0) : (l == 2 ? at(0, -1) : at(-1, 0)), a, ea, guard,
+                  l >= 2);
+    fx::link_near(U, S, swap ? mu : nu, l == 0 ? at(1, 0) : (l == 1 ? at(-1, 1) : (l == 2 ? at(0, -1) : at(-1, -1))), b, eb,
+                  guard, l == 1 || l == 3);
+    fx::near_product(a, ea, b, eb, w, ew, guard);
+    fx::link_near(U, S, swap ? mu : nu, l == 0 || l == 2 ? at(0, 0) : (l == 1 ? at(-1, 0) : at(0, -1)), a, ea, guard,
+                  l == 1 || l == 3);
+    fx::link_near(U, S, swap ? nu : mu, l == 0 ? at(0, 1) : (l == 1 ? at(-1, 0) : (l == 2 ? at(1, -1) : at(lm, ln))), b, eb,
+                  guard, l >= 2);
+    fx::near_product(a, ea, b, eb, v, ev, guard);
+    fx::Anti p;
+    fx::plaquette_parts(w, ew, v, ev, p);
+#pragma unroll
+    for (int k = 0; k < 8; k++) B.a[k] += fx::from_fixed(fx::component(p, k), p.e - fx::kScale);
+    defect += fx::from_fixed(fx::plaquette_trace(w, ew, v, ev), p.e - fx::kScale);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) B.a[k] *= k == 7 ? -0.25 * Consts<double>::inv_sqrt3() : -0.25;
+  if (fx::tripped(guard)) {
+    Alg<double> t;
+    double d;
+    clover_fp64(g, U, x, y, z, mu, nu, t, d);
+    B = t;
+    defect = d;
+  }
+}
+
 // Energy-momentum tensor map, grid (kZChunks, nz); partials per (z, chunk): 10 sums.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) emt_kernel(Geometry g, FieldPtrs<T> f, double aScale, double* partials) {
+__global__ void __launch_bounds__(kFxThreads, kFxMinBlocks) emt_kernel(Geometry g, FieldPtrs<T> f, double aScale, double* partials) {
   double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   const bool is_max[10] = {false, false, false, false, false, false, false, false, false, false};
   const int z = blockIdx.y;
@@ -383,43 +528,55 @@ __global__ void __launch_bounds__(kRedThreads) emt_kernel(Geometry g, FieldPtrs<
   double q[3];
   for (int mu = 0; mu < 3; mu++) q[mu] = g.a[mu] * aScale * aScale / a3;
   const double inv = 1.0 / ((double)g.nx * g.ny);
+  // the site's B waits in shared memory: held in registers through the transports it would spill
+  __shared__ double sB[24 * kFxThreads];
+  double* const tb = sB + threadIdx.x;
   for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < g.plane; r += (long long)gridDim.x * blockDim.x) {
     int x, y;
     decode_plane(g, r, x, y);
     const long long s = site_index(g, x, y, z);
     // magnetic: clover averages of UOld in the planes yz (B0), zx (B1), xy (B2)
-    Alg<double> B[3];
-    double Bs[3];
-    {
-      Mat<double> avg;
-      const int planes[3][2] = {{1, 2}, {2, 0}, {0, 1}};
-      for (int i = 0; i < 3; i++) {
-        clover(g, f.UOld, x, y, z, planes[i][0], planes[i][1], avg);
-        retr_itg(avg, 2.0, B[i]);
-        Bs[i] = 4.0 * (3.0 - avg.e[0].re - avg.e[4].re - avg.e[8].re);
-      }
+    double Bs[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int i = 0; i < 3; i++) {
+      Alg<double> b;
+      double d;
+      clover_fx(g, f.UOld, x, y, z, i == 2 ? 0 : i + 1, i == 0 ? 2 : i - 1, b, d);
+#pragma unroll
+      for (int k = 0; k < 8; k++) tb[(i * 8 + k) * kFxThreads] = b.a[k];
+      Bs[0] = i == 0 ? d : Bs[0];
+      Bs[1] = i == 1 ? d : Bs[1];
+      Bs[2] = i == 2 ? d : Bs[2];
     }
     // electric: average with the parallel-transported backward neighbour, using U
     Alg<double> Ev[3];
-    double Es[3];
-    {
-      const long long nbr[3] = {nbs(g, x, y, z, -1, 0, 0), nbs(g, x, y, z, 0, -1, 0), s - g.plane};
-      for (int mu = 0; mu < 3; mu++) {
-        Mat<double> u;
-        Alg<double> em, e, down;
-        load_link_d(f.U, S, mu, nbr[mu], u);
-        load_alg_d(f.E, S, mu * 8, nbr[mu], em);
-        inv_adj_mul(u, em, down);
-        load_alg_d(f.E, S, mu * 8, s, e);
-        double sq = 0.0;
+    double Es[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int mu = 0; mu < 3; mu++) {
+      const long long sb = mu == 0 ? nbs(g, x, y, z, -1, 0, 0) : (mu == 1 ? nbs(g, x, y, z, 0, -1, 0) : s - g.plane);
+      Alg<T> em;
+      Alg<double> e, down;
+      load_alg<T, long long>(f.E, S, mu * 8, sb, em);
+      transported(f.U, f.E, S, mu, sb, em, down);
+      load_alg_d(f.E, S, mu * 8, s, e);
+      double sq = 0.0;
 #pragma unroll
-        for (int a = 0; a < 8; a++) {
-          Ev[mu].a[a] = 0.5 * (e.a[a] + down.a[a]);
-          sq += 0.5 * (e.a[a] * e.a[a] + em.a[a] * em.a[a]);
-        }
-        Es[mu] = sq;
+      for (int a = 0; a < 8; a++) {
+        down.a[a] = 0.5 * (e.a[a] + down.a[a]);
+        sq += 0.5 * (e.a[a] * e.a[a] + (double)em.a[a] * (double)em.a[a]);
       }
+#pragma unroll
+      for (int n = 0; n < 3; n++)  // by selection: an index would move the array to local memory
+        if (n == mu) {
+          Ev[n] = down;
+          Es[n] = sq;
+        }
     }
+    Alg<double> B[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int k = 0; k < 8; k++) B[i].a[k] = tb[(i * 8 + k) * kFxThreads];
     const double e0 = q[0] * q[0] * Es[0], e1 = q[1] * q[1] * Es[1], e2 = q[2] * q[2] * Es[2];
     const double b0 = q[0] * q[0] * Bs[0], b1 = q[1] * q[1] * Bs[1], b2 = q[2] * q[2] * Bs[2];
     v[0] += (0.5 * (e0 + e1 + e2 + b0 + b1 + b2)) * inv;
@@ -457,8 +614,15 @@ static unsigned red_blocks(long long n) {
 
 template <typename T>
 cudaError_t launch_bulk(const Geometry& g, FieldPtrs<T> f, double* partials, double* result7, cudaStream_t stream) {
-  const unsigned nb = red_blocks(g.vol);
-  bulk_kernel<T><<<nb, kRedThreads, 0, stream>>>(g, f, partials);
+  unsigned nb;
+  if constexpr (std::is_same<T, double>::value) {
+    const long long n = (g.vol + kFxThreads - 1) / kFxThreads;
+    nb = (unsigned)(n < kFxBlocks ? n : kFxBlocks);
+    bulk_fp64_kernel<<<nb, kFxThreads, 0, stream>>>(g, f, partials);
+  } else {
+    nb = red_blocks(g.vol);
+    bulk_kernel<<<nb, kRedThreads, 0, stream>>>(g, f, partials);
+  }
   finish_kernel<7><<<1, kRedThreads, 0, stream>>>(partials, (int)nb, 0u, result7);
   return cudaGetLastError();
 }
@@ -469,7 +633,7 @@ cudaError_t launch_gauss(const Geometry& g, FieldPtrs<T> f, double a_scale, doub
                          double* zprofile, cudaStream_t stream) {
   const double norm = a_scale * a_scale * a_scale / (g.a[0] * g.a[1] * g.a[2]);
   dim3 grid(kZChunks, g.nz);
-  gauss_kernel<T><<<grid, kRedThreads, 0, stream>>>(g, f, norm, partials);
+  gauss_kernel<T><<<grid, kFxThreads, 0, stream>>>(g, f, norm, partials);
   double* slices = partials + (long long)g.nz * kZChunks * 2;
   finish_slices_kernel<2><<<(g.nz * 2 + 255) / 256, 256, 0, stream>>>(partials, g.nz, 2u, slices);
   finish_kernel<2><<<1, kRedThreads, 0, stream>>>(slices, g.nz, 2u, result2);
@@ -492,7 +656,7 @@ template <typename T>
 cudaError_t launch_emt_map(const Geometry& g, FieldPtrs<T> f, double a_scale, double* partials, double* result,
                            cudaStream_t stream) {
   dim3 grid(kZChunks, g.nz);
-  emt_kernel<T><<<grid, kRedThreads, 0, stream>>>(g, f, a_scale, partials);
+  emt_kernel<T><<<grid, kFxThreads, 0, stream>>>(g, f, a_scale, partials);
   finish_slices_kernel<10><<<(g.nz * 10 + 255) / 256, 256, 0, stream>>>(partials, g.nz, 0u, result);
   return cudaGetLastError();
 }
