@@ -163,17 +163,17 @@ constexpr int kMaxEntryHi = 0x3FF07AE1;  // 1.03
 __device__ __forceinline__ int habs(double v) { return __double2hiint(v) & 0x7fffffff; }
 __device__ __forceinline__ int habs(float v) { return ((__float_as_int(v) & 0x7fffffff) >> 3) + (896 << 20); }
 
-// A plain matrix with entries up to one (a link), exponent 0.
-template <typename T, typename I>
+// A plain matrix with entries up to one (a link), exponent 0; kDag: its dagger.
+template <bool kDag = false, typename T, typename I>
 __device__ __forceinline__ void link_plain(const cx<T>* __restrict__ U, I S, int mu, I s, M& m, Guard& g) {
   const cx<T>* p = U + ((I)(mu * 9) * S + s);
   int top = 0;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const cx<T> v = p[(I)k * S];
+    const cx<T> v = p[(I)(kDag ? k / 3 + 3 * (k % 3) : k) * S];
     top = max(top, max(habs(v.re), habs(v.im)));
     m.e[k].re = to_fixed_split(v.re, shift(kScale));
-    m.e[k].im = to_fixed_split(v.im, shift(kScale));
+    m.e[k].im = to_fixed_split(kDag ? -v.im : v.im, shift(kScale));
   }
   g.bad |= top > kMaxEntryHi;
 }
@@ -292,9 +292,10 @@ __device__ __forceinline__ ll component(const Anti& p, int k) {
   }
 }
 
-// P = (1 + w)(1 + v)^dagger of two near products
+// P = W V^dagger (kNear: (1 + w)(1 + v)^dagger of two near products)
+template <bool kNear = true>
 __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, int ev, Anti& o) {
-  const int ep = max(ew, ev);
+  const int ep = kNear ? max(ew, ev) : ew + ev;
   const int k = min(ep - ew - ev, 63), kw = min(ep - ew, 63), kv = min(ep - ev, 63);
   o.e = ep;
   constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
@@ -314,10 +315,13 @@ __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, 
       mad(xn, wj.re, vi.re);
       mad(xn, wj.im, vi.im);
     }
+    o.y[n] = finish_diff(yp, yn) >> k;
+    o.x[n] = finish_diff(xp, xn) >> k;
+    if (!kNear) continue;
     const ll yw = join(W.e[i + 3 * j].im) + join(W.e[j + 3 * i].im), yv = join(V.e[i + 3 * j].im) + join(V.e[j + 3 * i].im);
     const ll xw = join(W.e[i + 3 * j].re) - join(W.e[j + 3 * i].re), xv = join(V.e[j + 3 * i].re) - join(V.e[i + 3 * j].re);
-    o.y[n] = (finish_diff(yp, yn) >> k) + (yw >> kw) - (yv >> kv);
-    o.x[n] = (finish_diff(xp, xn) >> k) + (xw >> kw) + (xv >> kv);
+    o.y[n] += (yw >> kw) - (yv >> kv);
+    o.x[n] += (xw >> kw) + (xv >> kv);
   }
 #pragma unroll
   for (int i = 0; i < 3; i++) {
@@ -328,8 +332,45 @@ __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, 
       mad(p, w.im, v.re);
       mad(q, w.re, v.im);
     }
-    o.d[i] = (finish_diff(p, q) >> k) + (join(W.e[4 * i].im) >> kw) - (join(V.e[4 * i].im) >> kv);
+    o.d[i] = finish_diff(p, q) >> k;
+    if (kNear) o.d[i] += (join(W.e[4 * i].im) >> kw) - (join(V.e[4 * i].im) >> kv);
   }
+}
+
+// A B of two matrices with entries up to one, B daggered if kDag; watched, so that the next product has room
+template <bool kDag>
+__device__ __forceinline__ void product(const M& A, const M& B, M& P, Guard& g) {
+  R nB[9];
+#pragma unroll
+  for (int n = 0; n < 9; n++) nB[n] = neg(B.e[n].im);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      Acc re = acc_half(), im = acc_half();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const int n = kDag ? j + 3 * k : k + 3 * j;
+        const C& a = A.e[i + 3 * k];
+        mad(re, a.re, B.e[n].re);
+        mad(re, a.im, kDag ? B.e[n].im : nB[n]);
+        mad(im, a.im, B.e[n].re);
+        mad(im, a.re, kDag ? nB[n] : B.e[n].im);
+      }
+      watch(g, re.hh, im.hh);
+      P.e[i + 3 * j].re = split(finish(re));
+      P.e[i + 3 * j].im = split(finish(im));
+    }
+}
+// Re tr(A B^dagger) 2^60 of two plain matrices
+__device__ __forceinline__ ll trace_nd(const M& A, const M& B) {
+  Acc a = acc_half();
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    mad(a, A.e[k].re, B.e[k].re);
+    mad(a, A.e[k].im, B.e[k].im);
+  }
+  return finish(a);
 }
 
 // -Re tr(P - 1) 2^(60-e), e = max(ew, ev), of the same P: 3 - Re tr P without its cancellation

@@ -43,6 +43,8 @@
 #include <vector>
 
 #include "../../include/glasma_gb300.h"
+#include "fft.cuh"
+#include "fx.cuh"
 #include "gaugefix.h"
 #include "reduce.cuh"
 
@@ -55,12 +57,6 @@ constexpr int kGfBlocks = 1216;
 constexpr int kFftThreads = 256;
 constexpr int kFftMaxTile = 4096;  // complex doubles staged per block (64 KB)
 constexpr size_t kFftMaxSmem = 227 * 1024;  // shared memory a block may opt into
-// Build knob: power-of-two lengths through the mixed-radix Stockham kernel (radix 4) instead of the
-// radix-2 kernel.
-#ifndef GLASMA_FFT_POW2_STOCKHAM
-#define GLASMA_FFT_POW2_STOCKHAM 0
-#endif
-
 inline unsigned blocks_for(long long n, int threads, int cap) {
   long long b = (n + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -216,8 +212,7 @@ __global__ void accelerate32_kernel(int nx, int ny, int nz, float vf, const floa
     X[i] = make_float2(0.f, 0.f);
   }
 }
-template <typename C>
-__global__ void accelerate_kernel(int nx, int ny, int nz, double vd, const double* __restrict__ tab, C* X,
+__global__ void accelerate_kernel(int nx, int ny, int nz, double vd, const double* __restrict__ tab, double2* X,
                                   int project_zero) {
   const long long V = (long long)nx * ny * nz;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -229,19 +224,31 @@ __global__ void accelerate_kernel(int nx, int ny, int nz, double vd, const doubl
   const double p2 = tab[px] + tab[nx + py] + tab[nx + ny + pz];
   if (p2 > 0.0) {
     const double f = 1.0 / (vd * p2);
-    C v = X[i];
+    double2 v = X[i];
     v.x *= f;
     v.y *= f;
     X[i] = v;
   } else if (project_zero) {
-    X[i] = cmk((decltype(C::x))0, (decltype(C::x))0);
+    X[i] = make_double2(0.0, 0.0);
   }
 }
 
 // ---- update of G; partials {max step, sum step^2, guard count}
+// What the fixed-point form hands back, in FP64, with the reference's guard (CoulombGaugeDeviation.cpp:57-68; written so
+// that a NaN also trips it).  A fixed-point exponential is unitary to 1e-16 by construction: its argument is below one.
+static __device__ __noinline__ bool update_fp64(double alpha, const Alg<double>& upd, const Mat<double>& gm, Mat<double>& gn,
+                                         double& sr, double& si) {
+  Mat<double> wt;
+  expi(-alpha, upd, wt);
+  sr = 3.0 - wt.e[0].re - wt.e[4].re - wt.e[8].re;
+  si = -(wt.e[0].im + wt.e[4].im + wt.e[8].im);
+  mul_dn(wt, gm, gn);
+  return unitarity_norm(wt) <= 1e-13;
+}
+// G <- wt^d G = G + (X - 1) G with X = exp(+i alpha t.Delta), in fixed point on the integer pipe
 template <typename T, typename C>
-__global__ void __launch_bounds__(kGfThreads) update_kernel(Geometry g, const C* X, cx<T>* G, double alpha,
-                                                            double* partials) {
+__global__ void __launch_bounds__(kGfThreads, 1) update_kernel(Geometry g, const C* X, cx<T>* G, double alpha,
+                                                               double* partials) {
   double v[3] = {0.0, 0.0, 0.0};
   const int op[3] = {1, 0, 0};
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < g.vol;
@@ -249,24 +256,158 @@ __global__ void __launch_bounds__(kGfThreads) update_kernel(Geometry g, const C*
     Alg<double> upd;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const C v = X[(long long)q * g.vol + idx];
-      upd.a[2 * q] = (double)v.x;
-      upd.a[2 * q + 1] = (double)v.y;
+      const C x = X[(long long)q * g.vol + idx];
+      upd.a[2 * q] = (double)x.x;
+      upd.a[2 * q + 1] = (double)x.y;
     }
-    Mat<double> wt, gm, gn;
-    expi(-alpha, upd, wt);
-    // the reference's guard (CoulombGaugeDeviation.cpp:57-68); written so that a NaN also trips it
-    if (!(unitarity_norm(wt) <= 1e-13)) v[2] += 1.0;
-    const double sr = 3.0 - wt.e[0].re - wt.e[4].re - wt.e[8].re, si = -(wt.e[0].im + wt.e[4].im + wt.e[8].im);
+    const long long s = idx + g.plane;
+    Mat<double> gm, gn;
+    ld_d(G, g.S, 0, s, gm);
+    fx::M x;
+    int ex;
+    double sr, si;
+    bool fits = fx::near_exp(alpha, upd, x, ex);
+    if (fits) {
+      sr = fx::from_fixed(fx::join(x.e[0].re) + fx::join(x.e[4].re) + fx::join(x.e[8].re), ex - fx::kScale);
+      si = fx::from_fixed(fx::join(x.e[0].im) + fx::join(x.e[4].im) + fx::join(x.e[8].im), ex - fx::kScale);
+      fits = fx::add_product(x, ex, gm, gn);
+    }
+    if (!fits) {
+      const Mat<double> a = gm;
+      const Alg<double> u = upd;
+      Mat<double> b;
+      double r, i;
+      if (!update_fp64(alpha, u, a, b, r, i)) v[2] += 1.0;
+      gn = b;
+      sr = r;
+      si = i;
+    }
     const double step = sqrt(sr * sr + si * si);
     v[0] = fmax(v[0], step);
     v[1] += step * step;
-    const long long s = idx + g.plane;
-    ld_d(G, g.S, 0, s, gm);
-    mul_dn(wt, gm, gn);
     st_d(G, g.S, 0, s, gn);
   }
   red::block_reduce_store<3>(v, op, partials + (long long)blockIdx.x * 3);
+}
+
+// ---- what the deviation needs of the transformed links UG_mu(x) = G(x) U_mu(x) G^d(x+mu), and no more: the eight
+// ReTr(i t^a UG) and Re tr UG, 27 numbers a site instead of 54 written and read (A[(9 mu + k) V + x]); the sweeps need the
+// links themselves only at their end.  One thread per link.
+static __device__ __noinline__ void link_deviation_fp64(const Mat<double>& gx, const Mat<double>& u, const Mat<double>& gy,
+                                                 Alg<double>& al, double& tr) {
+  Mat<double> t, o;
+  mul_nn(gx, u, t);
+  mul_nd(t, gy, o);
+  retr_itg(o, 1.0, al);
+  tr = o.e[0].re + o.e[4].re + o.e[8].re;
+}
+__device__ __forceinline__ long long forward(const Geometry& g, long long idx, int mu) {
+  int x, y, z;
+  gf_decode(idx, g.nx, g.ny, g.vol, x, y, z);
+  return mu == 0 ? nbr(g, x, y, z, 1, 0, 0) : (mu == 1 ? nbr(g, x, y, z, 0, 1, 0) : idx + 2 * g.plane);
+}
+constexpr int kLinkThreads = 128;
+template <typename T>
+__global__ void __launch_bounds__(kLinkThreads, 3) link_deviation_kernel(Geometry g, const cx<T>* __restrict__ U,
+                                                                         const cx<T>* __restrict__ G,
+                                                                         double* __restrict__ A) {
+  const int mu = blockIdx.y;
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= g.vol) return;
+  const long long s = idx + g.plane, sf = forward(g, idx, mu);
+  fx::Guard guard = fx::guard_init();
+  fx::M a, b, t;
+  fx::link_plain(G, g.S, 0, s, a, guard);
+  fx::link_plain(U, g.S, mu, s, b, guard);
+  fx::product<false>(a, b, t, guard);
+  fx::link_plain(G, g.S, 0, sf, a, guard);
+  fx::Anti p;
+  fx::plaquette_parts<false>(t, 0, a, 0, p);
+  Alg<double> al;
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    al.a[k] = fx::from_fixed(fx::component(p, k), -fx::kScale) * (k == 7 ? -0.5 * Consts<double>::inv_sqrt3() : -0.5);
+  double tr = fx::from_fixed(fx::trace_nd(t, a), -fx::kScale);
+  if (fx::tripped(guard)) {
+    Mat<double> gx, u, gy;
+    Alg<double> r;
+    double q;
+    ld_d(G, g.S, 0, s, gx);
+    ld_d(U, g.S, mu * 9, s, u);
+    ld_d(G, g.S, 0, sf, gy);
+    link_deviation_fp64(gx, u, gy, r, q);
+    al = r;
+    tr = q;
+  }
+  double* o = A + (long long)(mu * 9) * g.vol + idx;
+#pragma unroll
+  for (int k = 0; k < 8; k++) o[(long long)k * g.vol] = al.a[k];
+  o[8 * g.vol] = tr;
+}
+__global__ void __launch_bounds__(kLinkThreads) link_deviation32_kernel(Geometry g, const cx<float>* __restrict__ U,
+                                                                        const cx<float>* __restrict__ G,
+                                                                        float* __restrict__ A) {
+  const int mu = blockIdx.y;
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= g.vol) return;
+  const long long s = idx + g.plane, sf = forward(g, idx, mu);
+  Mat<float> a, b, t, o;
+  load_link<float, long long>(G, g.S, 0, s, a);
+  load_link<float, long long>(U, g.S, mu, s, b);
+  mul_nn(a, b, t);
+  load_link<float, long long>(G, g.S, 0, sf, a);
+  mul_nd(t, a, o);
+  Alg<float> al;
+  retr_itg(o, 1.f, al);
+  float* p = A + (long long)(mu * 9) * g.vol + idx;
+#pragma unroll
+  for (int k = 0; k < 8; k++) p[(long long)k * g.vol] = al.a[k];
+  p[8 * g.vol] = o.e[0].re + o.e[4].re + o.e[8].re;
+}
+// Delta = sum_mu c_mu (al_mu(x) - al_mu(x-mu)) (ReTr(i t V^d) = -ReTr(i t V)) and Re tr w; X and the monitors as
+// deviation_kernel's.  Re: the sweeps' arithmetic; FP32 sums per thread, FP64 beyond.  The backward z link of slice 0 is
+// the identity ghost, with trace `ghost`: 3 in FP64 as in the reference's functional; the FP32 sweeps, whose links have no
+// ghosts, log the functional of the links inside the lattice (0).
+template <typename Re, typename C>
+__global__ void __launch_bounds__(kGfThreads) gather_deviation_kernel(Geometry g, const Re* __restrict__ A, Re c0, Re c1,
+                                                                      Re c2, Re ghost, C* X, double* partials,
+                                                                      int open_top) {
+  Re tmax = 0, tsq = 0, tmin = Re(3.0e38), tlf = 0;
+  const int op[4] = {1, 0, 2, 0};
+  const long long V = g.vol;
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < V; idx += (long long)gridDim.x * blockDim.x) {
+    int x, y, z;
+    gf_decode(idx, g.nx, g.ny, V, x, y, z);
+    Alg<Re> dev;
+#pragma unroll
+    for (int k = 0; k < 8; k++) dev.a[k] = 0;
+    Re lf = 0;
+#pragma unroll
+    for (int mu = 0; mu < 3; mu++) {
+      const Re c = mu == 0 ? c0 : (mu == 1 ? c1 : c2);
+      if (c == Re(0)) continue;
+      const Re cf = mu == 2 && open_top && z == g.nz - 1 ? Re(0) : c;
+      const Re cb = mu == 2 && z == 0 ? Re(0) : c;
+      const long long back = mu == 0 ? (x > 0 ? idx - 1 : idx + g.nx - 1)
+                                     : (mu == 1 ? (y > 0 ? idx - g.nx : idx + g.plane - g.nx) : (z > 0 ? idx - g.plane : idx));
+      const Re* p = A + (long long)(mu * 9) * V;
+#pragma unroll
+      for (int k = 0; k < 8; k++) dev.a[k] += cf * p[(long long)k * V + idx] - cb * p[(long long)k * V + back];
+      lf += cf * p[8 * V + idx] + c * (mu == 2 && z == 0 ? ghost : p[8 * V + back]);
+    }
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      tmax = max(tmax, dev.a[a] < 0 ? -dev.a[a] : dev.a[a]);
+      tsq += dev.a[a] * dev.a[a];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      X[(long long)q * V + idx] = cmk((decltype(C::x))dev.a[2 * q], (decltype(C::x))dev.a[2 * q + 1]);
+    tmin = min(tmin, lf);
+    tlf += lf;
+  }
+  double v[4] = {(double)tmax, (double)tsq, (double)tmin, (double)tlf};
+  red::block_reduce_store<4>(v, op, partials + (long long)blockIdx.x * 4);
 }
 
 // ---- mixed-precision sweeps (GLASMA_GF_MIXED, FP64 handles): the Fourier-accelerated iteration on
@@ -293,84 +434,12 @@ __global__ void narrow_kernel(const cx<double>* __restrict__ src, cx<float>* __r
   dst[i] = mk<float>((float)v.re, (float)v.im);
 }
 
-// UG_mu(x) = G(x) U_mu(x) G^d(x+mu) in FP32, interior sites
-__global__ void __launch_bounds__(128) transform_links32_kernel(Geometry g, const cx<float>* U, const cx<float>* G,
-                                                                cx<float>* UG) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= g.vol) return;
-  int x, y, z;
-  gf_decode(idx, g.nx, g.ny, g.vol, x, y, z);
-  const long long s = idx + g.plane;
-  const long long fwd[3] = {nbr(g, x, y, z, 1, 0, 0), nbr(g, x, y, z, 0, 1, 0), s + g.plane};
-  Mat<float> gx, u, gy, t, o;
-  ld_f(G, g.S, 0, s, gx);
-  for (int mu = 0; mu < 3; mu++) {
-    ld_f(U, g.S, mu * 9, s, u);
-    ld_f(G, g.S, 0, fwd[mu], gy);
-    mul_nn(gx, u, t);
-    mul_nd(t, gy, o);
-    st_f(UG, g.S, mu * 9, s, o);
-  }
-}
-
-// deviation_kernel in FP32 (site_w's sum, the projection and X); partials in FP64
-__global__ void __launch_bounds__(kGfThreads) deviation32_kernel(Geometry g, const cx<float>* UG, float c0, float c1,
-                                                                 float c2, float2* X, double* partials, int open_top) {
-  // each thread's sites summed in FP32 (a few dozen terms), the block and grid sums in FP64: FP64
-  // arithmetic and conversions run on GB300's slow FP64 pipe, which this kernel then leaves alone
-  double v[4];
-  float tmax = 0.f, tsq = 0.f, tmin = 3.0e38f, tlf = 0.f;
-  const int op[4] = {1, 0, 2, 0};
-  const float c[3] = {c0, c1, c2};
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < g.vol;
-       idx += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    gf_decode(idx, g.nx, g.ny, g.vol, x, y, z);
-    const long long s = idx + g.plane;
-    const long long back[3] = {nbr(g, x, y, z, -1, 0, 0), nbr(g, x, y, z, 0, -1, 0), s - g.plane};
-    const float fwd2 = (open_top && z == g.nz - 1) ? 0.f : 1.f;
-    Mat<float> w;
-    set_zero(w);
-    for (int mu = 0; mu < 3; mu++) {
-      if (c[mu] == 0.f) continue;
-      const float cf = mu == 2 ? fwd2 : 1.f;
-      Mat<float> u, d;
-      ld_f(UG, g.S, mu * 9, s, u);
-      ld_f(UG, g.S, mu * 9, back[mu], d);
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          const int k = i + 3 * j, kt = j + 3 * i;
-          w.e[k].re += c[mu] * (cf * u.e[k].re + d.e[kt].re);
-          w.e[k].im += c[mu] * (cf * u.e[k].im - d.e[kt].im);
-        }
-    }
-    Alg<float> dev;
-    retr_itg(w, 1.f, dev);
-#pragma unroll
-    for (int a = 0; a < 8; a++) {
-      tmax = fmaxf(tmax, fabsf(dev.a[a]));
-      tsq = fmaf(dev.a[a], dev.a[a], tsq);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) X[(long long)q * g.vol + idx] = make_float2(dev.a[2 * q], dev.a[2 * q + 1]);
-    const float lf = w.e[0].re + w.e[4].re + w.e[8].re;
-    tmin = fminf(tmin, lf);
-    tlf += lf;
-  }
-  v[0] = tmax;
-  v[1] = tsq;
-  v[2] = tmin;
-  v[3] = tlf;
-  red::block_reduce_store<4>(v, op, partials + (long long)blockIdx.x * 4);
-}
-
 // update_kernel in FP32.  The unitarity guard cannot hold FP64's 1e-13 here (an FP32 exponential is
 // unitary to ~1e-7): it trips at `guard`, which still catches the runaway the reference's guard exists for.
 __global__ void __launch_bounds__(kGfThreads) update32_kernel(Geometry g, const float2* X, cx<float>* G, float alpha,
                                                               double* partials, float guard) {
-  // per-thread sums in FP32, block and grid sums in FP64 (as deviation32_kernel)
+  // per-thread sums in FP32, block and grid sums in FP64 (FP64 arithmetic and
+  // conversions run on GB300's slow FP64 pipe)
   double v[3];
   float tmax = 0.f, tsq = 0.f, tbad = 0.f;
   const int op[3] = {1, 0, 0};
@@ -533,42 +602,73 @@ __global__ void __launch_bounds__(kGfThreads) local_update_kernel(Geometry g, co
   red::block_reduce_store<7>(v, op, partials + (long long)blockIdx.x * 7);
 }
 
-// ---- UG_mu(x) = G(x) U_mu(x) G^d(x+mu), interior sites
+// ---- UG_mu(x) = G(x) U_mu(x) G^d(x+mu), interior sites, one thread per link
+static __device__ __noinline__ void transform_link_fp64(const Mat<double>& gx, const Mat<double>& u, const Mat<double>& gy,
+                                                 Mat<double>& o) {
+  Mat<double> t;
+  mul_nn(gx, u, t);
+  mul_nd(t, gy, o);
+}
 template <typename T>
-__global__ void __launch_bounds__(128) transform_links_kernel(Geometry g, const cx<T>* U, const cx<T>* G, cx<T>* UG) {
+__global__ void __launch_bounds__(kLinkThreads, 3) transform_links_kernel(Geometry g, const cx<T>* __restrict__ U,
+                                                                          const cx<T>* __restrict__ G, cx<T>* UG) {
+  const int mu = blockIdx.y;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= g.vol) return;
-  int x, y, z;
-  gf_decode(idx, g.nx, g.ny, g.vol, x, y, z);
-  const long long s = idx + g.plane;
-  const long long fwd[3] = {nbr(g, x, y, z, 1, 0, 0), nbr(g, x, y, z, 0, 1, 0), s + g.plane};
-  Mat<double> gx, u, gy, t, o;
-  ld_d(G, g.S, 0, s, gx);
-  for (int mu = 0; mu < 3; mu++) {
+  const long long s = idx + g.plane, sf = forward(g, idx, mu);
+  fx::Guard guard = fx::guard_init();
+  fx::M a, b, t;
+  fx::link_plain(G, g.S, 0, s, a, guard);
+  fx::link_plain(U, g.S, mu, s, b, guard);
+  fx::product<false>(a, b, t, guard);
+  fx::link_plain(G, g.S, 0, sf, a, guard);
+  fx::product<true>(t, a, b, guard);
+  Mat<double> o;
+#pragma unroll
+  for (int k = 0; k < 9; k++)
+    o.e[k] = mk<double>(fx::from_fixed(fx::join(b.e[k].re), -fx::kScale), fx::from_fixed(fx::join(b.e[k].im), -fx::kScale));
+  if (fx::tripped(guard)) {
+    Mat<double> gx, u, gy, r;
+    ld_d(G, g.S, 0, s, gx);
     ld_d(U, g.S, mu * 9, s, u);
-    ld_d(G, g.S, 0, fwd[mu], gy);
-    mul_nn(gx, u, t);
-    mul_nd(t, gy, o);
-    st_d(UG, g.S, mu * 9, s, o);
+    ld_d(G, g.S, 0, sf, gy);
+    transform_link_fp64(gx, u, gy, r);
+    o = r;
   }
+  st_d(UG, g.S, mu * 9, s, o);
 }
 
-// ---- EG_mu(x) = G(x) E_mu(x) G^d(x)
+// ---- EG_mu(x) = G(x) E_mu(x) G^d(x), one thread per component vector
+static __device__ __noinline__ void adj_fp64(const Mat<double>& v, const Alg<double>& e, Alg<double>& o) { adj_mul(v, e, o); }
 template <typename T>
-__global__ void __launch_bounds__(128) transform_efield_kernel(Geometry g, const T* E, const cx<T>* G, T* EG) {
+__global__ void __launch_bounds__(kLinkThreads, 3) transform_efield_kernel(Geometry g, const T* __restrict__ E,
+                                                                           const cx<T>* __restrict__ G, T* EG) {
+  const int mu = blockIdx.y;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= g.vol) return;
   const long long s = idx + g.plane;
-  Mat<double> gx;
-  ld_d(G, g.S, 0, s, gx);
-  for (int mu = 0; mu < 3; mu++) {
-    Alg<double> e, o;
+  fx::Guard guard = fx::guard_init();
+  fx::M v, h;
+  int eh;
+  fx::ll q[8];
+  Alg<T> e;
+  Alg<double> o;
+  load_alg<T, long long>(E, g.S, mu * 8, s, e);
+  fx::link_plain<true>(G, g.S, 0, s, v, guard);
+  fx::herm_one(e, h, eh, guard);
+  fx::rotate_one(v, h, q, guard);
+  fx::to_alg(q, eh - fx::kScale - 1, 1.0, o);
+  if (fx::tripped(guard)) {
+    Mat<double> gx;
+    Alg<double> a, r;
+    ld_d(G, g.S, 0, s, gx);
 #pragma unroll
-    for (int a = 0; a < 8; a++) e.a[a] = (double)E[(long long)(mu * 8 + a) * g.S + s];
-    adj_mul(gx, e, o);
-#pragma unroll
-    for (int a = 0; a < 8; a++) EG[(long long)(mu * 8 + a) * g.S + s] = (T)o.a[a];
+    for (int k = 0; k < 8; k++) a.a[k] = (double)e.a[k];
+    adj_fp64(gx, a, r);
+    o = r;
   }
+#pragma unroll
+  for (int a = 0; a < 8; a++) EG[(long long)(mu * 8 + a) * g.S + s] = (T)o.a[a];
 }
 
 // ---- jG(x) = G(x) j(x) G^d(x): PERFORM_COLOR_CHARGE_TRANSFORMATION (S/CALC/GaugeTransformation.cpp:28-31),
@@ -747,8 +847,8 @@ __global__ void __launch_bounds__(kFftThreads) fft_mixed_kernel(C* X, int n, lon
       const int jm = j % Ns;
       const C* src = a + t * n + j;
       C* dst = b + t * n + (j - jm) * rad + jm;
-      auto twd = [&](int r) {  // w^(r jm tstep), conjugated for the inverse
-        C w = tw[(int)(((long long)r * jm * tstep) % n)];
+      auto twd = [&](int r) {  // w^(r jm tstep), conjugated for the inverse (the exponent is below n)
+        C w = tw[r * jm * tstep];
         if (inverse) w.y = -w.y;
         return w;
       };
@@ -847,8 +947,8 @@ int ilog2(int n) {
   while ((1 << l) < n) l++;
   return l;
 }
-// the radix-2 kernel reads exp(-2 pi i k/n) for k < n/2, the mixed-radix kernel for k < n
-int twiddle_count(int n) { return (is_pow2(n) && !GLASMA_FFT_POW2_STOCKHAM) ? (n / 2 > 0 ? n / 2 : 1) : n; }
+// exp(-2 pi i k/n) for k < n (the radix-2 kernel reads the first half)
+int twiddle_count(int n) { return n; }
 
 // Lines per block: up to kFftMaxTile complex values staged (half that for the mixed-radix kernel, which
 // keeps two buffers: at 2 x 64 KB a block of the z pass left one block per SM and the FP64 pipe 55 %
@@ -867,14 +967,26 @@ int tile_lines_for(int n, long long st, long long nlines_total, int max_tile = k
   return t;
 }
 
+// Lengths 2^a 3^b 5^c that fit go through fft.cuh; the kernels above keep the rest: the radix-2 kernel powers of two
+// whose line fits shared memory once but not twice (FP64 8192), the other one lengths with larger prime factors.
 template <typename C>
 cudaError_t fft_lines_t(C* X, int n, long long st, long long total, int inverse, const C* tw, cudaStream_t stream) {
+  if (n == 1) return cudaSuccess;
   const long long nlines = total / n;
-  const bool mixed = !(is_pow2(n) && !GLASMA_FFT_POW2_STOCKHAM);
+  fft::Plan plan;
+  fft::Shape shape;
+  if (fft::make_plan(n, plan) && fft::make_shape(plan, st == 1, false, sizeof(C), st == 1 ? nlines : st, shape)) {
+    const fft::Scale<typename fft::Real<C>::type> none{};
+    if (st == 1)
+      return inverse ? fft::launch<C, true, true, false>(X, plan, shape, st, total, tw, none, stream)
+                     : fft::launch<C, false, true, false>(X, plan, shape, st, total, tw, none, stream);
+    return inverse ? fft::launch<C, true, false, false>(X, plan, shape, st, total, tw, none, stream)
+                   : fft::launch<C, false, false, false>(X, plan, shape, st, total, tw, none, stream);
+  }
+  const bool mixed = !is_pow2(n);
   const int tl = tile_lines_for(n, st, nlines, mixed ? kFftMaxTile / 2 : kFftMaxTile);
   const long long tiles = nlines / tl;
-  if (n == 1) return cudaSuccess;
-  if (is_pow2(n) && !GLASMA_FFT_POW2_STOCKHAM) {
+  if (!mixed) {
     const size_t smem = ((size_t)(n / 2) + (size_t)tl * (n + 1)) * sizeof(C);
     cudaFuncSetAttribute(fft_pow2_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     fft_pow2_kernel<C><<<(unsigned)tiles, kFftThreads, smem, stream>>>(X, ilog2(n), st, ilog2(tl), st > 1 ? st / tl : 0,
@@ -916,6 +1028,7 @@ struct GaugeFixState {
   double p2a[3] = {0, 0, 0};  // the spacings the table was made for
   std::map<int, double2*> twiddles;
   std::map<int, float2*> twiddles32;
+  double* A = nullptr;  // the FP64 sweeps' 27 numbers per site (link_deviation_kernel), on first use
   std::vector<double> host_results;
 };
 
@@ -930,6 +1043,39 @@ cudaError_t fft3d_t(const GaugeFixState* s, C* X, int planes, int inverse, const
   cudaError_t e = fft_lines_t<C>(X, g.nx, 1, total, inverse, tws.at(g.nx), stream);
   if (e == cudaSuccess) e = fft_lines_t<C>(X, g.ny, g.nx, total, inverse, tws.at(g.ny), stream);
   if (e == cudaSuccess) e = fft_lines_t<C>(X, g.nz, g.plane, total, inverse, tws.at(g.nz), stream);
+  return e;
+}
+
+// The acceleration step on the four colour-pair planes: forward transform, Delta(p) / (V p^2), inverse transform; along z
+// the three in one pass (fft.cuh) where that kernel takes the length.
+template <typename C>
+cudaError_t accelerate_planes(const GaugeFixState* s, C* X, const typename fft::Real<C>::type* tab, int project,
+                              const std::map<int, C*>& tws, cudaStream_t stream) {
+  typedef typename fft::Real<C>::type Re;
+  const Geometry& g = s->g;
+  const long long total = 4 * g.vol;
+  auto lines = [&](int n, long long st, int inverse) { return fft_lines_t<C>(X, n, st, total, inverse, tws.at(n), stream); };
+  cudaError_t e = lines(g.nx, 1, 0);
+  if (e == cudaSuccess) e = lines(g.ny, g.nx, 0);
+  if (e != cudaSuccess) return e;
+  fft::Plan plan;
+  fft::Shape shape;
+  if (g.nz > 1 && fft::make_plan(g.nz, plan) && fft::make_shape(plan, false, true, sizeof(C), g.plane, shape)) {
+    const fft::Scale<Re> sc = {g.nx, g.ny, (Re)g.vol, tab, project};
+    e = fft::launch<C, false, false, true>(X, plan, shape, g.plane, total, tws.at(g.nz), sc, stream);
+  } else {
+    e = lines(g.nz, g.plane, 0);
+    if (e != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)((total + 255) / 256);
+    if constexpr (sizeof(Re) == 4)
+      accelerate32_kernel<<<blocks, 256, 0, stream>>>(g.nx, g.ny, g.nz, (float)g.vol, tab, X, project);
+    else
+      accelerate_kernel<<<blocks, 256, 0, stream>>>(g.nx, g.ny, g.nz, (double)g.vol, tab, X, project);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = lines(g.nz, g.plane, 1);
+  }
+  if (e == cudaSuccess) e = lines(g.ny, g.nx, 1);
+  if (e == cudaSuccess) e = lines(g.nx, 1, 1);
   return e;
 }
 
@@ -1005,30 +1151,32 @@ int prepare(GaugeFixState** ps, const GaugeFixArgs& a, std::string* err) {
   return GLASMA_OK;
 }
 
-// CopyFields (S/GAUGETRANSFORMATION/GaugeTransformation.cpp:93-97): interior slices only
+// CopyFields (S/GAUGETRANSFORMATION/GaugeTransformation.cpp:93-97), interior slices: what it copies into UG and EG is
+// overwritten by the transforms that follow, except where the iteration ends on its guard.
 template <typename T>
-cudaError_t copy_fields(const GaugeFixArgs& a) {
+cudaError_t copy_efield(const GaugeFixArgs& a) {
   const Geometry& g = a.g;
-  const cx<T>* U = static_cast<const cx<T>*>(a.U);
-  const T* E = static_cast<const T*>(a.E);
-  cx<T>* UG = static_cast<cx<T>*>(a.UG);
-  T* EG = static_cast<T*>(a.EG);
-  cudaError_t e = cudaSuccess;
-  for (int c = 0; c < 27 && e == cudaSuccess; c++)
-    e = cudaMemcpyAsync(UG + (long long)c * g.S + g.plane, U + (long long)c * g.S + g.plane, sizeof(cx<T>) * g.vol,
-                        cudaMemcpyDeviceToDevice, a.stream);
-  for (int c = 0; c < 24 && e == cudaSuccess; c++)
-    e = cudaMemcpyAsync(EG + (long long)c * g.S + g.plane, E + (long long)c * g.S + g.plane, sizeof(T) * g.vol,
-                        cudaMemcpyDeviceToDevice, a.stream);
-  return e;
+  return cudaMemcpy2DAsync(static_cast<T*>(a.EG) + g.plane, sizeof(T) * g.S, static_cast<const T*>(a.E) + g.plane,
+                           sizeof(T) * g.S, sizeof(T) * g.vol, 24, cudaMemcpyDeviceToDevice, a.stream);
+}
+// UG from U and G
+template <typename T>
+cudaError_t transform_links_only(const GaugeFixArgs& a) {
+  const dim3 tb((unsigned)((a.g.vol + kLinkThreads - 1) / kLinkThreads), 3);
+  transform_links_kernel<T><<<tb, kLinkThreads, 0, a.stream>>>(a.g, static_cast<const cx<T>*>(a.U),
+                                                      static_cast<const cx<T>*>(a.G), static_cast<cx<T>*>(a.UG));
+  return cudaGetLastError();
+}
+template <typename T>
+cudaError_t copy_links(const GaugeFixArgs& a) {
+  const Geometry& g = a.g;
+  return cudaMemcpy2DAsync(static_cast<cx<T>*>(a.UG) + g.plane, sizeof(cx<T>) * g.S, static_cast<const cx<T>*>(a.U) + g.plane,
+                           sizeof(cx<T>) * g.S, sizeof(cx<T>) * g.vol, 27, cudaMemcpyDeviceToDevice, a.stream);
 }
 // GaugeTransformLinks: UG from U and G, then the ghost slices of G
 template <typename T>
 cudaError_t transform_links_all(const GaugeFixArgs& a) {
-  const unsigned tb = (unsigned)((a.g.vol + 127) / 128);
-  transform_links_kernel<T><<<tb, 128, 0, a.stream>>>(a.g, static_cast<const cx<T>*>(a.U),
-                                                      static_cast<const cx<T>*>(a.G), static_cast<cx<T>*>(a.UG));
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = transform_links_only<T>(a);
   if (e == cudaSuccess) e = launch_sync_ghosts<cx<T>>(a.g, static_cast<cx<T>*>(a.G), 9, a.stream);
   return e;
 }
@@ -1037,8 +1185,8 @@ template <typename T>
 cudaError_t finish_fields(const GaugeFixArgs& a) {
   cudaError_t e = transform_links_all<T>(a);
   if (e != cudaSuccess) return e;
-  const unsigned tb = (unsigned)((a.g.vol + 127) / 128);
-  transform_efield_kernel<T><<<tb, 128, 0, a.stream>>>(a.g, static_cast<const T*>(a.E),
+  const dim3 tb((unsigned)((a.g.vol + kLinkThreads - 1) / kLinkThreads), 3);
+  transform_efield_kernel<T><<<tb, kLinkThreads, 0, a.stream>>>(a.g, static_cast<const T*>(a.E),
                                                        static_cast<const cx<T>*>(a.G), static_cast<T*>(a.EG));
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = launch_sync_ghosts<cx<T>>(a.g, static_cast<cx<T>*>(a.G), 9, a.stream)) != cudaSuccess) return e;
@@ -1059,9 +1207,24 @@ int run_impl(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_iter
     return GLASMA_ERR_CUDA;
   };
   cudaError_t e;
-  if (n_start == 0 && (e = copy_fields<T>(a)) != cudaSuccess) return cuda_err(e, "copy fields");
-  auto transform_links = [&]() { return transform_links_all<T>(a); };
-  if ((e = transform_links()) != cudaSuccess) return cuda_err(e, "transform links");
+  const bool sweeps = n_start < max_iters && tol < 1.0;
+  // The sweeps read 27 numbers of UG per site (A); without room for them they go over UG itself.
+  if (sweeps && !s->A && cudaMalloc(&s->A, sizeof(double) * 27 * g.vol) != cudaSuccess) {
+    cudaGetLastError();
+    s->A = nullptr;
+  }
+  double* const A = s->A;
+  const dim3 lb((unsigned)((g.vol + kLinkThreads - 1) / kLinkThreads), 3);
+  // GaugeTransformLinks reads the ghost G of the sweep before, then the ghosts are synced: the sync waits for the sweep's
+  // verdict, so that a failing one can still leave its UG
+  auto transform_links = [&]() {
+    if (!A) return transform_links_only<T>(a);
+    link_deviation_kernel<T><<<lb, kLinkThreads, 0, st>>>(g, static_cast<const cx<T>*>(a.U), G, A);
+    return cudaGetLastError();
+  };
+  auto sync_gauge = [&]() { return launch_sync_ghosts<cx<T>>(g, G, 9, st); };
+  if (sweeps && (e = transform_links()) != cudaSuccess) return cuda_err(e, "transform links");
+  if ((e = sync_gauge()) != cudaSuccess) return cuda_err(e, "sync gauge");
 
   const double cw[3] = {(a.a_scale / g.a[0]) * (a.a_scale / g.a[0]), (a.a_scale / g.a[1]) * (a.a_scale / g.a[1]),
                         g.nz > 1 ? (a.a_scale / g.a[2]) * (a.a_scale / g.a[2]) : 0.0};
@@ -1079,27 +1242,24 @@ int run_impl(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_iter
   if ((e = ensure_p2tab(s, g, st)) != cudaSuccess) return cuda_err(e, "momentum table");
   double2* X64 = static_cast<double2*>(s->X);
   float2* X32 = static_cast<float2*>(s->X);
-  const long long tot = 4 * g.vol;
   const int project = (flags & GLASMA_GF_PROJECT_ZERO_MODE) ? 1 : 0;
   const int open_top = (flags & GLASMA_GF_OPEN_Z) ? 1 : 0;
   while (n < max_iters && gmax > tol) {
-    if (fft32)
+    if (A && fft32)
+      gather_deviation_kernel<double, float2><<<nb, kGfThreads, 0, st>>>(g, A, cw[0], cw[1], cw[2], 3.0, X32, part_dev,
+                                                                         open_top);
+    else if (A)
+      gather_deviation_kernel<double, double2><<<nb, kGfThreads, 0, st>>>(g, A, cw[0], cw[1], cw[2], 3.0, X64, part_dev,
+                                                                          open_top);
+    else if (fft32)
       deviation_kernel<T, float2><<<nb, kGfThreads, 0, st>>>(g, UG, cw[0], cw[1], cw[2], X32, part_dev, open_top);
     else
       deviation_kernel<T, double2><<<nb, kGfThreads, 0, st>>>(g, UG, cw[0], cw[1], cw[2], X64, part_dev, open_top);
     red::finish_kernel<4><<<1, red::kThreads, 0, st>>>(part_dev, (int)nb, 1 | (0 << 2) | (2 << 4) | (0 << 6), res);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "deviation");
-    e = fft32 ? fft3d_t<float2>(s, X32, 4, 0, s->twiddles32, st) : fft3d_t<double2>(s, X64, 4, 0, s->twiddles, st);
-    if (e != cudaSuccess) return cuda_err(e, "fft forward");
-    if (fft32)
-      accelerate32_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(g.nx, g.ny, g.nz, (float)g.vol, s->p2tab32, X32,
-                                                                         project);
-    else
-      accelerate_kernel<double2><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(g.nx, g.ny, g.nz, (double)g.vol, s->p2tab,
-                                                                          X64, project);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "accelerate");
-    e = fft32 ? fft3d_t<float2>(s, X32, 4, 1, s->twiddles32, st) : fft3d_t<double2>(s, X64, 4, 1, s->twiddles, st);
-    if (e != cudaSuccess) return cuda_err(e, "fft backward");
+    e = fft32 ? accelerate_planes<float2>(s, X32, s->p2tab32, project, s->twiddles32, st)
+              : accelerate_planes<double2>(s, X64, s->p2tab, project, s->twiddles, st);
+    if (e != cudaSuccess) return cuda_err(e, "acceleration");
     if (fft32)
       update_kernel<T, float2><<<nb, kGfThreads, 0, st>>>(g, X32, G, alpha, part_upd);
     else
@@ -1126,8 +1286,12 @@ int run_impl(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_iter
     if (h[6] > 0.0) {
       *err = "gauge update left SU(3) by more than 1e-13 (the reference exits here)";
       status = GLASMA_ERR_NUMERICAL;
-      break;
+      if (A) e = transform_links_only<T>(a);
+      if (e == cudaSuccess) e = copy_efield<T>(a);
+      if (e != cudaSuccess) return cuda_err(e, "fields at the guard");
     }
+    if ((e = sync_gauge()) != cudaSuccess) return cuda_err(e, "sync gauge");
+    if (status != GLASMA_OK) break;
   }
   *iterations = n;
   if (status != GLASMA_OK) return status;
@@ -1145,13 +1309,13 @@ constexpr float kMixedGuard = 1e-5f;   // unitarity guard of the FP32 update
 struct Fp32Copies {
   cx<float>* U = nullptr;
   cx<float>* G = nullptr;
-  cx<float>* UG = nullptr;
+  float* A = nullptr;  // link_deviation32_kernel's 27 numbers per site
   cudaStream_t stream = nullptr;
   ~Fp32Copies() {
     if (stream) cudaStreamSynchronize(stream);
     cudaFree(U);
     cudaFree(G);
-    cudaFree(UG);
+    cudaFree(A);
   }
 };
 
@@ -1167,18 +1331,17 @@ int run_mixed(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_ite
   c.stream = st;
   cudaError_t e = cudaMalloc(&c.U, sizeof(cx<float>) * 27 * g.S);
   if (e == cudaSuccess) e = cudaMalloc(&c.G, sizeof(cx<float>) * 9 * g.S);
-  if (e == cudaSuccess) e = cudaMalloc(&c.UG, sizeof(cx<float>) * 27 * g.S);
+  if (e == cudaSuccess) e = cudaMalloc(&c.A, sizeof(float) * 27 * g.vol);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *err = std::string("cudaMalloc FP32 gauge-fixing copies: ") + cudaGetErrorString(e);
     return GLASMA_ERR_OUT_OF_MEMORY;
   }
-  if ((e = copy_fields<double>(a)) != cudaSuccess) return cuda_err(e, "copy fields");
   narrow_kernel<<<(unsigned)((27 * g.S + 255) / 256), 256, 0, st>>>(static_cast<const cx<double>*>(a.U), c.U, 27 * g.S);
   narrow_kernel<<<(unsigned)((9 * g.S + 255) / 256), 256, 0, st>>>(static_cast<const cx<double>*>(a.G), c.G, 9 * g.S);
-  const unsigned tb = (unsigned)((g.vol + 127) / 128);
+  const dim3 lb((unsigned)((g.vol + kLinkThreads - 1) / kLinkThreads), 3);
   auto transform32 = [&]() {
-    transform_links32_kernel<<<tb, 128, 0, st>>>(g, c.U, c.G, c.UG);
+    link_deviation32_kernel<<<lb, kLinkThreads, 0, st>>>(g, c.U, c.G, c.A);
     cudaError_t x = cudaGetLastError();
     if (x == cudaSuccess) x = launch_sync_ghosts<cx<float>>(g, c.G, 9, st);
     return x;
@@ -1195,21 +1358,18 @@ int run_mixed(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_ite
   double* res = a.scratch + (size_t)nb * 7;
   const double minf0 = 2.0 * 3 * (1.0 / (g.a[0] * g.a[0]) + 1.0 / (g.a[1] * g.a[1]) + 1.0 / (g.a[2] * g.a[2]));
   float2* X32 = static_cast<float2*>(s->X);
-  const long long tot = 4 * g.vol;
   const int project = (flags & GLASMA_GF_PROJECT_ZERO_MODE) ? 1 : 0;
   const int open_top = (flags & GLASMA_GF_OPEN_Z) ? 1 : 0;
   double h[8];
   double gmax = 1.0, best = 1e300;
   int n = 0, since_best = 0;
   while (n < max_iters && gmax > tol) {
-    deviation32_kernel<<<nb, kGfThreads, 0, st>>>(g, c.UG, cw[0], cw[1], cw[2], X32, part_dev, open_top);
+    gather_deviation_kernel<float, float2><<<nb, kGfThreads, 0, st>>>(g, c.A, cw[0], cw[1], cw[2], 0.f, X32, part_dev,
+                                                                       open_top);
     red::finish_kernel<4><<<1, red::kThreads, 0, st>>>(part_dev, (int)nb, 1 | (0 << 2) | (2 << 4) | (0 << 6), res);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "FP32 deviation");
-    if ((e = fft3d_t<float2>(s, X32, 4, 0, s->twiddles32, st)) != cudaSuccess) return cuda_err(e, "fft forward");
-    accelerate32_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(g.nx, g.ny, g.nz, (float)g.vol, s->p2tab32, X32,
-                                                                         project);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "accelerate");
-    if ((e = fft3d_t<float2>(s, X32, 4, 1, s->twiddles32, st)) != cudaSuccess) return cuda_err(e, "fft backward");
+    if ((e = accelerate_planes<float2>(s, X32, s->p2tab32, project, s->twiddles32, st)) != cudaSuccess)
+      return cuda_err(e, "acceleration");
     update32_kernel<<<nb, kGfThreads, 0, st>>>(g, X32, c.G, (float)alpha, part_upd, kMixedGuard);
     red::finish_kernel<3><<<1, red::kThreads, 0, st>>>(part_upd, (int)nb, 1 | (0 << 2) | (0 << 4), res + 4);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "FP32 update");
@@ -1233,6 +1393,9 @@ int run_mixed(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_ite
     if (h[6] > 0.0) {
       *iterations = n;
       *err = "FP32 gauge update left SU(3) by more than 1e-5";
+      e = copy_links<double>(a);
+      if (e == cudaSuccess) e = copy_efield<double>(a);
+      if (e != cudaSuccess) return cuda_err(e, "fields at the guard");
       return GLASMA_ERR_NUMERICAL;
     }
     if (gmax < 0.95 * best) {
@@ -1270,7 +1433,7 @@ int run_local_impl(const GaugeFixArgs& a, int los_alamos, double param, unsigned
     return GLASMA_ERR_CUDA;
   };
   cudaError_t e;
-  if ((e = copy_fields<T>(a)) != cudaSuccess) return cuda_err(e, "copy fields");
+  if ((e = copy_efield<T>(a)) != cudaSuccess) return cuda_err(e, "copy fields");
   if ((e = transform_links_all<T>(a)) != cudaSuccess) return cuda_err(e, "transform links");
   const double cw[3] = {(a.a_scale / g.a[0]) * (a.a_scale / g.a[0]), (a.a_scale / g.a[1]) * (a.a_scale / g.a[1]),
                         g.nz > 1 ? (a.a_scale / g.a[2]) * (a.a_scale / g.a[2]) : 0.0};
@@ -1373,6 +1536,7 @@ cudaError_t launch_transform_charge(const GaugeFixArgs& a, const void* J, double
 void gaugefix_destroy(GaugeFixState* s) {
   if (!s) return;
   if (s->X) cudaFree(s->X);
+  if (s->A) cudaFree(s->A);
   if (s->p2tab) cudaFree(s->p2tab);
   if (s->p2tab32) cudaFree(s->p2tab32);
   for (auto& kv : s->twiddles) cudaFree(kv.second);
