@@ -46,6 +46,13 @@ struct DevBuf {
   bool alloc(size_t bytes) { return cudaMalloc(&p, bytes) == cudaSuccess; }
 };
 
+// One write to every page of a host array that is about to be overwritten.
+void touch_pages(double* p, size_t bytes) {
+  volatile char* c = reinterpret_cast<volatile char*>(p);
+  for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+  if (bytes) c[bytes - 1] = 0;
+}
+
 double ratio(const double* num, const double* den, const double* q, double* Nout, double* Dout) {
   double N = 0.0, D = 0.0;
   bool has_den = false;

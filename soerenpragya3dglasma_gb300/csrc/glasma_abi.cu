@@ -509,6 +509,17 @@ static void* mapped_host(const void* p) {
   return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
+// Whether p is memory of the handle's own GPU: the layout kernels then read or write it in place, where other device
+// memory goes through the staging buffer and a copy (two more passes over the field).
+static bool own_device(const glasma_lattice* h, const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == h->device && reinterpret_cast<size_t>(p) % sizeof(double) == 0;
+}
+
 static int upload_common(glasma_lattice* h, int field, const double* src, cudaMemcpyKind kind) {
   GLASMA_CHECK_HANDLE(h);
   if (!valid_field(field)) return fail(GLASMA_ERR_INVALID_ARGUMENT, "unknown field");
@@ -524,6 +535,12 @@ static int upload_common(glasma_lattice* h, int field, const double* src, cudaMe
                           : glasma::launch_aos_to_soa<float>(dsrc, static_cast<float*>(h->f[field]), h->g.S, P, h->stream);
       return e == cudaSuccess ? GLASMA_OK : cuda_fail(e, "aos_to_soa from host");
     }
+  }
+  if (kind == cudaMemcpyDeviceToDevice && own_device(h, src)) {
+    cudaError_t e = h->precision == GLASMA_FP64
+                        ? glasma::launch_aos_to_soa<double>(src, static_cast<double*>(h->f[field]), h->g.S, P, h->stream)
+                        : glasma::launch_aos_to_soa<float>(src, static_cast<float*>(h->f[field]), h->g.S, P, h->stream);
+    return e == cudaSuccess ? GLASMA_OK : cuda_fail(e, "aos_to_soa from device");
   }
   st = ensure_staging(h, bytes);
   if (st) return st;
@@ -552,6 +569,14 @@ static int download_common(glasma_lattice* h, int field, double* dst, cudaMemcpy
       GLASMA_CUDA(cudaStreamSynchronize(h->stream), "download sync");
       return GLASMA_OK;
     }
+  }
+  if (kind == cudaMemcpyDeviceToDevice && own_device(h, dst)) {
+    cudaError_t e = h->precision == GLASMA_FP64
+                        ? glasma::launch_soa_to_aos<double>(static_cast<const double*>(h->f[field]), dst, h->g.S, P, h->stream)
+                        : glasma::launch_soa_to_aos<float>(static_cast<const float*>(h->f[field]), dst, h->g.S, P, h->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "soa_to_aos to device");
+    GLASMA_CUDA(cudaStreamSynchronize(h->stream), "download sync");
+    return GLASMA_OK;
   }
   st = ensure_staging(h, bytes);
   if (st) return st;

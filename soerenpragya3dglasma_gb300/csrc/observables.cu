@@ -183,8 +183,9 @@ __device__ __forceinline__ float plaq_sqdiff_f(const cx<float>* __restrict__ U, 
   return d2;
 }
 
-// n(u) = ||u||_F^2 - 3 in FP64 (every float x float product is exact in FP64)
-__device__ __forceinline__ double link_norm_dev(const cx<float>* __restrict__ U, long long S, int mu, long long s) {
+// n(u) = ||u||_F^2 - 3, in fixed point (fx.cuh: the squares to 2^-58, below FP64's rounding at 3) on the integer pipe:
+// in FP64 its conversions and fmas bound the FP32 bulk energy
+__device__ __noinline__ double link_norm_dev_fp64(const cx<float>* U, long long S, int mu, long long s) {
   const cx<float>* p = U + (long long)(mu * 9) * S + s;
   double n = -3.0;
 #pragma unroll
@@ -193,6 +194,43 @@ __device__ __forceinline__ double link_norm_dev(const cx<float>* __restrict__ U,
     n = fma((double)v.re, (double)v.re, fma((double)v.im, (double)v.im, n));
   }
   return n;
+}
+__device__ __forceinline__ double link_norm_dev(const cx<float>* __restrict__ U, long long S, int mu, long long s) {
+  const cx<float>* p = U + (long long)(mu * 9) * S + s;
+  fx::Acc a = fx::acc_half();
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const cx<float> v = p[(long long)k * S];
+    top = max(top, max(fx::habs(v.re), fx::habs(v.im)));
+    const fx::R re = fx::to_fixed_split(fabsf(v.re), fx::shift(fx::kScale)), im = fx::to_fixed_split(fabsf(v.im), fx::shift(fx::kScale));
+    fx::mad(a, re, re);
+    fx::mad(a, im, im);
+  }
+  // entries up to 1.03 only: eighteen squares up to 19 would leave the format's +-8 (they wrap in the 64-bit sum, which is
+  // exact again after the subtraction for every matrix whose norm^2 is below 11)
+  if (top > fx::kMaxEntryHi) return link_norm_dev_fp64(U, S, mu, s);
+  return fx::from_fixed(fx::finish(a) - 3 * (1LL << fx::kScale), -fx::kScale);
+}
+// sum of squares of eight FP32 components, to 2^-58 of it
+__device__ __forceinline__ double squares(const Alg<float>& e) {
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) top = max(top, fx::habs(e.a[k]));
+  if (top >= 0x43100000 || top < ((1023 - 100) << 20)) {  // beyond 2^50 or below 2^-100: FP64
+    double q = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) q = fma((double)e.a[k], (double)e.a[k], q);
+    return q;
+  }
+  const int em = fx::exponent_of(top) + 1, sh = fx::shift(fx::kScale - em);
+  fx::Acc a = fx::acc_half();
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const fx::R r = fx::to_fixed_split(fabsf(e.a[k]), sh);
+    fx::mad(a, r, r);
+  }
+  return fx::from_fixed(fx::finish(a), 2 * em - fx::kScale);
 }
 
 // Site arithmetic of the FP64 sums on the integer pipe (fx.cuh): the magnetic terms are -Re tr(P - 1) from products of
@@ -323,20 +361,17 @@ __global__ void __launch_bounds__(kRedThreads) bulk_kernel(Geometry g, FieldPtrs
     v[0] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 1, 2, s, syp, szp) - 2.0 * (2.0 * nz + wz * ny + gy);
     v[1] += 2.0 * (double)plaq_sqdiff_f(f.U, S, 2, 0, s, szp, sxp) - 2.0 * (2.0 * nz + wz * nx + gx);
     for (int mu = 0; mu < 3; mu++) {
-      Alg<double> e;
-      load_alg_d(f.E, S, mu * 8, s, e);
-      double q = 0.0;
-#pragma unroll
-      for (int k = 0; k < 8; k++) q += e.a[k] * e.a[k];
-      v[3 + mu] += q;
+      Alg<float> e;
+      load_alg<float, long long>(f.E, S, mu * 8, s, e);
+      v[3 + mu] += squares(e);
       if (mu == 2) {
-        Alg<double> jp, jm;
-        load_alg_d(f.Jp, S, 0, s, jp);
-        load_alg_d(f.Jm, S, 0, s, jm);
+        Alg<float> jp, jm;
+        load_alg<float, long long>(f.Jp, S, 0, s, jp);
+        load_alg<float, long long>(f.Jm, S, 0, s, jm);
         double w = 0.0;
 #pragma unroll
-        for (int k = 0; k < 8; k++) w += e.a[k] * (jp.a[k] - jm.a[k]) * 0.70710678118654752440084436210484903928483593768847;
-        v[6] += w;
+        for (int k = 0; k < 8; k++) w += (double)e.a[k] * ((double)jp.a[k] - (double)jm.a[k]);
+        v[6] += w * 0.70710678118654752440084436210484903928483593768847;
       }
     }
   }

@@ -626,15 +626,16 @@ __device__ __forceinline__ float add_stochastic(float a, float b, unsigned salt)
   const float s = a + b, bb = s - a;
   const float r = (a - (s - bb)) + (b - bb);
   if (r == 0.f) return s;
-  const float t = nextafterf(s, r > 0.f ? 3.0e38f : -3.0e38f);
-  const float p = fabsf(r / (t - s));
+  // the neighbour of s (not zero: r is then) on r's side; u < |r| / gap as u gap < |r|, without the division
+  const float t = __int_as_float(__float_as_int(s) + ((r > 0.f) == (s > 0.f) ? 1 : -1));
+  const float gap = fabsf(t - s);
   unsigned h = (__float_as_uint(a) * 0x9E3779B1u) ^ (__float_as_uint(b) * 0x85EBCA77u) ^ salt;
   h ^= h >> 15;
   h *= 0x2C1B3C6Du;
   h ^= h >> 12;
   h *= 0x297A2D39u;
   h ^= h >> 15;
-  return (float)(h >> 8) * (1.f / 16777216.f) < p ? t : s;
+  return (float)(h >> 8) * (1.f / 16777216.f) * gap < fabsf(r) ? t : s;
 }
 // out = (1 + Xm1) u.  In FP32 the real parts of the diagonal are added with stochastic rounding: near
 // the identity they receive only the second-order -(Q^2)_ii/2 per step (the first-order i Q u is
