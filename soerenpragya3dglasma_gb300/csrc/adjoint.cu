@@ -70,6 +70,63 @@ double ratio(const double* num, const double* den, const double* q, double* Nout
 }  // namespace
 
 namespace glasma {
+// The FP64 kernels' rotations, plaquettes and exponential pull-back in fixed point on the integer pipe (fx.cuh): true when
+// its numbers held the operands.  FP32 has its own pipe and always answers false.
+template <bool kAdj, typename R>
+__device__ __forceinline__ bool fixed_rotated(const cx<R>* U, long long S, int mu, long long s, const Alg<R>& e, Alg<R>& o) {
+  if constexpr (sizeof(R) == 8) {
+    fx::Guard g = fx::guard_init();
+    fx::M v, h;
+    int eh;
+    fx::ll q[8];
+    fx::link_plain<kAdj>(U, S, mu, s, v, g);  // Adj(V) = InvAdj(V^d)
+    fx::herm_one(e, h, eh, g);
+    fx::rotate_one(v, h, q, g);
+    fx::to_alg(q, eh - fx::kScale - 1, 1.0, o);
+    return !fx::tripped(g);
+  }
+  return false;
+}
+template <bool kAdj, typename R>
+__device__ __forceinline__ bool fixed_rotated_pair(const cx<R>* U, long long S, int mu, long long s, const Alg<R>& e1,
+                                                   const Alg<R>& e2, Alg<R>& o1, Alg<R>& o2) {
+  if constexpr (sizeof(R) == 8) {
+    fx::Guard g = fx::guard_init();
+    fx::M v;
+    fx::link_plain(U, S, mu, s, v, g);
+    fx::adj_pair<!kAdj>(v, e1, e2, o1, o2, g);
+    return !fx::tripped(g);
+  }
+  return false;
+}
+template <typename R>
+__device__ __forceinline__ bool fixed_plaquette(const cx<R>* U, long long S, int p, int q, long long sa, long long sb,
+                                                long long sc, Mat<R>& h, Alg<R>& al) {
+  if constexpr (sizeof(R) == 8) {
+    fx::Guard g = fx::guard_init();
+    fx::M a, b, w, v;
+    int ea, eb, ew, ev;
+    fx::link_near(U, S, p, sa, a, ea, g);
+    fx::link_near(U, S, q, sb, b, eb, g);
+    fx::near_product(a, ea, b, eb, w, ew, g);
+    fx::link_near(U, S, q, sa, a, ea, g);
+    fx::link_near(U, S, p, sc, b, eb, g);
+    fx::near_product(a, ea, b, eb, v, ev, g);
+    fx::Anti t;
+    fx::plaquette_full(w, ew, v, ev, t, h);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      al.a[k] = fx::from_fixed(fx::component(t, k), t.e - fx::kScale) * (k == 7 ? -0.5 * Consts<double>::inv_sqrt3() : -0.5);
+    return !fx::tripped(g);
+  }
+  return false;
+}
+template <typename R>
+__device__ __forceinline__ bool fixed_series(const Alg<R>& q, const Alg<R>& l, int terms, const R* inv, Alg<R>& o) {
+  if constexpr (sizeof(R) == 8) return fx::exp_series(q, l, terms, inv, o);
+  return false;
+}
+
 namespace adj64 {
 #define ADJ_REAL double
 #include "adjoint_kernels.inc"

@@ -806,5 +806,124 @@ __device__ __forceinline__ bool add_product(const M& a, int ea, const Mat<double
   return !g.bad;
 }
 
+// P - 1 of P = (1 + w)(1 + v)^dagger in full: its anti-Hermitian part, and the Hermitian part h of P - 1 as doubles
+// (h_ij, i <= j).
+__device__ __forceinline__ void plaquette_full(const M& W, int ew, const M& V, int ev, Anti& o, Mat<double>& h) {
+  const int ep = max(ew, ev);
+  const int k = min(ep - ew - ev, 63), kw = min(ep - ew, 63), kv = min(ep - ev, 63);
+  o.e = ep;
+  R nV[9];
+#pragma unroll
+  for (int n = 0; n < 9; n++) nV[n] = neg(V.e[n].im);
+  auto entry = [&](int i, int j, ll& re, ll& im) {
+    Acc a = acc_half(), b = acc_half();
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+      const C& w = W.e[i + 3 * t];
+      mad(a, w.re, V.e[j + 3 * t].re);
+      mad(a, w.im, V.e[j + 3 * t].im);
+      mad(b, w.im, V.e[j + 3 * t].re);
+      mad(b, w.re, nV[j + 3 * t]);
+    }
+    re = (finish(a) >> k) + (join(W.e[i + 3 * j].re) >> kw) + (join(V.e[j + 3 * i].re) >> kv);
+    im = (finish(b) >> k) + (join(W.e[i + 3 * j].im) >> kw) - (join(V.e[j + 3 * i].im) >> kv);
+  };
+  constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
+#pragma unroll
+  for (int n = 0; n < 3; n++) {
+    const int i = pi[n], j = pj[n];
+    ll ru, iu, rl, il;
+    entry(i, j, ru, iu);
+    entry(j, i, rl, il);
+    o.y[n] = iu + il;
+    o.x[n] = ru - rl;
+    h.e[i + 3 * j] = mk<double>(from_fixed(ru + rl, ep - kScale - 1), from_fixed(iu - il, ep - kScale - 1));
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    ll r, m;
+    entry(i, i, r, m);
+    o.d[i] = m;
+    h.e[4 * i] = mk<double>(from_fixed(r, ep - kScale), 0.0);
+  }
+}
+
+// sum_n (q x)^n l / (n + 1)! in fixed point (x the structure-constant product), n up to `terms`; inv[n] = 1 / n.  |q| below one
+// in every component.  With the eighth components times sqrt 3 every structure constant but f^123 is 1/2.
+__device__ __forceinline__ bool exp_series(const Alg<double>& q, const Alg<double>& l, int terms, const double* inv,
+                                           Alg<double>& out) {
+  const double r3 = 1.7320508075688772935;
+  int tq = 0, tl = 0;
+  Alg<double> qs = q, ls = l;
+  qs.a[7] *= r3;
+  ls.a[7] *= r3;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    tq = max(tq, habs(qs.a[k]));
+    tl = max(tl, habs(ls.a[k]));
+  }
+  if (tq >= 0x40000000 || tl >= 0x43100000) return false;  // 2; 2^50 or more, or not finite
+  const int eq = max(exponent_of(tq), kMinExp), el = max(exponent_of(tl), kMinExp) + 1;
+  const int down = min(-min(eq, 0), 63), up = max(eq, 0);
+  R Q[8], T[8];
+  ll sum[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    Q[k] = to_fixed_split(qs.a[k], shift(kScale - eq));
+    sum[k] = to_fixed(ls.a[k], shift(kScale - el));
+    T[k] = split(sum[k]);
+  }
+#pragma unroll 1
+  for (int n = 1; n <= terms; n++) {
+    R N[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) N[k] = neg(T[k]);
+    auto d = [&](Acc& a, int i, int j) {  // Q_i T_j - Q_j T_i
+      mad(a, Q[i - 1], T[j - 1]);
+      mad(a, Q[j - 1], N[i - 1]);
+    };
+    ll c[8];
+    {
+      Acc a = acc_half(), b = acc_half();
+      d(a, 2, 3), d(b, 4, 7), d(b, 6, 5);
+      c[0] = finish(a) + (finish(b) >> 1);
+      a = b = acc_half();
+      d(a, 3, 1), d(b, 4, 6), d(b, 5, 7);
+      c[1] = finish(a) + (finish(b) >> 1);
+      a = b = acc_half();
+      d(a, 1, 2), d(b, 4, 5), d(b, 7, 6);
+      c[2] = finish(a) + (finish(b) >> 1);
+      a = acc_half();
+      d(a, 7, 1), d(a, 6, 2), d(a, 5, 3), d(a, 5, 8);
+      c[3] = finish(a) >> 1;
+      a = acc_half();
+      d(a, 1, 6), d(a, 7, 2), d(a, 3, 4), d(a, 8, 4);
+      c[4] = finish(a) >> 1;
+      a = acc_half();
+      d(a, 5, 1), d(a, 2, 4), d(a, 3, 7), d(a, 7, 8);
+      c[5] = finish(a) >> 1;
+      a = acc_half();
+      d(a, 1, 4), d(a, 2, 5), d(a, 6, 3), d(a, 8, 6);
+      c[6] = finish(a) >> 1;
+      a = acc_half();
+      d(a, 4, 5), d(a, 6, 7);
+      const ll r = finish(a);
+      c[7] = r + (r >> 1);
+    }
+    const R f = to_fixed_split(inv[n + 1], shift(kScale));
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      Acc a = acc_half();
+      mad(a, split((c[k] >> down) << up), f);
+      const ll t = finish(a);
+      T[k] = split(t);
+      sum[k] += t;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) out.a[k] = from_fixed(sum[k], el - kScale) * (k == 7 ? 1.0 / 3.0 * r3 : 1.0);
+  return true;
+}
+
 }  // namespace fx
 }  // namespace glasma
