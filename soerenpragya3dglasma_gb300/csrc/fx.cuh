@@ -152,9 +152,7 @@ __device__ __forceinline__ double from_fixed_fp64(ll q, int k) {
   const double v = (hi - 19342822341709703277445120.0) + lo;  // 2^84 + 2^63 + 2^52
   return q == 0 ? 0.0 : __hiloint2double(__double2hiint(v) + (int)((unsigned)k << 20), __double2loint(v));
 }
-// 2^k as a double, -1022 <= k <= 1023
-__device__ __forceinline__ double pow2(int k) { return __hiloint2double((k + 1023) << 20, 0); }
-constexpr int kMinExp = -400;  // smaller values are held at 2^-460
+constexpr int kMinExp = -900;  // smaller values are held at 2^-960
 // |v| < 2^exponent_of(largest |high word| of v)
 __device__ __forceinline__ int exponent_of(int habs) { return (habs >> 20) - 1022; }
 constexpr int kMaxEntryHi = 0x3FF07AE1;  // 1.03
@@ -207,7 +205,7 @@ __device__ __forceinline__ void link_near(const cx<T>* __restrict__ U, I S, int 
     }
   }
   g.bad |= max(top, topd) > kMaxEntryHi;
-  const int ed = 64 - __clzll(dor) - kScale;  // |diagonal - 1| < 2^ed
+  const int ed = dor == 0 ? kMinExp : 64 - __clzll(dor) - kScale;  // |diagonal - 1| < 2^ed
   int ee = max(max(exponent_of(top), ed), kMinExp);
   ee = min(ee, 0);
   e = ee;
@@ -386,9 +384,9 @@ __device__ __forceinline__ ll plaquette_trace(const M& W, int ew, const M& V, in
   return -((finish(a) >> min(ep - ew - ev, 63)) + (w >> min(ep - ew, 63)) + (v >> min(ep - ev, 63)));
 }
 
-// M = H(p) + i H(q) with H_ij = y_ij - i x_ij, H_ji its conjugate (i < j), H_ii = 2 d_i: H(p) is -4 t.al up to a
-// multiple of 1, which a rotation leaves alone.  Exponent e; the two exponents may differ.
-__device__ __forceinline__ void herm_pair(const Anti& p, const Anti& q, M& m, int& e, ll& tr_re, ll& tr_im) {
+// M = H(p) + i H(q) with H_ij = y_ij - i x_ij, H_ji its conjugate (i < j), H_ii = 2 d_i - 2/3 sum d: H(p) = -4 t.al.
+// Exponent e; the two exponents may differ.
+__device__ __forceinline__ void herm_pair(const Anti& p, const Anti& q, M& m, int& e) {
   const int em = max(p.e, q.e) + 1;
   const int kp = min(em - p.e, 63), kq = min(em - q.e, 63);
   e = em;
@@ -402,22 +400,22 @@ __device__ __forceinline__ void herm_pair(const Anti& p, const Anti& q, M& m, in
     m.e[j + 3 * i].re = split(y1 - x2);
     m.e[j + 3 * i].im = split(y2 + x1);
   }
-  tr_re = tr_im = 0;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const ll a = p.d[i] >> (kp - 1), b = q.d[i] >> (kq - 1);
-    m.e[4 * i].re = split(a);
-    m.e[4 * i].im = split(b);
-    tr_re += a;
-    tr_im += b;
-  }
+  constexpr ll third = 0x5555555555555556LL;
+  const ll tp = __mul64hi(p.d[0] + p.d[1] + p.d[2], third), tq = __mul64hi(q.d[0] + q.d[1] + q.d[2], third);
+  const ll a0 = (p.d[0] - tp) >> (kp - 1), a1 = (p.d[1] - tp) >> (kp - 1);
+  const ll b0 = (q.d[0] - tq) >> (kq - 1), b1 = (q.d[1] - tq) >> (kq - 1);
+  m.e[0].re = split(a0);
+  m.e[0].im = split(b0);
+  m.e[4].re = split(a1);
+  m.e[4].im = split(b1);
+  m.e[8].re = split(-a0 - a1);
+  m.e[8].im = split(-b0 - b1);
 }
 
 // The Hermitian and anti-Hermitian parts of C = V^dagger M V (kInv) or V M V^dagger, as split_herm_pair gives them
-// (the last of each without its 1/sqrt(3)); V plain, in units of M.  tr: the trace of M (C_22 follows from it).
+// (the last of each without its 1/sqrt(3)); V plain, in units of M.  M is traceless, and C_22 follows from that.
 template <bool kInv>
-__device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll tr_re, ll tr_im, ll (&o1)[8], ll (&o2)[8],
-                                            Guard& g) {
+__device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll (&o1)[8], ll (&o2)[8], Guard& g) {
   ll cr[9], ci[9];
   R nV[9];
 #pragma unroll
@@ -465,7 +463,7 @@ __device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll tr_re, l
   o1[4] = ci[2] - ci[6];
   o1[5] = cr[7] + cr[5];
   o1[6] = ci[5] - ci[7];
-  o1[7] = 3 * (cr[0] + cr[4]) - 2 * tr_re;
+  o1[7] = 3 * (cr[0] + cr[4]);
   o2[0] = ci[3] + ci[1];
   o2[1] = cr[3] - cr[1];
   o2[2] = ci[0] - ci[4];
@@ -473,7 +471,7 @@ __device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll tr_re, l
   o2[4] = cr[6] - cr[2];
   o2[5] = ci[7] + ci[5];
   o2[6] = cr[7] - cr[5];
-  o2[7] = 3 * (ci[0] + ci[4]) - 2 * tr_im;
+  o2[7] = 3 * (ci[0] + ci[4]);
 }
 
 // C = V^dagger H V for Hermitian H, as alg_from_herm reads it (the last component without its 1/sqrt(3), all doubled as
@@ -558,8 +556,7 @@ __device__ __forceinline__ void herm_one(const Alg<T>& p, M& m, int& e, Guard& g
 }
 
 // M = 2 (t.p + i t.q) from two FP64 algebra vectors, exponent two above their largest component's.
-__device__ __forceinline__ void herm_pair(const Alg<double>& p, const Alg<double>& q, M& m, int& e, ll& tr_re, ll& tr_im,
-                                          Guard& g) {
+__device__ __forceinline__ void herm_pair(const Alg<double>& p, const Alg<double>& q, M& m, int& e, Guard& g) {
   int top = 0;
 #pragma unroll
   for (int k = 0; k < 8; k++) top = max(top, max(habs(p.a[k]), habs(q.a[k])));
@@ -586,7 +583,6 @@ __device__ __forceinline__ void herm_pair(const Alg<double>& p, const Alg<double
   m.e[4].im = split(s2 - c2);
   m.e[8].re = split(-2 * s1);
   m.e[8].im = split(-2 * s2);
-  tr_re = tr_im = 0;
 }
 
 // +-2^k o, the last component over sqrt 3; kFp64: by the FP64 pipe
@@ -605,9 +601,9 @@ __device__ __forceinline__ void adj_pair(const M& V, const Alg<double>& e1, cons
                                          Alg<double>& out2, Guard& g) {
   M m;
   int e;
-  ll tr_re, tr_im, o1[8], o2[8];
-  herm_pair(e1, e2, m, e, tr_re, tr_im, g);
-  rotate_pair<kInv>(V, m, tr_re, tr_im, o1, o2, g);
+  ll o1[8], o2[8];
+  herm_pair(e1, e2, m, e, g);
+  rotate_pair<kInv>(V, m, o1, o2, g);
   to_alg(o1, e - kScale - 1, 1.0, out1);
   to_alg(o2, e - kScale - 1, 1.0, out2);
 }
@@ -725,7 +721,10 @@ __device__ __forceinline__ bool near_exp(double c, const Alg<double>& al, M& X, 
   }
   const ll d0 = times(b[0], b[0]) + mod[0] + mod[1], d1 = times(b[1], b[1]) + mod[0] + mod[2],
            d2 = times(b[2], b[2]) + mod[1] + mod[2];
-  const double c1 = from_fixed(d0 + d1 + d2, 2 * em - kScale - 3), c0 = from_fixed(det, 3 * em - kScale - 3);
+  // below 2^-100 both are lost next to one (and the exponent of det would leave the doubles' range)
+  const bool weak = em < -100;
+  const double c1 = weak ? 0.0 : from_fixed(d0 + d1 + d2, 2 * em - kScale - 3);
+  const double c0 = weak ? 0.0 : from_fixed(det, 3 * em - kScale - 3);
   double f[6];
   if (c1 < 0.02) {
     const double z = c0 * c0;

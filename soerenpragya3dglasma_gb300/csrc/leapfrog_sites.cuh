@@ -608,20 +608,20 @@ __device__ __forceinline__ void plaquette_site_fx(const Geometry& g, const Field
   auto rotation = [&](int n) {
     fx::M v, m;
     int e;
-    ll tr_re, tr_im, o1[8], o2[8];
+    ll o1[8], o2[8];
     fx::link_plain(f.U, S, n == 3 ? 2 : 2 - n, n == 3 ? s - plane : s, v, guard);
     if (n < 3) {
       fx::Anti a1, a2;
       get(n == 0 ? 1 : 0, a1);
       get(n == 2 ? 1 : 2, a2);
-      fx::herm_pair(a1, a2, m, e, tr_re, tr_im);
+      fx::herm_pair(a1, a2, m, e);
     } else {
       Alg<double> jp, jm;
       load_alg(f.Jp, S, 0, s - plane, jp);
       load_alg(f.Jm, S, 0, s - plane, jm);
-      fx::herm_pair(jp, jm, m, e, tr_re, tr_im, guard);
+      fx::herm_pair(jp, jm, m, e, guard);
     }
-    fx::rotate_pair<true>(v, m, tr_re, tr_im, o1, o2, guard);
+    fx::rotate_pair<true>(v, m, o1, o2, guard);
     if (n < 3) {
       const int k1 = n == 0 ? kC02q : (n == 1 ? kC01q : kC01p), k2 = n == 0 ? kC12q : (n == 1 ? kC12p : kC02p);
       Alg<double> out, out2;
