@@ -126,6 +126,37 @@ __device__ __forceinline__ bool fixed_series(const Alg<R>& q, const Alg<R>& l, i
   if constexpr (sizeof(R) == 8) return fx::exp_series(q, l, terms, inv, o);
   return false;
 }
+template <typename R>
+__device__ __forceinline__ bool fixed_cross(const Alg<R>& a, const Alg<R>& b, Alg<R>& o) {
+  if constexpr (sizeof(R) == 8) return fx::cross(a, b, o);
+  return false;
+}
+template <typename R>
+__device__ __forceinline__ bool fixed_trace_with(const Mat<R>& h, const Alg<R>& n, Alg<R>& o) {
+  if constexpr (sizeof(R) == 8) return fx::trace_with(h, n, o);
+  return false;
+}
+// X = exp(i c t.e) and out = X^d u
+template <typename R>
+__device__ __forceinline__ bool fixed_step_back(R c, const Alg<R>& e, const Mat<R>& u, Mat<R>& x, Mat<R>& out) {
+  if constexpr (sizeof(R) == 8) {
+    fx::M X, D;
+    int ex;
+    if (!fx::near_exp(c, e, X, ex)) return false;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const fx::C& t = X.e[i + 3 * j];
+        x.e[i + 3 * j] = mk<double>((i == j ? 1.0 : 0.0) + fx::from_fixed(fx::join(t.re), ex - fx::kScale),
+                                    fx::from_fixed(fx::join(t.im), ex - fx::kScale));
+        D.e[j + 3 * i].re = t.re;
+        D.e[j + 3 * i].im = fx::neg(t.im);
+      }
+    return fx::add_product(D, ex, u, out);
+  }
+  return false;
+}
 
 namespace adj64 {
 #define ADJ_REAL double

@@ -847,68 +847,164 @@ __device__ __forceinline__ void plaquette_full(const M& W, int ew, const M& V, i
   }
 }
 
-// sum_n (q x)^n l / (n + 1)! in fixed point (x the structure-constant product), n up to `terms`; inv[n] = 1 / n.  |q| below one
-// in every component.  With the eighth components times sqrt 3 every structure constant but f^123 is 1/2.
+// The structure-constant product c = q x t (c^k = f^klm q_l t_m) of two vectors whose eighth components carry a factor
+// sqrt 3, as c's does: every constant but f^123 is 1/2 then.
+__device__ __forceinline__ void cross8(const R (&Q)[8], const R (&T)[8], ll (&c)[8]) {
+  R N[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) N[k] = neg(T[k]);
+  auto d = [&](Acc& a, int i, int j) {  // Q_i T_j - Q_j T_i
+    mad(a, Q[i - 1], T[j - 1]);
+    mad(a, Q[j - 1], N[i - 1]);
+  };
+  Acc a = acc_half(), b = acc_half();
+  d(a, 2, 3), d(b, 4, 7), d(b, 6, 5);
+  c[0] = finish(a) + (finish(b) >> 1);
+  a = b = acc_half();
+  d(a, 3, 1), d(b, 4, 6), d(b, 5, 7);
+  c[1] = finish(a) + (finish(b) >> 1);
+  a = b = acc_half();
+  d(a, 1, 2), d(b, 4, 5), d(b, 7, 6);
+  c[2] = finish(a) + (finish(b) >> 1);
+  a = acc_half();
+  d(a, 7, 1), d(a, 6, 2), d(a, 5, 3), d(a, 5, 8);
+  c[3] = finish(a) >> 1;
+  a = acc_half();
+  d(a, 1, 6), d(a, 7, 2), d(a, 3, 4), d(a, 8, 4);
+  c[4] = finish(a) >> 1;
+  a = acc_half();
+  d(a, 5, 1), d(a, 2, 4), d(a, 3, 7), d(a, 7, 8);
+  c[5] = finish(a) >> 1;
+  a = acc_half();
+  d(a, 1, 4), d(a, 2, 5), d(a, 6, 3), d(a, 8, 6);
+  c[6] = finish(a) >> 1;
+  a = acc_half();
+  d(a, 4, 5), d(a, 6, 7);
+  const ll r = finish(a);
+  c[7] = r + (r >> 1);
+}
+constexpr double kRoot3 = 1.7320508075688772935;
+// the larger |high word| of a vector's components, the eighth times sqrt 3
+__device__ __forceinline__ int top_of(const Alg<double>& v, double v8) {
+  int t = habs(v8);
+#pragma unroll
+  for (int k = 0; k < 7; k++) t = max(t, habs(v.a[k]));
+  return t;
+}
+// its components below 2^(60-e) |v| < 2^60
+__device__ __forceinline__ void to_fixed_alg(const Alg<double>& v, double v8, int e, R (&o)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) o[k] = to_fixed_split(k == 7 ? v8 : v.a[k], shift(kScale - e));
+}
+constexpr int kMaxHi = 0x43100000;  // 2^50
+
+// out = a x b; false where the format does not hold the operands
+__device__ __forceinline__ bool cross(const Alg<double>& a, const Alg<double>& b, Alg<double>& out) {
+  const double a8 = a.a[7] * kRoot3, b8 = b.a[7] * kRoot3;
+  const int ta = top_of(a, a8), tb = top_of(b, b8);
+  if (max(ta, tb) >= kMaxHi) return false;
+  const int ea = max(exponent_of(ta), kMinExp / 2), eb = max(exponent_of(tb), kMinExp / 2) + 1;
+  R A[8], B[8];
+  ll c[8];
+  to_fixed_alg(a, a8, ea, A);
+  to_fixed_alg(b, b8, eb, B);
+  cross8(A, B, c);
+#pragma unroll
+  for (int k = 0; k < 8; k++) out.a[k] = from_fixed(c[k], ea + eb - kScale) * (k == 7 ? kRoot3 / 3 : 1.0);
+  return true;
+}
+
+// out^k = Re tr(t^k H t.n) = 1/4 Re tr(t^k {H, 2 t.n}) for Hermitian H (h_ii, and h_ij for i < j)
+__device__ __forceinline__ bool trace_with(const Mat<double>& h, const Alg<double>& n, Alg<double>& out) {
+  const double n8 = n.a[7] * Consts<double>::inv_sqrt3();
+  int th = 0, tn = top_of(n, n8);
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i <= j; i++) th = max(th, max(habs(h.e[i + 3 * j].re), habs(h.e[i + 3 * j].im)));
+  if (max(th, tn) >= kMaxHi) return false;
+  // sums of two diagonal entries stay below 1, those of 2 t.n (up to 1.16 of the components) below 1 too
+  const int eh = max(exponent_of(th), kMinExp / 2) + 1, en = max(exponent_of(tn), kMinExp / 2) + 2;
+  const int sh = shift(kScale - eh), sn = shift(kScale - en);
+  ll hd[3], bd[3];
+  C ho[3], bo[3];  // 01, 02, 12
+  constexpr int at[3] = {3, 6, 7}, comp[3] = {0, 3, 5};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    hd[k] = to_fixed(h.e[4 * k].re, sh);
+    ho[k].re = to_fixed_split(h.e[at[k]].re, sh);
+    ho[k].im = to_fixed_split(h.e[at[k]].im, sh);
+    bo[k].re = to_fixed_split(n.a[comp[k]], sn);
+    bo[k].im = to_fixed_split(-n.a[comp[k] + 1], sn);
+  }
+  const ll b3 = to_fixed(n.a[2], sn), b8 = to_fixed(n8, sn);
+  bd[0] = b8 + b3;
+  bd[1] = b8 - b3;
+  bd[2] = -2 * b8;
+  // the diagonal: h_i b_i and r_n = Re(h_n conj(b_n))
+  ll hb[3], r[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    Acc a = acc_half(), b = acc_half();
+    mad(a, split(hd[k]), split(bd[k]));
+    mad(b, ho[k].re, bo[k].re);
+    mad(b, ho[k].im, bo[k].im);
+    hb[k] = finish(a);
+    r[k] = finish(b);
+  }
+  // off the diagonal: (h_i + h_j) b_n + (b_i + b_j) h_n + u v + w x, with the conjugates the indices ask for
+  ll re[3], im[3];
+  auto off = [&](int n_, int i, int j, const C& u, int su, const C& v, int sv, const C& w, int sw, const C& x, int sx) {
+    Acc a = acc_half(), b = acc_half();
+    const R hh = split(hd[i] + hd[j]), bb = split(bd[i] + bd[j]);
+    mad(a, hh, bo[n_].re);
+    mad(b, hh, bo[n_].im);
+    mad(a, bb, ho[n_].re);
+    mad(b, bb, ho[n_].im);
+    auto times = [&](const C& p, int sp, const C& q, int sq) {
+      const R pi = sp < 0 ? neg(p.im) : p.im, qi = sq < 0 ? neg(q.im) : q.im;
+      mad(a, p.re, q.re);
+      mad(a, neg(pi), qi);
+      mad(b, p.re, qi);
+      mad(b, pi, q.re);
+    };
+    times(u, su, v, sv);
+    times(w, sw, x, sx);
+    re[n_] = finish(a);
+    im[n_] = finish(b);
+  };
+  off(0, 0, 1, ho[1], 1, bo[2], -1, bo[1], 1, ho[2], -1);
+  off(1, 0, 2, ho[0], 1, bo[2], 1, bo[0], 1, ho[2], 1);
+  off(2, 1, 2, ho[0], -1, bo[1], 1, bo[0], -1, ho[1], 1);
+  const int k = eh + en - kScale;
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    out.a[comp[m]] = from_fixed(re[m], k - 2);
+    out.a[comp[m] + 1] = -from_fixed(im[m], k - 2);
+  }
+  out.a[2] = from_fixed((hb[0] - hb[1]) + (r[1] - r[2]), k - 2);
+  out.a[7] = from_fixed((hb[0] + hb[1] - 2 * hb[2]) + (2 * r[0] - r[1] - r[2]), k - 2) * Consts<double>::inv_sqrt3();
+  return true;
+}
+
+// sum_n (q x)^n l / (n + 1)! in fixed point, n up to `terms`; inv[n] = 1 / n.  |q| below one in every component.
 __device__ __forceinline__ bool exp_series(const Alg<double>& q, const Alg<double>& l, int terms, const double* inv,
                                            Alg<double>& out) {
-  const double r3 = 1.7320508075688772935;
-  int tq = 0, tl = 0;
-  Alg<double> qs = q, ls = l;
-  qs.a[7] *= r3;
-  ls.a[7] *= r3;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    tq = max(tq, habs(qs.a[k]));
-    tl = max(tl, habs(ls.a[k]));
-  }
-  if (tq >= 0x40000000 || tl >= 0x43100000) return false;  // 2; 2^50 or more, or not finite
+  const double q8 = q.a[7] * kRoot3, l8 = l.a[7] * kRoot3;
+  const int tq = top_of(q, q8), tl = top_of(l, l8);
+  if (tq >= 0x40000000 || tl >= kMaxHi) return false;  // 2
   const int eq = max(exponent_of(tq), kMinExp), el = max(exponent_of(tl), kMinExp) + 1;
   const int down = min(-min(eq, 0), 63), up = max(eq, 0);
   R Q[8], T[8];
   ll sum[8];
+  to_fixed_alg(q, q8, eq, Q);
+  to_fixed_alg(l, l8, el, T);
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    Q[k] = to_fixed_split(qs.a[k], shift(kScale - eq));
-    sum[k] = to_fixed(ls.a[k], shift(kScale - el));
-    T[k] = split(sum[k]);
-  }
+  for (int k = 0; k < 8; k++) sum[k] = join(T[k]);
 #pragma unroll 1
   for (int n = 1; n <= terms; n++) {
-    R N[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) N[k] = neg(T[k]);
-    auto d = [&](Acc& a, int i, int j) {  // Q_i T_j - Q_j T_i
-      mad(a, Q[i - 1], T[j - 1]);
-      mad(a, Q[j - 1], N[i - 1]);
-    };
     ll c[8];
-    {
-      Acc a = acc_half(), b = acc_half();
-      d(a, 2, 3), d(b, 4, 7), d(b, 6, 5);
-      c[0] = finish(a) + (finish(b) >> 1);
-      a = b = acc_half();
-      d(a, 3, 1), d(b, 4, 6), d(b, 5, 7);
-      c[1] = finish(a) + (finish(b) >> 1);
-      a = b = acc_half();
-      d(a, 1, 2), d(b, 4, 5), d(b, 7, 6);
-      c[2] = finish(a) + (finish(b) >> 1);
-      a = acc_half();
-      d(a, 7, 1), d(a, 6, 2), d(a, 5, 3), d(a, 5, 8);
-      c[3] = finish(a) >> 1;
-      a = acc_half();
-      d(a, 1, 6), d(a, 7, 2), d(a, 3, 4), d(a, 8, 4);
-      c[4] = finish(a) >> 1;
-      a = acc_half();
-      d(a, 5, 1), d(a, 2, 4), d(a, 3, 7), d(a, 7, 8);
-      c[5] = finish(a) >> 1;
-      a = acc_half();
-      d(a, 1, 4), d(a, 2, 5), d(a, 6, 3), d(a, 8, 6);
-      c[6] = finish(a) >> 1;
-      a = acc_half();
-      d(a, 4, 5), d(a, 6, 7);
-      const ll r = finish(a);
-      c[7] = r + (r >> 1);
-    }
+    cross8(Q, T, c);
     const R f = to_fixed_split(inv[n + 1], shift(kScale));
 #pragma unroll
     for (int k = 0; k < 8; k++) {
@@ -920,7 +1016,7 @@ __device__ __forceinline__ bool exp_series(const Alg<double>& q, const Alg<doubl
     }
   }
 #pragma unroll
-  for (int k = 0; k < 8; k++) out.a[k] = from_fixed(sum[k], el - kScale) * (k == 7 ? 1.0 / 3.0 * r3 : 1.0);
+  for (int k = 0; k < 8; k++) out.a[k] = from_fixed(sum[k], el - kScale) * (k == 7 ? kRoot3 / 3 : 1.0);
   return true;
 }
 
