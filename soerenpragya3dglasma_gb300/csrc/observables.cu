@@ -416,6 +416,74 @@ __global__ void __launch_bounds__(kFxThreads, kFxMinBlocks) gauss_kernel(Geometr
   block_reduce_store<2>(v, is_max, partials + ((long long)z * kZChunks + blockIdx.x) * 2);
 }
 
+// ||U U^d - 1||_F^2
+template <typename T>
+__device__ __forceinline__ double unitarity_direct(const cx<T>* U, long long S, int mu, long long s) {
+  Mat<double> u;
+  load_link_d(U, S, mu, s, u);
+  const double n = unitarity_norm(u);
+  return n * n;
+}
+template <typename T>
+__device__ __noinline__ double unitarity_far(const cx<T>* U, long long S, int mu, long long s) {
+  return unitarity_direct(U, S, mu, s);
+}
+// FP32 links: U U^d - 1 and the sum of its squares in fixed point (2^-58 beside deviations of ~1e-7), where FP64 kept the FP64
+// pipe busy with the 18 conversions and 54 products a link needs.  96x80x250: 1.50 ms in FP64, 0.26 here.  FP64 links deviate by
+// rounding only, and stay in FP64.
+__device__ __forceinline__ double unitarity_fx(const cx<float>* U, long long S, int mu, long long s) {
+  fx::Guard g = fx::guard_init();
+  fx::M m;
+  fx::link_plain(U, S, mu, s, m, g);
+  fx::R nI[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) nI[k] = fx::neg(m.e[k].im);
+  fx::ll d[9];  // the diagonal, then the real and imaginary parts above it
+  int n = 3;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = i; j < 3; j++) {
+      fx::Acc a = fx::acc_half(), b = fx::acc_half();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const fx::C &p = m.e[i + 3 * k], &q = m.e[j + 3 * k];
+        fx::mad(a, p.re, q.re);
+        fx::mad(a, p.im, q.im);
+        if (i != j) {
+          fx::mad(b, p.im, q.re);
+          fx::mad(b, p.re, nI[j + 3 * k]);
+        }
+      }
+      if (i == j) {
+        d[i] = fx::finish(a) - (1LL << fx::kScale);
+      } else {
+        d[n++] = fx::finish(a);
+        d[n++] = fx::finish(b);
+      }
+    }
+  unsigned long long any = 0;
+#pragma unroll
+  for (int k = 0; k < 9; k++) any |= (unsigned long long)(d[k] ^ (d[k] >> 63));
+  const int up = __clzll((long long)any) - 4;  // |d| 2^up < 2^60
+  fx::Acc diag = fx::acc_half(), off = fx::acc_half();
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const fx::ll t = up >= 0 ? d[k] << up : d[k] >> -up;
+    const fx::R r = fx::split((t ^ (t >> 63)) - (t >> 63));
+    fx::mad(k < 3 ? diag : off, r, r);
+  }
+  if (fx::tripped(g)) return unitarity_far(U, S, mu, s);
+  // six squares of off-diagonal numbers count twice
+  return fx::from_fixed(fx::finish(diag), -2 * up - fx::kScale) + fx::from_fixed(fx::finish(off), 1 - 2 * up - fx::kScale);
+}
+__device__ __forceinline__ double unitarity_of(const cx<float>* U, long long S, int mu, long long s) {
+  return unitarity_fx(U, S, mu, s);
+}
+__device__ __forceinline__ double unitarity_of(const cx<double>* U, long long S, int mu, long long s) {
+  return unitarity_direct(U, S, mu, s);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) unitarity_kernel(Geometry g, const cx<T>* U, double* partials) {
   double v[2] = {0.0, 0.0};
@@ -424,12 +492,11 @@ __global__ void __launch_bounds__(kRedThreads) unitarity_kernel(Geometry g, cons
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int mu = i < g.vol ? 0 : (i < 2 * g.vol ? 1 : 2);
     const long long s = i - (long long)mu * g.vol + g.plane;
-    Mat<double> u;
-    load_link_d(U, g.S, mu, s, u);
-    const double nrm = unitarity_norm(u);
-    v[0] += nrm * nrm;
-    v[1] = fmax(v[1], nrm);
+    const double n = unitarity_of(U, g.S, mu, s);
+    v[0] += n;
+    v[1] = fmax(v[1], n);
   }
+  v[1] = sqrt(v[1]);
   block_reduce_store<2>(v, is_max, partials + (long long)blockIdx.x * 2);
 }
 
@@ -520,21 +587,26 @@ __device__ __forceinline__ void clover_fx(const Geometry& g, const cx<T>* __rest
   defect = 0.0;
 #pragma unroll 1
   for (int l = 0; l < 4; l++) {
-    const bool swap = l == 1 || l == 2;            // the first link of W is U_nu
-    const int lm = (l & 1) ? -1 : 0, ln = l >= 2 ? -1 : 0;  // the leaf's lower corner: x + lm mu + ln nu
-    fx::M a, b, w, v;
-    int ea, eb, ew, ev;
-    // W: first link
-    fx::link_near(U, S, swap ? nu : mu, l == 0 || l == 1 ? at(0, 0) : (l == 2 ? at(0, -1) : at(-1, 0)), a, ea, guard,
-                  l >= 2);
-    fx::link_near(U, S, swap ? mu : nu, l == 0 ? at(1, 0) : (l == 1 ? at(-1, 1) : (l == 2 ? at(0, -1) : at(-1, -1))), b, eb,
-                  guard, l == 1 || l == 3);
-    fx::near_product(a, ea, b, eb, w, ew, guard);
-    fx::link_near(U, S, swap ? mu : nu, l == 0 || l == 2 ? at(0, 0) : (l == 1 ? at(-1, 0) : at(0, -1)), a, ea, guard,
-                  l == 1 || l == 3);
-    fx::link_near(U, S, swap ? nu : mu, l == 0 ? at(0, 1) : (l == 1 ? at(-1, 0) : (l == 2 ? at(1, -1) : at(lm, ln))), b, eb,
-                  guard, l >= 2);
-    fx::near_product(a, ea, b, eb, v, ev, guard);
+    // the leaf's lower corner c = x + lm mu + ln nu: its mu links are at c and c + nu, its nu links at c and c + mu
+    const int lm = (l & 1) ? -1 : 0, ln = l >= 2 ? -1 : 0;
+    const long long c = at(lm, ln), cm = at(lm + 1, ln), cn = at(lm, ln + 1);
+    fx::M w, v;
+    int ew, ev;
+    // W, then V, by one copy of the code (with two the kernel waits for instructions: 64x64x256 FP64 4.66 ms for 4.61)
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      const bool mu_up = ((l & 1) ^ h) != 0, nu_up = (l < 2) != (h != 0), swap = (l == 1 || l == 2) != (h != 0);
+      const long long s_mu = mu_up ? cn : c, s_nu = nu_up ? cm : c;
+      fx::M a, b;
+      int ea, eb;
+      if (h) {
+        w = v;
+        ew = ev;
+      }
+      fx::link_near(U, S, swap ? nu : mu, swap ? s_nu : s_mu, a, ea, guard, swap ? l >= 2 : (l & 1) != 0);
+      fx::link_near(U, S, swap ? mu : nu, swap ? s_mu : s_nu, b, eb, guard, swap ? (l & 1) != 0 : l >= 2);
+      fx::near_product(a, ea, b, eb, v, ev, guard);
+    }
     fx::Anti p;
     fx::plaquette_parts(w, ew, v, ev, p);
 #pragma unroll

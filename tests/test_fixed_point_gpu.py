@@ -137,6 +137,19 @@ def test_fp32_energy_and_unitarity_of_the_stored_fields(oracle, amp, e_amp, N):
     assert np.allclose(uni, oracle.unitarity(held, N), rtol=1e-3, atol=1e-15)
 
 
+# links as FP32 leaves them (deviations of 1e-7, 1e-16 / 1e-7 known in FP64), exact ones, and ones that fall back
+@pytest.mark.parametrize("amp,scale", [(0.3, 1.0), (0.0, 1.0), (0.3, 0.5), (0.3, 1.5)])
+@pytest.mark.parametrize("N", [(2, 2, 2), (9, 7, 33)])
+def test_fp32_unitarity(oracle, amp, scale, N):
+    f = O.random_fields(N, 79, link_amp=amp)
+    f["U"][::2] *= scale
+    with Lattice(N, A, precision="fp32") as lat:
+        lat.upload("U", f["U"])
+        got = lat.unitarity()
+        held = lat.download("U")
+    assert np.allclose(got, oracle.unitarity({"U": held}, N), rtol=1e-8, atol=0)
+
+
 LENGTHS = [2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 25, 27, 32, 45, 60, 64, 81, 96, 125, 128, 160, 240, 243, 256, 360, 486, 512, 625, 720,
            1024, 2048, 3000, 4096, 6561, 8192, 7, 14, 22, 49, 1001]
 
