@@ -27,7 +27,8 @@
 // (S/GAUGETRANSFORMATION/ALGORITHMS/LosAlamos.cpp, Jacobi.cpp) run through the same loop with a
 // local update in place of the FFT steps: local_update_kernel, one launch per checkerboard pass.
 //
-// All arithmetic is FP64 (G / UG / EG are stored in the handle's precision), except that with
+// All arithmetic is of FP64 accuracy (the matrix products of the Fourier sweeps in fixed point, fx.cuh; G / UG / EG are
+// stored in the handle's precision), except that with
 // GLASMA_GF_FFT_FP32 the two transforms of the acceleration step run in FP32: they only
 // precondition the step, so the iteration still converges to the same gauge, measured in FP64.
 //
@@ -35,10 +36,10 @@
 // X[q] = Delta^{2q} + i Delta^{2q+1}: four complex 3D transforms per direction instead of the
 // reference's eight (the real factor, even in p, keeps the two colours apart on the way back).
 // A 3D transform is three passes of batched 1D transforms along x, y and z over X[q][z][y][x].
-// A block stages a tile of lines in shared memory (consecutive lines for the x pass; for the y
-// and z passes a tile of consecutive x, so every global access is a contiguous run), transforms it
-// there and writes it back in place: radix-2 decimation in time for power-of-two lengths, a
-// mixed-radix Stockham transform (radices 4, 2, 3, 5, other primes directly) otherwise.  On GB300 the FP64 transform is bound by the FP64 pipe, not by HBM.
+// Lengths 2^a 3^b 5^c go through fft.cuh (register-blocked passes; the acceleration step along z, its factor and the
+// inverse along z in one of them).  The kernels here keep what that does not take: a block stages a tile of lines in shared
+// memory (consecutive lines for the x pass; for the y and z passes a tile of consecutive x, so every global access is a
+// contiguous run) and transforms it there, by radix 2 for powers of two, by mixed-radix Stockham passes otherwise.
 #include <map>
 #include <vector>
 

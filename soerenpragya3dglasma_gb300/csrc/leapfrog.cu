@@ -10,7 +10,10 @@
 //                                (finished by K1), so the whole tail of the step is pointwise;
 //                                exp(i cU E) is formed once per link and applied twice.
 //
-// The electric force uses the staple form
+// That is the two-pass method.  The default is the plaquette method (leapfrog_sites.cuh): the force one plaquette at a time,
+// its rotated terms handed to the link kernel through a buffer; FP64 does its matrix products in fixed point (fx.cuh).
+//
+// The electric force of K1 uses the staple form
 //   E_mu^a += gamma c_mu ReTr(i t^a U_mu(x) sum_nu c_nu [S_{+nu} + S_{-nu}]),
 //   S_{+nu} = U_nu(x+mu) U_mu^d(x+nu) U_nu^d(x),  S_{-nu} = U_nu^d(x+mu-nu) U_mu^d(x-nu) U_nu(x-nu),
 // which is the reference's nine-plaquette expression (S/CALC/Plaquettes.cpp:83-97 with

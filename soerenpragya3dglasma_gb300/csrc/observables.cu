@@ -11,8 +11,8 @@
 //
 // Every reduction is two-pass and deterministic: a fixed grid writes FP64 block partials
 // (warp shuffles, then shared memory), a one-block pass sums them in a fixed order.
-// Site arithmetic runs in FP64, except the magnetic term of the bulk energy on FP32 lattices,
-// which uses the identity
+// Site arithmetic runs in FP64 accuracy: the matrix products in fixed point on the integer pipe (fx.cuh), or in FP64, out of
+// line, where that does not hold the links.  The magnetic term of the bulk energy on FP32 lattices uses the identity
 //   3 - ReTr(a b c^d d^d) = 1/2 ||A - B||^2 - 1/2 (n(a) + n(b) + n(c) + n(d)),
 //   A = a b, B = d c, n(u) = ||u||_F^2 - 3  (zero for unitary u),
 // exact with n(A) + n(B) in place of the four link terms and equal to it to first order in the links'
