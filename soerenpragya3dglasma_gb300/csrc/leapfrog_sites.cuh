@@ -532,7 +532,7 @@ __device__ __forceinline__ void plaquette_site_direct(const Geometry& g, const F
 
 // plaquette_site for FP64 fields with the products on the integer pipe (fx.cuh).  Bound by FP64, the direct form
 // runs ~2000 FP64 operations per site; here they are ~5,000 mad.wide and ~15,000 other integer operations, with ~300
-// FP64 ones beside them (the sums into E, conversions): 128x128x512 30.7 ms in FP64, 10.6 here.  One copy of the plaquette and of the rotation in the code, so
+// FP64 ones beside them (the sums into E, conversions): 128x128x512 30.7 ms in FP64, 10.9 here.  One copy of the plaquette and of the rotation in the code, so
 // that it stays inside the instruction cache; the three anti-Hermitian parts wait in shared memory for their rotations.
 // kRoles = 1: a thread does its site's three plaquettes and four rotation pairs in turn.  kRoles = 4: a block of four
 // warps does 32 sites, warp r plaquette r, rotation r and the sum into E_r (warp 3 the currents' rotation and JStat):
@@ -888,7 +888,7 @@ __device__ __forceinline__ void link_site(const Geometry& g, const FieldPtrs<T>&
   if constexpr (std::is_same<T, double>::value) {
     // One copy of the product and of the current transport in the code, run once or twice per link: written out
     // (three products, two exponentials) the fixed-point body overflowed the instruction cache (5.6 fetch stalls
-    // per issue, 14.3 ms at 128x128x512; 11.0 like this, 21.9 in FP64).
+    // per issue, 14.3 ms at 128x128x512; 10.6 like this, 21.9 in FP64).
     const bool doubled = p.do_second && !p.save_uold && !(mu == 2 && p.do_j);
     LinkStep<double> X;
     X.set(doubled ? 2.0 * pick3(p.cU, mu) : pick3(p.cU, mu), e);
