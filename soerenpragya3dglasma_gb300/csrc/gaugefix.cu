@@ -471,17 +471,139 @@ __global__ void __launch_bounds__(kGfThreads) update32_kernel(Geometry g, const 
   red::block_reduce_store<3>(v, op, partials + (long long)blockIdx.x * 3);
 }
 
-// G = the SU(3) projection (FP64 Newton, reunitarize_newton) of the widened FP32 G, every site
-__global__ void widen_gauge_kernel(const cx<float>* __restrict__ G32, cx<double>* __restrict__ G, long long S) {
-  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S) return;
-  Mat<double> m;
+// G = the SU(3) projection of the widened FP32 G, every site: the unitary polar factor, then the determinant's phase divided out.
+__device__ __noinline__ void widen_newton(const cx<float>* G32, long long S, long long s, Mat<double>& m) {
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const cx<float> v = G32[(long long)k * S + s];
     m.e[k] = mk<double>((double)v.re, (double)v.im);
   }
   reunitarize_newton(m);
+}
+// The same in fixed point for matrices within 2^-17 of SU(3), as FP32 sweeps leave them.  With e = U^d U - 1 (Hermitian, to 2^-59)
+// the polar factor is U (1 + e)^(-1/2) = U (1 - e/2 + 3/8 e^2 - 5/16 e^3), the next term below 2^-68; det U = |det U| e^(i theta)
+// adds the factor 1 - i phi - phi^2/2, phi = theta/3.  Terms of second order and above are at most 2^-32, so FP32 holds them
+// to 2^-56.  Bound by FP64 in reunitarize_newton (two inverses and the phase's functions), 3.79 ms at
+// 128x128x256; here by issue, 3.4 ms less.
+__device__ __forceinline__ bool widen_fx(const cx<float>* __restrict__ G32, long long S, long long s, Mat<double>& out) {
+  fx::Guard g = fx::guard_init();
+  fx::M u;
+  fx::link_plain(G32, S, 0, s, u, g);
+  fx::R nI[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) nI[k] = fx::neg(u.e[k].im);
+  constexpr float unit = 1.f / (1LL << fx::kScale);
+  fx::ll er[9], ei[9];
+  int top = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = i; j < 3; j++) {  // e_ij = sum_k conj(u_ki) u_kj
+      fx::Acc a = fx::acc_half(), b = fx::acc_half();
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const fx::C &p = u.e[k + 3 * i], &q = u.e[k + 3 * j];
+        fx::mad(a, p.re, q.re);
+        fx::mad(a, p.im, q.im);
+        if (i != j) {
+          fx::mad(b, p.re, q.im);
+          fx::mad(b, nI[k + 3 * i], q.re);
+        }
+      }
+      const fx::ll re = fx::finish(a) - (i == j ? 1LL << fx::kScale : 0), im = i == j ? 0 : fx::finish(b);
+      er[i + 3 * j] = er[j + 3 * i] = re;
+      ei[i + 3 * j] = im;
+      ei[j + 3 * i] = -im;
+      top = max(top, max(abs((int)(re >> 32)), abs((int)(im >> 32))));
+    }
+  // det U by the first row's cofactors; theta = atan(Im / Re) with Re = 1 + r
+  fx::ll dr = 0, di = 0;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+    fx::Acc a = fx::acc_half(), b = fx::acc_half();
+    auto times = [&](const fx::C& p, const fx::C& q, const fx::R& nq, bool minus) {  // p q or -p q
+      fx::C t = p;
+      if (minus) {
+        t.re = fx::neg(p.re);
+        t.im = fx::neg(p.im);
+      }
+      fx::mad(a, t.re, q.re);
+      fx::mad(a, t.im, nq);
+      fx::mad(b, t.re, q.im);
+      fx::mad(b, t.im, q.re);
+    };
+    times(u.e[1 + 3 * j1], u.e[2 + 3 * j2], nI[2 + 3 * j2], false);
+    times(u.e[1 + 3 * j2], u.e[2 + 3 * j1], nI[2 + 3 * j1], true);
+    const fx::R cr = fx::split(fx::finish(a)), ci = fx::split(fx::finish(b));
+    a = b = fx::acc_half();
+    fx::mad(a, cr, u.e[3 * j].re);
+    fx::mad(a, ci, nI[3 * j]);
+    fx::mad(b, cr, u.e[3 * j].im);
+    fx::mad(b, ci, u.e[3 * j].re);
+    dr += fx::finish(a);
+    di += fx::finish(b);
+  }
+  const fx::ll r = dr - (1LL << fx::kScale);
+  top = max(top, max(abs((int)(r >> 32)), abs((int)(di >> 32))));
+  if (g.bad || top >= 1 << (28 - 17)) return false;
+  const float rf = (float)r * unit, df = (float)di * unit;
+  // theta = d - d r + d r^2 - d^3 / 3, phi = theta / 3
+  const float t2 = df * (rf * (rf - 1.f) - df * df * (1.f / 3.f));
+  const fx::ll theta = di + (fx::ll)(t2 * (float)(1LL << fx::kScale));
+  const fx::ll phi = __mul64hi(theta, 0x5555555555555556LL);
+  const float pf = (float)phi * unit;
+  // c = -e/2 + F, F = 3/8 e^2 - 5/16 e^3 - i phi c - phi^2/2, and -i phi on the diagonal
+  cx<float> e[9], e2[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) e[k] = mk<float>((float)er[k] * unit, (float)ei[k] * unit);
+  auto entry = [&](const cx<float>(&a)[9], const cx<float>(&b)[9], int i, int j) {
+    cx<float> t = mk<float>(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 3; k++) cfma(t, a[i + 3 * k], b[k + 3 * j]);
+    return t;
+  };
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) e2[i + 3 * j] = entry(e, e, i, j);
+  fx::M c;  // exponent -16
+  constexpr float to = (float)(1LL << fx::kScale);
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const int k = i + 3 * j;
+      const cx<float> e3 = entry(e2, e, i, j);
+      const cx<float> h = mk<float>(0.375f * e2[k].re - 0.3125f * e3.re, 0.375f * e2[k].im - 0.3125f * e3.im);
+      const cx<float> all = mk<float>(h.re - 0.5f * e[k].re, h.im - 0.5f * e[k].im);
+      const float fr = h.re + pf * all.im - (i == j ? 0.5f * pf * pf : 0.f), fi = h.im - pf * all.re;
+      c.e[k].re = fx::split(((fx::ll)(fr * to) - (er[k] >> 1)) << 16);
+      c.e[k].im = fx::split(((fx::ll)(fi * to) - (ei[k] >> 1) - (i == j ? phi : 0)) << 16);
+    }
+  fx::R nC[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) nC[k] = fx::neg(c.e[k].im);
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      fx::Acc re, im;
+      fx::entry_nn(u, i, c, nC, j, re, im);
+      out.e[i + 3 * j] = mk<double>(fx::from_fixed(fx::join(u.e[i + 3 * j].re) + (fx::finish(re) >> 16), -fx::kScale),
+                                    fx::from_fixed(fx::join(u.e[i + 3 * j].im) + (fx::finish(im) >> 16), -fx::kScale));
+    }
+  return true;
+}
+__global__ void __launch_bounds__(128) widen_gauge_kernel(const cx<float>* __restrict__ G32, cx<double>* __restrict__ G, long long S) {
+  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= S) return;
+  Mat<double> m;
+  if (!widen_fx(G32, S, s, m)) {
+    Mat<double> t;
+    widen_newton(G32, S, s, t);
+    m = t;
+  }
 #pragma unroll
   for (int k = 0; k < 9; k++) G[(long long)k * S + s] = m.e[k];
 }
@@ -1408,7 +1530,7 @@ int run_mixed(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_ite
     if (gmax <= kMixedSwitch) break;
   }
   // hand over: G from the FP32 sweeps, widened and projected, then the FP64 sweeps
-  widen_gauge_kernel<<<(unsigned)((g.S + 255) / 256), 256, 0, st>>>(c.G, static_cast<cx<double>*>(a.G), g.S);
+  widen_gauge_kernel<<<(unsigned)((g.S + 127) / 128), 128, 0, st>>>(c.G, static_cast<cx<double>*>(a.G), g.S);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "widen gauge");
   *iterations = n;
   if (gmax <= tol && n > 0) {

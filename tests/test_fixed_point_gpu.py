@@ -193,6 +193,23 @@ def test_gauge_sweeps_on_ragged_lattices(oracle, N, project):
         assert np.max(np.abs(lat.download("EG") - EG)) < 1e-11
 
 
+# G leaves the FP32 sweeps by the expansion about SU(3), or, further than 2^-17 from it, by Newton's iteration.  Both are
+# exact to rounding (1e-4 squared twice); the products of an entry and of the determinant, and the few FP64 sweeps that may
+# follow, add some ten roundings each: 1e-14.
+@pytest.mark.parametrize("scale", [1.0, 1 + 1e-4])
+@pytest.mark.parametrize("N,iters", [((3, 2, 4), 2), ((9, 7, 11), 40)])
+def test_mixed_sweeps_leave_su3(scale, N, iters):
+    f = O.random_fields(N, 80, link_amp=0.2)
+    with Lattice(N) as lat:
+        lat.upload("U", f["U"])
+        lat.upload("E", f["E"])
+        lat.upload("G", scale * O.identity_gauge(N))
+        lat.coulomb_fix(0.08, iters, open_z=True, mixed=True)
+        G = O.links_as_matrices(lat.download("G"))[1:-1]
+    assert np.max(np.abs(G @ np.swapaxes(G.conj(), -1, -2) - np.eye(3))) < 1e-14
+    assert np.max(np.abs(np.linalg.det(G) - 1)) < 1e-14
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("N", [(2, 2, 2), (5, 3, 7), (33, 4, 3)])
 def test_device_buffers_give_the_same_bytes(precision, N):
