@@ -369,9 +369,9 @@ def run_ours(args):
         ach = alg / (ms * 1e-3) / 1e9
         key = "%s_%s" % (name, prec)
         tr = traffic.get(key)
-        # what limits the kernel, from the ncu capture of the same kernel: the FP64 kernels keep GB300's
-        # FP64 pipe >90 % busy (hence their small HBM fraction), the FP32 ones are bound by HBM traffic
-        # and issue
+        # what limits the kernel, from the ncu capture of the same kernel: the FP64 staple kernels keep
+        # GB300's FP64 pipe >90 % busy (hence their small HBM fraction), the fixed-point ones are bound by
+        # latency and the integer multiplier, the FP32 ones by HBM traffic and issue
         pa = traffic.get("pipe_active", {}).get(key)
         bound = "fp64_pipe" if pa and pa.get("pipe") == "fp64" and pa.get("frac", 0) > 0.8 else "hbm"
         out = {"bound": bound, "kernel": name, "achieved": ach, "peak": peak, "unit": "GB/s",

@@ -169,11 +169,12 @@ int glasma_set_march_chunk(glasma_lattice* h, int slices);
  * end of every glasma_step call row 2 is written back, so every other call sees full links.  Rows 0
  * and 1 are taken as the link: a link that is not in SU(3) when the call starts is replaced by the
  * SU(3)-completion of its first two rows.  GLASMA_ERR_UNSUPPORTED for 12 on FP64 handles (their
- * kernels are bound by the FP64 pipe, which the reconstruction would load further).
+ * kernels are bound by arithmetic, which the reconstruction would add to).
  * No reference counterpart (the reference stores full links, S/LATTICE/GaugeLinks.cpp). */
 int glasma_set_link_storage(glasma_lattice* h, int reals_per_link);
 
-/* Arithmetic of the plaquette method's force kernel on FP64 handles: GLASMA_FP64_NATIVE (default) or
+/* Arithmetic of the plaquette method's force kernel on FP64 handles: GLASMA_FP64_NATIVE (default;
+ * FP64 accuracy, the matrix products in 60-bit fixed point on the integer pipe) or
  * GLASMA_FP64_DOUBLE_FLOAT, double-float arithmetic on the FP32 pipe (each value an unevaluated sum of
  * two floats, ~48-bit significand; the FP64 fields are converted on load and store).  GB300 runs FP64
  * at 1/64 of its FP32 rate.  Ignored by FP32 handles and the other step methods. */

@@ -178,8 +178,8 @@ void prefer_l1(K kernel) {
   }
 }
 
-// Two-row (12-real) link storage is built for FP32 only: the FP64 kernels are bound by the FP64 pipe,
-// and the row reconstruction would add FP64 work to save bytes that do not bound them.
+// Two-row (12-real) link storage is built for FP32 only: the FP64 kernels are bound by arithmetic,
+// and the row reconstruction would add to it to save bytes that do not bound them.
 template <typename T>
 bool two_row(int link_rows) {
   return sizeof(T) == 4 && link_rows == 2;
