@@ -484,7 +484,7 @@ __device__ __noinline__ void widen_newton(const cx<float>* G32, long long S, lon
 // the polar factor is U (1 + e)^(-1/2) = U (1 - e/2 + 3/8 e^2 - 5/16 e^3), the next term below 2^-68; det U = |det U| e^(i theta)
 // adds the factor 1 - i phi - phi^2/2, phi = theta/3.  Terms of second order and above are at most 2^-32, so FP32 holds them
 // to 2^-56.  Bound by FP64 in reunitarize_newton (two inverses and the phase's functions), 3.79 ms at
-// 128x128x256; here by issue, 3.4 ms less.
+// 128x128x256; here by issue, 0.58 ms.
 __device__ __forceinline__ bool widen_fx(const cx<float>* __restrict__ G32, long long S, long long s, Mat<double>& out) {
   fx::Guard g = fx::guard_init();
   fx::M u;
