@@ -116,9 +116,14 @@ __device__ __forceinline__ ll magnitude(double v, int sh) {
       ((unsigned long long)((h & 0xfffff) | 0x100000) << 40) | ((unsigned long long)(unsigned)__double2loint(v) << 8);
   return shifted(m, sh - ((h >> 20) & 0x7ff));
 }
+// A float times 2^76, exactly: subnormal numbers become normal ones, and a zero, taken for the smallest of those, falls below
+// 2^-203, under the last place of every k up to 199 (kMinExpOf<float>).  (A double's smallest exponents are out of reach of
+// every k in use.)  One multiplication of the FP32 pipe, which these kernels leave idle.
+constexpr int kLift = 76;
+__device__ __forceinline__ int lifted(float v) { return __float_as_int(v * 0x1p76f); }
 __device__ __forceinline__ ll magnitude(float v, int sh) {
-  const int h = __float_as_int(v);
-  return shifted((unsigned long long)((h & 0x7fffff) | 0x800000) << 37, sh - 896 - ((h >> 23) & 0xff));
+  const int h = lifted(v);
+  return shifted((unsigned long long)((h & 0x7fffff) | 0x800000) << 37, sh - (896 - kLift) - ((h >> 23) & 0xff));
 }
 __device__ __forceinline__ int sign_word(double v) { return __double2hiint(v) >> 31; }
 __device__ __forceinline__ int sign_word(float v) { return __float_as_int(v) >> 31; }
@@ -152,14 +157,17 @@ __device__ __forceinline__ double from_fixed_fp64(ll q, int k) {
   const double v = (hi - 19342822341709703277445120.0) + lo;  // 2^84 + 2^63 + 2^52
   return q == 0 ? 0.0 : __hiloint2double(__double2hiint(v) + (int)((unsigned)k << 20), __double2loint(v));
 }
-constexpr int kMinExp = -900;  // smaller values are held at 2^-960
+// Exponents from here on: smaller values are held at 2^(kMinExp - 60).
+template <typename T>
+constexpr int kMinExpOf = sizeof(T) == 8 ? -900 : -139;
+constexpr int kMinExp = kMinExpOf<double>;
 // |v| < 2^exponent_of(largest |high word| of v)
 __device__ __forceinline__ int exponent_of(int habs) { return (habs >> 20) - 1022; }
 constexpr int kMaxEntryHi = 0x3FF07AE1;  // 1.03
 
 // the high word of |v| as a double
 __device__ __forceinline__ int habs(double v) { return __double2hiint(v) & 0x7fffffff; }
-__device__ __forceinline__ int habs(float v) { return ((__float_as_int(v) & 0x7fffffff) >> 3) + (896 << 20); }
+__device__ __forceinline__ int habs(float v) { return ((lifted(v) & 0x7fffffff) >> 3) + ((896 - kLift) << 20); }
 
 // A plain matrix with entries up to one (a link), exponent 0; kDag: its dagger.
 template <bool kDag = false, typename T, typename I>
@@ -205,8 +213,9 @@ __device__ __forceinline__ void link_near(const cx<T>* __restrict__ U, I S, int 
     }
   }
   g.bad |= max(top, topd) > kMaxEntryHi;
-  const int ed = dor == 0 ? kMinExp : 64 - __clzll(dor) - kScale;  // |diagonal - 1| < 2^ed
-  int ee = max(max(exponent_of(top), ed), kMinExp);
+  constexpr int least = kMinExpOf<T>;
+  const int ed = dor == 0 ? least : 64 - __clzll(dor) - kScale;  // |diagonal - 1| < 2^ed
+  int ee = max(max(exponent_of(top), ed), least);
   ee = min(ee, 0);
   e = ee;
   const int kb = shift(kScale - ee);
@@ -537,7 +546,7 @@ __device__ __forceinline__ void herm_one(const Alg<T>& p, M& m, int& e, Guard& g
 #pragma unroll
   for (int k = 0; k < 8; k++) top = max(top, habs(p.a[k]));
   g.bad |= top >= 0x43100000;  // 2^50 or more, or not finite
-  const int em = max(exponent_of(min(top, 0x43100000)), kMinExp) + 2;
+  const int em = max(exponent_of(min(top, 0x43100000)), kMinExpOf<T>) + 2;
   e = em;
   const int sh = shift(kScale - em);
   // a_8 / sqrt 3 in FP64: exact in the format to 2^-60 whatever T is

@@ -1,0 +1,75 @@
+"""The limits of the fixed-point kernels (csrc/fx.cuh): numbers that the format holds differently or not at all, which have
+to come out as FP64 gives them.
+
+Tolerances.  The kernels and the oracle each make some tens of FP64 roundings of 1.1e-16 per site: 1e-12 of the largest
+number of a slice, the bar of the other parity tests.  What is stored in FP32 adds its own rounding, 6e-8."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from soerenpragya3dglasma_gb300 import Lattice, build
+
+pytestmark = pytest.mark.gpu
+
+A = (1.0, 1.1, 0.9)
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    build.build()
+
+
+def _rotated(V, e):
+    """2 tr(t^a V (t.e) V^dagger)."""
+    return O.algebra_from_herm(V @ O.herm_from_algebra(e) @ np.swapaxes(V.conj(), -1, -2))
+
+
+def _random_gauge(N, seed):
+    """A random SU(3) matrix per site in the layout of G, [.., j, i], ghost slices synced."""
+    G = O.random_fields(N, seed, link_amp=0.8)["U"][..., 0, :, :].copy()
+    O.sync_ghosts(G)
+    return G
+
+
+# ---- FP32 lattices: zeros and subnormal numbers
+@pytest.mark.parametrize("links", ["identity", "random"])
+def test_fp32_zero_fields_measure_exactly_zero(links):
+    N = (5, 4, 6)
+    with Lattice(N, A, precision="fp32") as lat:
+        if links == "random":
+            lat.upload("U", O.random_fields(N, 90, link_amp=0.3)["U"])
+            lat.upload("G", _random_gauge(N, 91))
+        lat.upload("E", O.zero_efield(N))
+        worst, mean, profile = lat.gauss(profile=True)
+        assert worst == 0 and mean == 0 and not profile.any()
+        assert not lat.emt_map().any()  # UOld is the identity
+        lat.coulomb_fix(0.08, 0)
+        assert not lat.download("EG").any()
+
+
+@pytest.mark.parametrize("size", [1e-22, 1e-33, 1e-36, 1e-40, 1e-43])
+def test_fp32_dilute_slices(oracle, size):
+    """Slices of E at `size`, half of their components zero, beside slices of order one."""
+    N = (5, 4, 12)
+    f = O.random_fields(N, 92, link_amp=0.3, e_amp=0.1, j_amp=0.0)
+    f["UOld"] = O.identity_links(N)
+    f["E"][6:] *= 10 * size
+    f["E"][6:][np.random.default_rng(1).random(f["E"][6:].shape) < 0.5] = 0.0
+    O.sync_ghosts(f["E"])
+    G = _random_gauge(N, 93)
+    with Lattice(N, A, precision="fp32") as lat:
+        lat.upload_fields(f)
+        held = lat.download_fields()
+        profile, emt = lat.gauss(profile=True)[2], lat.emt_map()
+        lat.upload("G", G)
+        g = O.links_as_matrices(lat.download("G"))
+        lat.coulomb_fix(0.08, 0)
+        EG = lat.download("EG")
+    want_p, want_t = oracle.gauss(held, N, A, profile=True)[2], oracle.emt_map(held, N, A)
+    want_e = _rotated(g[..., None, :, :], held["E"])
+    for z in range(N[2]):
+        assert abs(profile[z] - want_p[z]) <= 1e-12 * want_p[z], z
+        assert np.max(np.abs(emt[z] - want_t[z])) <= 1e-12 * want_t[z, 0], z
+        # stored in FP32: half an ulp of the largest component, or of the subnormal numbers (1.4e-45)
+        d, top = np.abs(EG[z + 1] - want_e[z + 1]), np.max(np.abs(want_e[z + 1]))
+        assert np.max(d) <= 6e-8 * top + 0.8e-45, z
