@@ -207,9 +207,9 @@ __device__ __forceinline__ double link_norm_dev(const cx<float>* __restrict__ U,
     fx::mad(a, re, re);
     fx::mad(a, im, im);
   }
-  // entries up to 1.03 only: eighteen squares up to 19 would leave the format's +-8 (they wrap in the 64-bit sum, which is
-  // exact again after the subtraction for every matrix whose norm^2 is below 11)
-  if (top > fx::kMaxEntryHi) return link_norm_dev_fp64(U, S, mu, s);
+  // Eighteen squares may add up to 19, beyond the format's +-8.  finish's 64-bit sum wraps there and is exact again after the
+  // subtraction for norm^2 below 11; a.hh itself, 2^56 per unit, does not wrap.
+  if (top > fx::kMaxEntryHi || (int)(a.hh >> 32) >= 10 << 24) return link_norm_dev_fp64(U, S, mu, s);
   return fx::from_fixed(fx::finish(a) - 3 * (1LL << fx::kScale), -fx::kScale);
 }
 // sum of squares of eight FP32 components, to 2^-58 of it

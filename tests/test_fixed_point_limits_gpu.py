@@ -73,3 +73,17 @@ def test_fp32_dilute_slices(oracle, size):
         # stored in FP32: half an ulp of the largest component, or of the subnormal numbers (1.4e-45)
         d, top = np.abs(EG[z + 1] - want_e[z + 1]), np.max(np.abs(want_e[z + 1]))
         assert np.max(d) <= 6e-8 * top + 0.8e-45, z
+
+
+# ---- links far from SU(3): what the fixed-point sums cannot hold goes through FP64
+@pytest.mark.parametrize("u", [0.6, 0.74, 0.78, 0.9, 1.02, 1.2])
+@pytest.mark.parametrize("N", [(2, 2, 2), (9, 7, 33)])
+def test_fp32_norms_of_links_off_the_group(N, u):
+    """The same matrix on every link, all entries u + iu: the products of a plaquette's halves are equal, and the FP32 bulk
+    energy is -2 (n(a) + n(b) + n(c) + n(d)) per plaquette, n = ||link||^2 - 3."""
+    U = np.full((N[2] + 2, N[1], N[0], 3, 3, 3), u + 1j * u)
+    with Lattice(N, A, precision="fp32") as lat:
+        lat.upload("U", U)
+        magnetic = lat.bulk()[3:6]
+    n = 18 * float(np.float32(u)) ** 2 - 3
+    assert np.allclose(magnetic, -8 * n * N[0] * N[1] * N[2], rtol=1e-12, atol=0)
