@@ -18,8 +18,8 @@
 // where FP64's is to ~2^-53 of it.
 //
 // What the format cannot hold is found, not assumed away: a link entry above 1.03 (or not finite), a row of a
-// product of two links whose norm is not near one, and an accumulator out of range set Guard, and the caller
-// runs the FP64 arithmetic for that site instead.
+// product of two links whose norm is not near one, an accumulator or a sum of two or three out of range set Guard, and the
+// caller runs the FP64 arithmetic for that site instead.
 #pragma once
 
 #include "su3.cuh"
@@ -421,6 +421,17 @@ __device__ __forceinline__ void herm_pair(const Anti& p, const Anti& q, M& m, in
   m.e[8].im = split(-b0 - b1);
 }
 
+// Sums of watched numbers (below 4 each) that may pass the format's 8, from their high words (2^28 is one): 3 (a + b), and
+// a + b - 2 c.  Links of SU(3) stay far below; a matrix with large entries that is not unitary need not.
+__device__ __forceinline__ void watch_sum(Guard& g, ll a, ll b) {
+  constexpr unsigned most = 5u << 27;  // 2.5
+  g.bad |= (unsigned)((int)(a >> 32) + (int)(b >> 32)) + most > 2 * most;
+}
+__device__ __forceinline__ void watch_eighth(Guard& g, ll a, ll b, ll c) {
+  constexpr int most = 15 << 25;  // 7.5 / 4
+  g.bad |= abs((int)(a >> 34) + (int)(b >> 34) - (int)(c >> 33)) > most;
+}
+
 // The Hermitian and anti-Hermitian parts of C = V^dagger M V (kInv) or V M V^dagger, as split_herm_pair gives them
 // (the last of each without its 1/sqrt(3)); V plain, in units of M.  M is traceless, and C_22 follows from that.
 template <bool kInv>
@@ -465,6 +476,8 @@ __device__ __forceinline__ void rotate_pair(const M& V, const M& Mm, ll (&o1)[8]
       ci[i + 3 * j] = finish(im);
     }
   }
+  watch_sum(g, cr[0], cr[4]);
+  watch_sum(g, ci[0], ci[4]);
   o1[0] = cr[3] + cr[1];
   o1[1] = ci[1] - ci[3];
   o1[2] = cr[0] - cr[4];
@@ -530,6 +543,7 @@ __device__ __forceinline__ void rotate_one(const M& V, const M& H, ll (&o)[8], G
       ci[i + 3 * j] = finish(im);
     }
   }
+  watch_eighth(g, cr[0], cr[4], cr[8]);
   o[0] = 2 * cr[3];
   o[1] = -2 * ci[3];
   o[2] = cr[0] - cr[4];

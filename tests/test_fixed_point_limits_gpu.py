@@ -87,3 +87,62 @@ def test_fp32_norms_of_links_off_the_group(N, u):
         magnetic = lat.bulk()[3:6]
     n = 18 * float(np.float32(u)) ** 2 - 3
     assert np.allclose(magnetic, -8 * n * N[0] * N[1] * N[2], rtol=1e-12, atol=0)
+
+
+# A matrix that is far from unitary although every entry is below 1.03, and an algebra vector whose rotation by it adds up to
+# more than the format's 8 in the eighth component: the columns (or rows) of V lie along eigenvectors of t.e.
+ALONG = 0.99 * np.array([-1.0, 0, 0, -1, 0, -1, 0, 0])  # 2 t.e has eigenvalues -1.98 along (1,1,1) and 0.99 across
+
+
+def _far_matrix(columns):
+    return 1.02 * (1 + 1j) * np.array(columns, dtype=np.complex128).T
+
+
+ROTATES_BEYOND = _far_matrix([(1, -1, 0), (1, -1, 0), (1, 1, 1)])
+PAIR_BEYOND = _far_matrix([(1, 1, 1), (1, 1, 1), (1, -1, 0)])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_transports_by_links_off_the_group(oracle, precision, sign):
+    N = (4, 3, 5)
+    f = O.new_fields(N)
+    f["U"][...] = ROTATES_BEYOND.T  # [.., j, i]
+    f["E"][...] = sign * ALONG
+    with Lattice(N, A, precision=precision) as lat:
+        lat.upload("U", f["U"])
+        lat.upload("E", f["E"])
+        held = lat.download_fields()
+        got, emt = lat.gauss(profile=True), lat.emt_map()
+        G = np.broadcast_to(ROTATES_BEYOND.conj(), O.identity_gauge(N).shape).copy()  # G = V^dagger, stored [.., j, i]
+        lat.upload("G", G)
+        g = O.links_as_matrices(lat.download("G"))
+        lat.coulomb_fix(0.08, 0)
+        EG = lat.download("EG")
+    want = oracle.gauss(held, N, A, profile=True)
+    for k in range(3):
+        assert np.allclose(got[k], want[k], rtol=1e-12, atol=0), k
+    want = oracle.emt_map(held, N, A)
+    assert np.max(np.abs(emt - want)) <= 1e-12 * np.max(np.abs(want))
+    want = _rotated(g[..., None, :, :], held["E"])
+    assert np.max(np.abs(EG - want)[1:-1]) <= (1e-12 if precision == "fp64" else 1e-7) * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("N", [(4, 3, 8), (16, 16, 80)])  # a site over four warps, or in one thread
+@pytest.mark.parametrize("which", ["Jp", "Jm"])
+def test_currents_through_links_off_the_group(which, N):
+    """JStat after one step at the slice above a layer of such z links: its rotation is by that link, its plaquettes are not.
+    The pair of rotations takes the last diagonal entry from the trace, as the FP64 kernels do."""
+    dt, z0 = 0.1, 3
+    f = O.random_fields(N, 94, link_amp=0.3, e_amp=0.1, j_amp=0.0)
+    f["U"][z0 + 1, ..., 2, :, :] = PAIR_BEYOND.T
+    f[which][...] = ALONG
+    with Lattice(N, A) as lat:
+        lat.upload_fields(f)
+        lat.set_step_method("plaquette")
+        lat.step(dt, 1)
+        got = lat.download(which + "Stat")[z0 + 2]
+    C = PAIR_BEYOND.conj().T @ O.herm_from_algebra(ALONG) @ PAIR_BEYOND
+    C[2, 2] = -(C[0, 0] + C[1, 1])
+    want = (-1 if which == "Jp" else 1) * dt / A[2] * (ALONG - O.algebra_from_herm(C))
+    assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
