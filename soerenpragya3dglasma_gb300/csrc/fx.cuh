@@ -246,6 +246,23 @@ __device__ __forceinline__ void entry_nn(const M& A, int i, const M& B, const R 
   }
 }
 
+// The rows of 1 + A must have norm one (to 10 %): looked at where an entry of A may reach 1/8.
+__device__ __forceinline__ void unit_rows(const M& A, int e, Guard& g) {
+  if (e < -2) return;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    ll n = 0;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const C& a = A.e[i + 3 * j];
+      const int x = (a.re.h >> -e) + (i == j ? kOneH : 0), y = a.im.h >> -e;
+      n += (ll)x * x + (ll)y * y;
+    }
+    const int t = (int)(n >> 32);  // 2^56 is one: 2^24 here
+    g.bad |= n < 0 || t < (int)(0.81 * (1 << 24)) || t > (int)(1.21 * (1 << 24));
+  }
+}
+
 // w = (1 + A)(1 + B) - 1, its exponent at most 0 and at least 3 above A's and B's (below the cap), so |w| < 2^e / 2
 // there; at the cap |w| <= 2.
 __device__ __forceinline__ void near_product(const M& A, int ea, const M& B, int eb, M& W, int& ew, Guard& g) {
@@ -264,19 +281,7 @@ __device__ __forceinline__ void near_product(const M& A, int ea, const M& B, int
       W.e[i + 3 * j].re = split((finish(re) >> kk) + (join(a.re) >> ka) + (join(b.re) >> kb));
       W.e[i + 3 * j].im = split((finish(im) >> kk) + (join(a.im) >> ka) + (join(b.im) >> kb));
     }
-  if (ew == 0) {  // entries near or above 1/8: the rows of 1 + w must have norm one (to 10 %)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      ll n = 0;
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        const int x = W.e[i + 3 * j].re.h + (i == j ? kOneH : 0), y = W.e[i + 3 * j].im.h;
-        n += (ll)x * x + (ll)y * y;
-      }
-      const int t = (int)(n >> 32);  // 2^56 is one: 2^24 here
-      g.bad |= n < 0 || t < (int)(0.81 * (1 << 24)) || t > (int)(1.21 * (1 << 24));
-    }
-  }
+  if (ew == 0) unit_rows(W, 0, g);  // entries near or above 1/8
 }
 
 // The anti-Hermitian part of a matrix P: y_ij = Im(P_ij + P_ji), x_ij = Re(P_ij - P_ji) for (ij) = 01, 02, 12 and
@@ -299,10 +304,9 @@ __device__ __forceinline__ ll component(const Anti& p, int k) {
   }
 }
 
-// P = W V^dagger (kNear: (1 + w)(1 + v)^dagger of two near products)
-template <bool kNear = true>
+// P = (1 + w)(1 + v)^dagger of two near products
 __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, int ev, Anti& o) {
-  const int ep = kNear ? max(ew, ev) : ew + ev;
+  const int ep = max(ew, ev);
   const int k = min(ep - ew - ev, 63), kw = min(ep - ew, 63), kv = min(ep - ev, 63);
   o.e = ep;
   constexpr int pi[3] = {0, 0, 1}, pj[3] = {1, 2, 2};
@@ -324,7 +328,6 @@ __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, 
     }
     o.y[n] = finish_diff(yp, yn) >> k;
     o.x[n] = finish_diff(xp, xn) >> k;
-    if (!kNear) continue;
     const ll yw = join(W.e[i + 3 * j].im) + join(W.e[j + 3 * i].im), yv = join(V.e[i + 3 * j].im) + join(V.e[j + 3 * i].im);
     const ll xw = join(W.e[i + 3 * j].re) - join(W.e[j + 3 * i].re), xv = join(V.e[j + 3 * i].re) - join(V.e[i + 3 * j].re);
     o.y[n] += (yw >> kw) - (yv >> kv);
@@ -339,45 +342,8 @@ __device__ __forceinline__ void plaquette_parts(const M& W, int ew, const M& V, 
       mad(p, w.im, v.re);
       mad(q, w.re, v.im);
     }
-    o.d[i] = finish_diff(p, q) >> k;
-    if (kNear) o.d[i] += (join(W.e[4 * i].im) >> kw) - (join(V.e[4 * i].im) >> kv);
+    o.d[i] = (finish_diff(p, q) >> k) + (join(W.e[4 * i].im) >> kw) - (join(V.e[4 * i].im) >> kv);
   }
-}
-
-// A B of two matrices with entries up to one, B daggered if kDag; watched, so that the next product has room
-template <bool kDag>
-__device__ __forceinline__ void product(const M& A, const M& B, M& P, Guard& g) {
-  R nB[9];
-#pragma unroll
-  for (int n = 0; n < 9; n++) nB[n] = neg(B.e[n].im);
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      Acc re = acc_half(), im = acc_half();
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        const int n = kDag ? j + 3 * k : k + 3 * j;
-        const C& a = A.e[i + 3 * k];
-        mad(re, a.re, B.e[n].re);
-        mad(re, a.im, kDag ? B.e[n].im : nB[n]);
-        mad(im, a.im, B.e[n].re);
-        mad(im, a.re, kDag ? nB[n] : B.e[n].im);
-      }
-      watch(g, re.hh, im.hh);
-      P.e[i + 3 * j].re = split(finish(re));
-      P.e[i + 3 * j].im = split(finish(im));
-    }
-}
-// Re tr(A B^dagger) 2^60 of two plain matrices
-__device__ __forceinline__ ll trace_nd(const M& A, const M& B) {
-  Acc a = acc_half();
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    mad(a, A.e[k].re, B.e[k].re);
-    mad(a, A.e[k].im, B.e[k].im);
-  }
-  return finish(a);
 }
 
 // -Re tr(P - 1) 2^(60-e), e = max(ew, ev), of the same P: 3 - Re tr P without its cancellation

@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(kGfThreads, 1) update_kernel(Geometry g, const
 
 // ---- what the deviation needs of the transformed links UG_mu(x) = G(x) U_mu(x) G^d(x+mu), and no more: the eight
 // ReTr(i t^a UG) and Re tr UG, 27 numbers a site instead of 54 written and read (A[(9 mu + k) V + x]); the sweeps need the
-// links themselves only at their end.  One thread per link.
+// links themselves only at their end.  One thread per link; in fixed point as (1 + A)(1 + B)(1 + C)^d, so that the deviation
+// of weak fields keeps its digits.
 static __device__ __noinline__ void link_deviation_fp64(const Mat<double>& gx, const Mat<double>& u, const Mat<double>& gy,
                                                  Alg<double>& al, double& tr) {
   Mat<double> t, o;
@@ -318,17 +319,19 @@ __global__ void __launch_bounds__(kLinkThreads, 3) link_deviation_kernel(Geometr
   const long long s = idx + g.plane, sf = forward(g, idx, mu);
   fx::Guard guard = fx::guard_init();
   fx::M a, b, t;
-  fx::link_plain(G, g.S, 0, s, a, guard);
-  fx::link_plain(U, g.S, mu, s, b, guard);
-  fx::product<false>(a, b, t, guard);
-  fx::link_plain(G, g.S, 0, sf, a, guard);
+  int ea, eb, et;
+  fx::link_near(G, g.S, 0, s, a, ea, guard);
+  fx::link_near(U, g.S, mu, s, b, eb, guard);
+  fx::near_product(a, ea, b, eb, t, et, guard);
+  fx::link_near(G, g.S, 0, sf, a, ea, guard);
+  fx::unit_rows(a, ea, guard);
   fx::Anti p;
-  fx::plaquette_parts<false>(t, 0, a, 0, p);
+  fx::plaquette_parts(t, et, a, ea, p);
   Alg<double> al;
 #pragma unroll
   for (int k = 0; k < 8; k++)
-    al.a[k] = fx::from_fixed(fx::component(p, k), -fx::kScale) * (k == 7 ? -0.5 * Consts<double>::inv_sqrt3() : -0.5);
-  double tr = fx::from_fixed(fx::trace_nd(t, a), -fx::kScale);
+    al.a[k] = fx::from_fixed(fx::component(p, k), p.e - fx::kScale) * (k == 7 ? -0.5 * Consts<double>::inv_sqrt3() : -0.5);
+  double tr = 3.0 - fx::from_fixed(fx::plaquette_trace(t, et, a, ea), p.e - fx::kScale);
   if (fx::tripped(guard)) {
     Mat<double> gx, u, gy;
     Alg<double> r;
@@ -741,15 +744,17 @@ __global__ void __launch_bounds__(kLinkThreads, 3) transform_links_kernel(Geomet
   const long long s = idx + g.plane, sf = forward(g, idx, mu);
   fx::Guard guard = fx::guard_init();
   fx::M a, b, t;
-  fx::link_plain(G, g.S, 0, s, a, guard);
-  fx::link_plain(U, g.S, mu, s, b, guard);
-  fx::product<false>(a, b, t, guard);
-  fx::link_plain(G, g.S, 0, sf, a, guard);
-  fx::product<true>(t, a, b, guard);
+  int ea, eb, et;
+  fx::link_near(G, g.S, 0, s, a, ea, guard);
+  fx::link_near(U, g.S, mu, s, b, eb, guard);
+  fx::near_product(a, ea, b, eb, t, et, guard);
+  fx::link_near(G, g.S, 0, sf, a, ea, guard, true);
+  fx::near_product(t, et, a, ea, b, eb, guard);
   Mat<double> o;
 #pragma unroll
   for (int k = 0; k < 9; k++)
-    o.e[k] = mk<double>(fx::from_fixed(fx::join(b.e[k].re), -fx::kScale), fx::from_fixed(fx::join(b.e[k].im), -fx::kScale));
+    o.e[k] = mk<double>((k % 4 == 0 ? 1.0 : 0.0) + fx::from_fixed(fx::join(b.e[k].re), eb - fx::kScale),
+                        fx::from_fixed(fx::join(b.e[k].im), eb - fx::kScale));
   if (fx::tripped(guard)) {
     Mat<double> gx, u, gy, r;
     ld_d(G, g.S, 0, s, gx);

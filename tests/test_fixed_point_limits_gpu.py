@@ -146,3 +146,60 @@ def test_currents_through_links_off_the_group(which, N):
     C[2, 2] = -(C[0, 0] + C[1, 1])
     want = (-1 if which == "Jp" else 1) * dt / A[2] * (ALONG - O.algebra_from_herm(C))
     assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+# ---- Coulomb gauge fixing: weak fields keep their digits, transformations off the group go through FP64
+def _weak_links(N, seed, size):
+    """1 + i q - q^2 / 2 with q of `size`: the entries themselves, where an eigenvector form would round at 1e-16."""
+    q = size * O.herm_from_algebra(np.random.default_rng(seed).standard_normal((N[2] + 2, N[1], N[0], 3, 8)))
+    return O.matrices_to_links(np.eye(3) + 1j * q - 0.5 * q @ q)
+
+
+def _synced(F):
+    O.sync_ghosts(F)
+    return F
+
+
+@pytest.mark.parametrize("size", [1e-4, 1e-10, 1e-20, 1e-60])
+@pytest.mark.parametrize("fft_fp32", [False, True])
+def test_gauge_fixing_of_weak_fields(oracle, size, fft_fp32):
+    """Deviations relative to the fields' size.  The log's steps are 3 - tr X ~ size^2, which FP64 forms cannot hold."""
+    N = (6, 5, 8)
+    f = O.random_fields(N, 95, e_amp=0.1)
+    f["U"] = _synced(_weak_links(N, 96, size))
+    G = O.identity_gauge(N)
+    iters = 1 if fft_fp32 else 3  # FP32 transforms round the step at 6e-8
+    st, olog, UG, _ = oracle.coulomb_fix(f, G, N, (1.0, 1.0, 1.0), 0.08, iters, tol=1e-300,
+                                         flags=O.GF_PROJECT_ZERO_MODE | O.GF_OPEN_Z)
+    assert st == 0
+    with Lattice(N) as lat:
+        lat.upload("U", f["U"])
+        lat.upload("E", f["E"])
+        log = lat.coulomb_fix(0.08, iters, tol=1e-300, project_zero_mode=True, open_z=True, fft_fp32=fft_fp32)
+        got = lat.download("UG")
+    assert np.allclose(log[:, 1:3], olog[:, 1:3], rtol=1e-12, atol=0)
+    assert np.allclose(log[:, 5:], olog[:, 5:], rtol=1e-12, atol=0)
+    if not fft_fp32:
+        off = ~np.eye(3, dtype=bool)
+        assert np.max(np.abs((got - UG)[1:-1][..., off])) <= 1e-12 * np.max(np.abs(UG[1:-1][..., off]))
+        assert np.max(np.abs((got - UG)[1:-1].imag)) <= 1e-12 * np.max(np.abs(UG[1:-1].imag))
+
+
+@pytest.mark.parametrize("scale", [1.02, 0.6])
+def test_gauge_transformations_off_the_group(oracle, scale):
+    """G of equal entries below 1.03, U in SU(3): G U G^dagger has entries up to six."""
+    N = (4, 3, 6)
+    f = O.random_fields(N, 97, link_amp=0.8, e_amp=0.1)
+    G = np.full(O.identity_gauge(N).shape, scale * (1 + 1j))
+    H = G.copy()
+    st, olog, UG, EG = oracle.coulomb_fix(f, G, N, (1.0, 1.0, 1.0), 1e-3, 1)
+    assert st == 0
+    with Lattice(N) as lat:
+        lat.upload("U", f["U"])
+        lat.upload("E", f["E"])
+        lat.upload("G", H)
+        log = lat.coulomb_fix(1e-3, 1)
+        got = {k: lat.download(k) for k in ("G", "UG", "EG")}
+    assert np.allclose(log, olog, rtol=1e-11, atol=1e-13)
+    for k, want in (("G", G), ("UG", UG), ("EG", EG)):
+        assert np.max(np.abs(got[k] - want)[1:-1]) <= 1e-12 * np.max(np.abs(want)), k
