@@ -114,19 +114,14 @@ __device__ __forceinline__ void gf_decode(long long idx, int nx, int ny, long lo
 
 // w(x) = sum_mu c_mu (UG_mu(x) + UG_mu^d(x - mu)) at interior site s = (x, y, z); c2 = 0 when Nz = 1
 // (GET_LOCAL_GAUGE_VIOLATION, S/GAUGETRANSFORMATION/CoulombGaugeDeviation.cpp:23-41).
-// open_top (GLASMA_GF_OPEN_Z): the forward z link of the top slice, which points into the ghost slice,
-// is left out, so that every link in w is counted at both of its ends (the backward z link of slice 0
-// is the identity ghost, which adds nothing to Delta) and Delta is the gradient of one functional.
 template <typename T>
 __device__ __forceinline__ void site_w(const Geometry& g, const cx<T>* UG, int x, int y, int z, long long s, double c0,
-                                       double c1, double c2, Mat<double>& w, int open_top = 0) {
+                                       double c1, double c2, Mat<double>& w) {
   const double c[3] = {c0, c1, c2};
   const long long back[3] = {nbr(g, x, y, z, -1, 0, 0), nbr(g, x, y, z, 0, -1, 0), s - g.plane};
-  const double fwd2 = (open_top && z == g.nz - 1) ? 0.0 : 1.0;
   set_zero(w);
   for (int mu = 0; mu < 3; mu++) {
     if (c[mu] == 0.0) continue;
-    const double cf = mu == 2 ? fwd2 : 1.0;
     Mat<double> u, d;
     ld_d(UG, g.S, mu * 9, s, u);
     ld_d(UG, g.S, mu * 9, back[mu], d);
@@ -135,43 +130,10 @@ __device__ __forceinline__ void site_w(const Geometry& g, const cx<T>* UG, int x
 #pragma unroll
       for (int j = 0; j < 3; j++) {
         const int k = i + 3 * j, kt = j + 3 * i;
-        w.e[k].re += c[mu] * (cf * u.e[k].re + d.e[kt].re);
-        w.e[k].im += c[mu] * (cf * u.e[k].im - d.e[kt].im);
+        w.e[k].re += c[mu] * (u.e[k].re + d.e[kt].re);
+        w.e[k].im += c[mu] * (u.e[k].im - d.e[kt].im);
       }
   }
-}
-
-// ---- deviation: X[q] = Delta^{2q} + i Delta^{2q+1}, q < 4 (Delta is real: two colours share one
-// complex transform, and since the acceleration multiplies by a real factor even in p, the inverse
-// transform returns them in the real and imaginary parts); partials {max|Delta|, sum Delta^2,
-// min ReTr w, sum ReTr w}
-template <typename T, typename C>
-__global__ void __launch_bounds__(kGfThreads) deviation_kernel(Geometry g, const cx<T>* UG, double c0, double c1,
-                                                               double c2, C* X, double* partials, int open_top) {
-  double v[4] = {0.0, 0.0, 1.0e300, 0.0};
-  const int op[4] = {1, 0, 2, 0};
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < g.vol;
-       idx += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    gf_decode(idx, g.nx, g.ny, g.vol, x, y, z);
-    const long long s = idx + g.plane;
-    Mat<double> w;
-    site_w(g, UG, x, y, z, s, c0, c1, c2, w, open_top);
-    Alg<double> dev;
-    retr_itg(w, 1.0, dev);
-#pragma unroll
-    for (int a = 0; a < 8; a++) {
-      v[0] = fmax(v[0], fabs(dev.a[a]));
-      v[1] += dev.a[a] * dev.a[a];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      X[(long long)q * g.vol + idx] = cmk((decltype(C::x))dev.a[2 * q], (decltype(C::x))dev.a[2 * q + 1]);
-    const double lf = w.e[0].re + w.e[4].re + w.e[8].re;
-    v[2] = fmin(v[2], lf);
-    v[3] += lf;
-  }
-  red::block_reduce_store<4>(v, op, partials + (long long)blockIdx.x * 4);
 }
 
 // ---- momentum-space acceleration of the 4 colour-pair planes
@@ -292,9 +254,20 @@ __global__ void __launch_bounds__(kGfThreads, 1) update_kernel(Geometry g, const
 }
 
 // ---- what the deviation needs of the transformed links UG_mu(x) = G(x) U_mu(x) G^d(x+mu), and no more: the eight
-// ReTr(i t^a UG) and Re tr UG, 27 numbers a site instead of 54 written and read (A[(9 mu + k) V + x]); the sweeps need the
-// links themselves only at their end.  One thread per link; in fixed point as (1 + A)(1 + B)(1 + C)^d, so that the deviation
-// of weak fields keeps its digits.
+// ReTr(i t^a UG) and Re tr UG, 27 numbers a site instead of 54 written and read (A[(9 mu + k) stride + x]); the sweeps need
+// the links themselves only at their end, and until then these numbers lie in UG's own memory (deviations_in).  One thread
+// per link; in fixed point as (1 + A)(1 + B)(1 + C)^d, so that the deviation of weak fields keeps its digits.
+// One double per complex component of UG, in its interior slices: the ghost slices stay as they are.
+template <typename T>
+struct Deviations {
+  double* p;
+  long long stride;
+};
+template <typename T>
+Deviations<T> deviations_in(const Geometry& g, void* UG) {
+  constexpr long long per = sizeof(cx<T>) / sizeof(double);  // doubles per complex number: 2 or 1
+  return {static_cast<double*>(UG) + per * g.plane, per * g.S};
+}
 static __device__ __noinline__ void link_deviation_fp64(const Mat<double>& gx, const Mat<double>& u, const Mat<double>& gy,
                                                  Alg<double>& al, double& tr) {
   Mat<double> t, o;
@@ -312,7 +285,7 @@ constexpr int kLinkThreads = 128;
 template <typename T>
 __global__ void __launch_bounds__(kLinkThreads, 3) link_deviation_kernel(Geometry g, const cx<T>* __restrict__ U,
                                                                          const cx<T>* __restrict__ G,
-                                                                         double* __restrict__ A) {
+                                                                         Deviations<T> A) {
   const int mu = blockIdx.y;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= g.vol) return;
@@ -343,10 +316,10 @@ __global__ void __launch_bounds__(kLinkThreads, 3) link_deviation_kernel(Geometr
     al = r;
     tr = q;
   }
-  double* o = A + (long long)(mu * 9) * g.vol + idx;
+  double* o = A.p + (long long)(mu * 9) * A.stride + idx;
 #pragma unroll
-  for (int k = 0; k < 8; k++) o[(long long)k * g.vol] = al.a[k];
-  o[8 * g.vol] = tr;
+  for (int k = 0; k < 8; k++) o[(long long)k * A.stride] = al.a[k];
+  o[8 * A.stride] = tr;
 }
 __global__ void __launch_bounds__(kLinkThreads) link_deviation32_kernel(Geometry g, const cx<float>* __restrict__ U,
                                                                         const cx<float>* __restrict__ G,
@@ -368,12 +341,16 @@ __global__ void __launch_bounds__(kLinkThreads) link_deviation32_kernel(Geometry
   for (int k = 0; k < 8; k++) p[(long long)k * g.vol] = al.a[k];
   p[8 * g.vol] = o.e[0].re + o.e[4].re + o.e[8].re;
 }
-// Delta = sum_mu c_mu (al_mu(x) - al_mu(x-mu)) (ReTr(i t V^d) = -ReTr(i t V)) and Re tr w; X and the monitors as
-// deviation_kernel's.  Re: the sweeps' arithmetic; FP32 sums per thread, FP64 beyond.  The backward z link of slice 0 is
-// the identity ghost, with trace `ghost`: 3 in FP64 as in the reference's functional; the FP32 sweeps, whose links have no
-// ghosts, log the functional of the links inside the lattice (0).
+// Delta = sum_mu c_mu (al_mu(x) - al_mu(x-mu)) (ReTr(i t V^d) = -ReTr(i t V)) and Re tr w; X[q] = Delta^{2q} + i Delta^{2q+1},
+// q < 4 (Delta is real: two colours share one complex transform, and since the acceleration multiplies by a real factor even
+// in p, the inverse transform returns them in the real and imaginary parts); partials {max|Delta|, sum Delta^2, min ReTr w,
+// sum ReTr w}.  open_top (GLASMA_GF_OPEN_Z): the forward z link of the top slice, which points into the ghost slice, is left
+// out, so that every link in w is counted at both of its ends and Delta is the gradient of one functional.  Re: the sweeps'
+// arithmetic; FP32 sums per thread, FP64 beyond.  The backward z link of slice 0 is the identity ghost, which adds nothing to
+// Delta, with trace `ghost`: 3 in FP64 as in the reference's functional; the FP32 sweeps, whose links have no ghosts, log the
+// functional of the links inside the lattice (0).
 template <typename Re, typename C>
-__global__ void __launch_bounds__(kGfThreads) gather_deviation_kernel(Geometry g, const Re* __restrict__ A, Re c0, Re c1,
+__global__ void __launch_bounds__(kGfThreads) gather_deviation_kernel(Geometry g, const Re* __restrict__ A, long long stride, Re c0, Re c1,
                                                                       Re c2, Re ghost, C* X, double* partials,
                                                                       int open_top) {
   Re tmax = 0, tsq = 0, tmin = Re(3.0e38), tlf = 0;
@@ -394,10 +371,10 @@ __global__ void __launch_bounds__(kGfThreads) gather_deviation_kernel(Geometry g
       const Re cb = mu == 2 && z == 0 ? Re(0) : c;
       const long long back = mu == 0 ? (x > 0 ? idx - 1 : idx + g.nx - 1)
                                      : (mu == 1 ? (y > 0 ? idx - g.nx : idx + g.plane - g.nx) : (z > 0 ? idx - g.plane : idx));
-      const Re* p = A + (long long)(mu * 9) * V;
+      const Re* p = A + (long long)(mu * 9) * stride;
 #pragma unroll
-      for (int k = 0; k < 8; k++) dev.a[k] += cf * p[(long long)k * V + idx] - cb * p[(long long)k * V + back];
-      lf += cf * p[8 * V + idx] + c * (mu == 2 && z == 0 ? ghost : p[8 * V + back]);
+      for (int k = 0; k < 8; k++) dev.a[k] += cf * p[(long long)k * stride + idx] - cb * p[(long long)k * stride + back];
+      lf += cf * p[8 * stride + idx] + c * (mu == 2 && z == 0 ? ghost : p[8 * stride + back]);
     }
 #pragma unroll
     for (int a = 0; a < 8; a++) {
@@ -1156,7 +1133,6 @@ struct GaugeFixState {
   double p2a[3] = {0, 0, 0};  // the spacings the table was made for
   std::map<int, double2*> twiddles;
   std::map<int, float2*> twiddles32;
-  double* A = nullptr;  // the FP64 sweeps' 27 numbers per site (link_deviation_kernel), on first use
   std::vector<double> host_results;
 };
 
@@ -1329,24 +1305,20 @@ int run_impl(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_iter
   const Geometry& g = a.g;
   cudaStream_t st = a.stream;
   cx<T>* G = static_cast<cx<T>*>(a.G);
-  const cx<T>* UG = static_cast<const cx<T>*>(a.UG);
   auto cuda_err = [&](cudaError_t e, const char* where) {
     *err = std::string(where) + ": " + cudaGetErrorString(e);
     return GLASMA_ERR_CUDA;
   };
   cudaError_t e;
   const bool sweeps = n_start < max_iters && tol < 1.0;
-  // The sweeps read 27 numbers of UG per site (A); without room for them they go over UG itself.
-  if (sweeps && !s->A && cudaMalloc(&s->A, sizeof(double) * 27 * g.vol) != cudaSuccess) {
-    cudaGetLastError();
-    s->A = nullptr;
-  }
-  double* const A = s->A;
+  const Deviations<T> A = deviations_in<T>(g, a.UG);
   const dim3 lb((unsigned)((g.vol + kLinkThreads - 1) / kLinkThreads), 3);
+  const bool fft32 = (flags & GLASMA_GF_FFT_FP32) != 0;
+  if (fft32 && (e = ensure_twiddles32(s, st)) != cudaSuccess) return cuda_err(e, "FP32 twiddles");
+  if ((e = ensure_p2tab(s, g, st)) != cudaSuccess) return cuda_err(e, "momentum table");
   // GaugeTransformLinks reads the ghost G of the sweep before, then the ghosts are synced: the sync waits for the sweep's
   // verdict, so that a failing one can still leave its UG
   auto transform_links = [&]() {
-    if (!A) return transform_links_only<T>(a);
     link_deviation_kernel<T><<<lb, kLinkThreads, 0, st>>>(g, static_cast<const cx<T>*>(a.U), G, A);
     return cudaGetLastError();
   };
@@ -1365,24 +1337,17 @@ int run_impl(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_iter
   int n = n_start;
   int status = GLASMA_OK;
   const double minf0 = 2.0 * 3 * (1.0 / (g.a[0] * g.a[0]) + 1.0 / (g.a[1] * g.a[1]) + 1.0 / (g.a[2] * g.a[2]));
-  const bool fft32 = (flags & GLASMA_GF_FFT_FP32) != 0;
-  if (fft32 && (e = ensure_twiddles32(s, st)) != cudaSuccess) return cuda_err(e, "FP32 twiddles");
-  if ((e = ensure_p2tab(s, g, st)) != cudaSuccess) return cuda_err(e, "momentum table");
   double2* X64 = static_cast<double2*>(s->X);
   float2* X32 = static_cast<float2*>(s->X);
   const int project = (flags & GLASMA_GF_PROJECT_ZERO_MODE) ? 1 : 0;
   const int open_top = (flags & GLASMA_GF_OPEN_Z) ? 1 : 0;
   while (n < max_iters && gmax > tol) {
-    if (A && fft32)
-      gather_deviation_kernel<double, float2><<<nb, kGfThreads, 0, st>>>(g, A, cw[0], cw[1], cw[2], 3.0, X32, part_dev,
-                                                                         open_top);
-    else if (A)
-      gather_deviation_kernel<double, double2><<<nb, kGfThreads, 0, st>>>(g, A, cw[0], cw[1], cw[2], 3.0, X64, part_dev,
-                                                                          open_top);
-    else if (fft32)
-      deviation_kernel<T, float2><<<nb, kGfThreads, 0, st>>>(g, UG, cw[0], cw[1], cw[2], X32, part_dev, open_top);
+    if (fft32)
+      gather_deviation_kernel<double, float2><<<nb, kGfThreads, 0, st>>>(g, A.p, A.stride, cw[0], cw[1], cw[2], 3.0, X32,
+                                                                         part_dev, open_top);
     else
-      deviation_kernel<T, double2><<<nb, kGfThreads, 0, st>>>(g, UG, cw[0], cw[1], cw[2], X64, part_dev, open_top);
+      gather_deviation_kernel<double, double2><<<nb, kGfThreads, 0, st>>>(g, A.p, A.stride, cw[0], cw[1], cw[2], 3.0, X64,
+                                                                          part_dev, open_top);
     red::finish_kernel<4><<<1, red::kThreads, 0, st>>>(part_dev, (int)nb, 1 | (0 << 2) | (2 << 4) | (0 << 6), res);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "deviation");
     e = fft32 ? accelerate_planes<float2>(s, X32, s->p2tab32, project, s->twiddles32, st)
@@ -1414,7 +1379,7 @@ int run_impl(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_iter
     if (h[6] > 0.0) {
       *err = "gauge update left SU(3) by more than 1e-13 (the reference exits here)";
       status = GLASMA_ERR_NUMERICAL;
-      if (A) e = transform_links_only<T>(a);
+      e = transform_links_only<T>(a);
       if (e == cudaSuccess) e = copy_efield<T>(a);
       if (e != cudaSuccess) return cuda_err(e, "fields at the guard");
     }
@@ -1492,7 +1457,7 @@ int run_mixed(GaugeFixState* s, const GaugeFixArgs& a, double alpha, int max_ite
   double gmax = 1.0, best = 1e300;
   int n = 0, since_best = 0;
   while (n < max_iters && gmax > tol) {
-    gather_deviation_kernel<float, float2><<<nb, kGfThreads, 0, st>>>(g, c.A, cw[0], cw[1], cw[2], 0.f, X32, part_dev,
+    gather_deviation_kernel<float, float2><<<nb, kGfThreads, 0, st>>>(g, c.A, g.vol, cw[0], cw[1], cw[2], 0.f, X32, part_dev,
                                                                        open_top);
     red::finish_kernel<4><<<1, red::kThreads, 0, st>>>(part_dev, (int)nb, 1 | (0 << 2) | (2 << 4) | (0 << 6), res);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(e, "FP32 deviation");
@@ -1664,7 +1629,6 @@ cudaError_t launch_transform_charge(const GaugeFixArgs& a, const void* J, double
 void gaugefix_destroy(GaugeFixState* s) {
   if (!s) return;
   if (s->X) cudaFree(s->X);
-  if (s->A) cudaFree(s->A);
   if (s->p2tab) cudaFree(s->p2tab);
   if (s->p2tab32) cudaFree(s->p2tab32);
   for (auto& kv : s->twiddles) cudaFree(kv.second);

@@ -203,3 +203,38 @@ def test_gauge_transformations_off_the_group(oracle, scale):
     assert np.allclose(log, olog, rtol=1e-11, atol=1e-13)
     for k, want in (("G", G), ("UG", UG), ("EG", EG)):
         assert np.max(np.abs(got[k] - want)[1:-1]) <= 1e-12 * np.max(np.abs(want)), k
+
+
+@pytest.mark.parametrize("precision,mixed", [("fp64", False), ("fp64", True), ("fp32", False)])
+def test_gauge_sweeps_keep_no_memory(precision, mixed):
+    """What the sweeps need beyond the handle's fields and transforms is given back (27 doubles a site would be 85 MB here)."""
+    torch = pytest.importorskip("torch")
+    N = (64, 64, 96)
+    with Lattice(N, precision=precision) as lat:
+        lat.fill_synthetic(1)
+        lat.coulomb_fix(0.08, 0, mixed=mixed)
+        lat.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        lat.coulomb_fix(0.08, 3, mixed=mixed, open_z=True)
+        lat.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] < 16 << 20
+
+
+@pytest.mark.parametrize("N", [(4, 3, 5), (6, 5, 2)])
+def test_gauge_sweeps_of_fp32_handles(oracle, N):
+    """FP32 handles: the deviations of FP64 arithmetic, links and transformations stored in FP32; the ghost links stay."""
+    f = O.random_fields(N, 98, link_amp=0.1, e_amp=0.1)
+    with Lattice(N, precision="fp32") as lat:
+        lat.upload("U", f["U"])
+        lat.upload("E", f["E"])
+        held = {k: lat.download(k) for k in ("U", "E")}
+        G = O.identity_gauge(N)
+        st, olog, UG, EG = oracle.coulomb_fix(held, G, N, (1.0, 1.0, 1.0), 0.08, 2, flags=O.GF_PROJECT_ZERO_MODE)
+        log = lat.coulomb_fix(0.08, 2, project_zero_mode=True)
+        got = {k: lat.download(k) for k in ("G", "UG", "EG")}
+    assert st == 0
+    assert np.allclose(log[0], olog[0], rtol=1e-11, atol=1e-13)
+    assert np.allclose(log[1], olog[1], rtol=1e-5, atol=1e-6)
+    assert np.array_equal(got["UG"][[0, -1]], UG[[0, -1]])
+    for k, want in (("G", G), ("UG", UG), ("EG", EG)):
+        assert np.max(np.abs(got[k] - want)[1:-1]) <= 5e-7, k
