@@ -258,6 +258,8 @@ __global__ void __launch_bounds__(kGfThreads, 1) update_kernel(Geometry g, const
 // the links themselves only at their end, and until then these numbers lie in UG's own memory (deviations_in).  One thread
 // per link; in fixed point as (1 + A)(1 + B)(1 + C)^d, so that the deviation of weak fields keeps its digits.
 // One double per complex component of UG, in its interior slices: the ghost slices stay as they are.
+// 48x40x100: 115 us (86 with exponent 0 throughout, which lost the digits of weak fields); the whole links 140 us (101), with
+// two blocks per SM (147 with three).
 template <typename T>
 struct Deviations {
   double* p;
@@ -350,12 +352,14 @@ __global__ void __launch_bounds__(kLinkThreads) link_deviation32_kernel(Geometry
 // Delta, with trace `ghost`: 3 in FP64 as in the reference's functional; the FP32 sweeps, whose links have no ghosts, log the
 // functional of the links inside the lattice (0).
 template <typename Re, typename C>
-__global__ void __launch_bounds__(kGfThreads) gather_deviation_kernel(Geometry g, const Re* __restrict__ A, long long stride, Re c0, Re c1,
+__global__ void __launch_bounds__(kGfThreads) gather_deviation_kernel(Geometry g, const Re* __restrict__ A, long long A_stride, Re c0, Re c1,
                                                                       Re c2, Re ghost, C* X, double* partials,
                                                                       int open_top) {
   Re tmax = 0, tsq = 0, tmin = Re(3.0e38), tlf = 0;
   const int op[4] = {1, 0, 2, 0};
   const long long V = g.vol;
+  // the FP32 sweeps' numbers are a buffer of their own, without ghost slices
+  const long long stride = sizeof(Re) == 4 ? V : A_stride;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < V; idx += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
     gf_decode(idx, g.nx, g.ny, V, x, y, z);
@@ -713,7 +717,7 @@ static __device__ __noinline__ void transform_link_fp64(const Mat<double>& gx, c
   mul_nd(t, gy, o);
 }
 template <typename T>
-__global__ void __launch_bounds__(kLinkThreads, 3) transform_links_kernel(Geometry g, const cx<T>* __restrict__ U,
+__global__ void __launch_bounds__(kLinkThreads, 2) transform_links_kernel(Geometry g, const cx<T>* __restrict__ U,
                                                                           const cx<T>* __restrict__ G, cx<T>* UG) {
   const int mu = blockIdx.y;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
