@@ -238,3 +238,48 @@ def test_gauge_sweeps_of_fp32_handles(oracle, N):
     assert np.array_equal(got["UG"][[0, -1]], UG[[0, -1]])
     for k, want in (("G", G), ("UG", UG), ("EG", EG)):
         assert np.max(np.abs(got[k] - want)[1:-1]) <= 5e-7, k
+
+
+# ---- adjoint: cotangents that are not finite, or of other sizes than the forces they are rotated with
+DT = 0.1
+
+
+def _adjoint(f, N, precision, form):
+    with Lattice(N, A, precision=precision) as lat:
+        lat.upload_fields(f)
+        return lat.adjoint(DT, 2, 3, 6, form, checkpoint_every=1)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_adjoint_keeps_a_nan_to_its_cotangents(precision):
+    """A NaN weight on E_x in slices 3 to 5.  The x links of slice 6 get a cotangent only as the far side of the plaquettes
+    that begin in slice 5, so two steps' E_x gradient there is NaN through that rotation alone.  Slices the NaN does not
+    reach have the gradient of the other weights."""
+    N = (4, 5, 12)
+    f = O.random_fields(N, 99, link_amp=0.25, e_amp=0.3, j_amp=0.05)
+    _, g = _adjoint(f, N, precision, ((float("nan"), 0.5, 0.5, 0.5, 0.5, 0.5), (0,) * 6))
+    _, want = _adjoint(f, N, precision, ((0, 0.5, 0.5, 0.5, 0.5, 0.5), (0,) * 6))
+    gx = g["E"][1:-1, ..., 0, :]
+    assert np.all(np.isnan(gx[3:7]))
+    for k in g:
+        far = np.r_[1:2, 9:13]
+        assert np.all(np.isfinite(g[k][far])), k
+        assert np.allclose(g[k][far], want[k][far], rtol=1e-4, atol=1e-6), k
+
+
+def _gradients_scale(precision, sizes, eps, tiny):
+    N = (4, 5, 10)
+    f = O.random_fields(N, 100, link_amp=0.25, e_amp=0.3, j_amp=0.05)
+    _, want = _adjoint(f, N, precision, ((0.5,) * 6, (0,) * 6))
+    for size in sizes:
+        _, g = _adjoint(f, N, precision, ((0.5 * size,) * 6, (0,) * 6))
+        for k in g:
+            top = np.max(np.abs(want[k]))
+            assert np.max(np.abs(g[k] / size - want[k])) <= eps * top + 1000 * tiny / size, (k, size)
+
+
+@pytest.mark.parametrize("precision,sizes", [("fp64", [1e-30, 1e-100, 1e100]), ("fp32", [1e-12, 1e-25, 1e-30, 1e-34, 1e20])])
+def test_adjoint_is_linear_in_its_weights(precision, sizes):
+    """Cotangents of any size the arithmetic holds give the gradient of weights of one times that size (numbers that
+    become subnormal on the way lose what they lose there)."""
+    _gradients_scale(precision, sizes, *((1e-12, 5e-324) if precision == "fp64" else (3e-5, 1.4e-45)))
