@@ -161,6 +161,12 @@ __device__ __forceinline__ double from_fixed_fp64(ll q, int k) {
 template <typename T>
 constexpr int kMinExpOf = sizeof(T) == 8 ? -900 : -139;
 constexpr int kMinExp = kMinExpOf<double>;
+// High words of numbers below 2^kMinExp (kHalf: 2^(kMinExp/2)) that are not zero: they would keep fewer than their digits, so
+// FP64 takes them.  (Numbers below 2^-1042, whose high word is zero, count as zeros; every float is held.)
+template <bool kHalf = false>
+__device__ __forceinline__ bool tiny(int top) {
+  return (unsigned)(top - 1) < (unsigned)((1022 + (kHalf ? kMinExp / 2 : kMinExp)) << 20) - 1;
+}
 // |v| < 2^exponent_of(largest |high word| of v)
 __device__ __forceinline__ int exponent_of(int habs) { return (habs >> 20) - 1022; }
 constexpr int kMaxEntryHi = 0x3FF07AE1;  // 1.03
@@ -216,6 +222,7 @@ __device__ __forceinline__ void link_near(const cx<T>* __restrict__ U, I S, int 
   constexpr int least = kMinExpOf<T>;
   const int ed = dor == 0 ? least : 64 - __clzll(dor) - kScale;  // |diagonal - 1| < 2^ed
   int ee = max(max(exponent_of(top), ed), least);
+  if (sizeof(T) == 8) g.bad |= ee == least && top != 0;  // tiny
   ee = min(ee, 0);
   e = ee;
   const int kb = shift(kScale - ee);
@@ -525,7 +532,7 @@ __device__ __forceinline__ void herm_one(const Alg<T>& p, M& m, int& e, Guard& g
   int top = 0;
 #pragma unroll
   for (int k = 0; k < 8; k++) top = max(top, habs(p.a[k]));
-  g.bad |= top >= 0x43100000;  // 2^50 or more, or not finite
+  g.bad |= top >= 0x43100000 || (sizeof(T) == 8 && tiny(top));  // 2^50 or more, or not finite
   const int em = max(exponent_of(min(top, 0x43100000)), kMinExpOf<T>) + 2;
   e = em;
   const int sh = shift(kScale - em);
@@ -549,7 +556,7 @@ __device__ __forceinline__ void herm_pair(const Alg<double>& p, const Alg<double
   int top = 0;
 #pragma unroll
   for (int k = 0; k < 8; k++) top = max(top, max(habs(p.a[k]), habs(q.a[k])));
-  g.bad |= top >= 0x43100000;  // 2^50 or more, or not finite
+  g.bad |= top >= 0x43100000 || tiny(top);  // 2^50 or more, or not finite
   const int em = max(exponent_of(min(top, 0x43100000)), kMinExp) + 2;
   e = em;
   const int kb = shift(kScale - em);
@@ -641,7 +648,7 @@ __device__ __forceinline__ bool near_exp(double c, const Alg<double>& al, M& X, 
     q.a[k] = c * al.a[k];
     top = max(top, habs(q.a[k]));
   }
-  if (top >= 0x3ff00000) return false;  // also NaN and infinity
+  if (top >= 0x3ff00000 || tiny(top)) return false;  // also NaN and infinity
   const int em = max(exponent_of(top), kMinExp) + 1;
   const int sh = shift(kScale - em);
   const ll s8 = to_fixed(q.a[7] * Consts<double>::inv_sqrt3(), sh), q2 = to_fixed(q.a[2], sh);
@@ -891,7 +898,7 @@ constexpr int kMaxHi = 0x43100000;  // 2^50
 __device__ __forceinline__ bool cross(const Alg<double>& a, const Alg<double>& b, Alg<double>& out) {
   const double a8 = a.a[7] * kRoot3, b8 = b.a[7] * kRoot3;
   const int ta = top_of(a, a8), tb = top_of(b, b8);
-  if (max(ta, tb) >= kMaxHi) return false;
+  if (max(ta, tb) >= kMaxHi || tiny<true>(ta) || tiny<true>(tb)) return false;  // the product's exponent is the sum
   const int ea = max(exponent_of(ta), kMinExp / 2), eb = max(exponent_of(tb), kMinExp / 2) + 1;
   R A[8], B[8];
   ll c[8];
@@ -911,7 +918,7 @@ __device__ __forceinline__ bool trace_with(const Mat<double>& h, const Alg<doubl
   for (int j = 0; j < 3; j++)
 #pragma unroll
     for (int i = 0; i <= j; i++) th = max(th, max(habs(h.e[i + 3 * j].re), habs(h.e[i + 3 * j].im)));
-  if (max(th, tn) >= kMaxHi) return false;
+  if (max(th, tn) >= kMaxHi || tiny<true>(th) || tiny<true>(tn)) return false;
   // sums of two diagonal entries stay below 1, those of 2 t.n (up to 1.16 of the components) below 1 too
   const int eh = max(exponent_of(th), kMinExp / 2) + 1, en = max(exponent_of(tn), kMinExp / 2) + 2;
   const int sh = shift(kScale - eh), sn = shift(kScale - en);
@@ -976,12 +983,13 @@ __device__ __forceinline__ bool trace_with(const Mat<double>& h, const Alg<doubl
   return true;
 }
 
-// sum_n (q x)^n l / (n + 1)! in fixed point, n up to `terms`; inv[n] = 1 / n.  |q| below one in every component.
+// sum_n (q x)^n l / (n + 1)! in fixed point, n up to `terms`; inv[n] = 1 / n.  The caller has |q| < 1 (as a vector), so no term
+// is larger than l and the sum below 2 |l|; a component of q, the eighth times sqrt 3, then stays below 2.
 __device__ __forceinline__ bool exp_series(const Alg<double>& q, const Alg<double>& l, int terms, const double* inv,
                                            Alg<double>& out) {
   const double q8 = q.a[7] * kRoot3, l8 = l.a[7] * kRoot3;
   const int tq = top_of(q, q8), tl = top_of(l, l8);
-  if (tq >= 0x40000000 || tl >= kMaxHi) return false;  // 2
+  if (tq >= 0x40000000 || tl >= kMaxHi || tiny(tl)) return false;  // 2
   const int eq = max(exponent_of(tq), kMinExp), el = max(exponent_of(tl), kMinExp) + 1;
   const int down = min(-min(eq, 0), 63), up = max(eq, 0);
   R Q[8], T[8];

@@ -283,3 +283,36 @@ def test_adjoint_is_linear_in_its_weights(precision, sizes):
     """Cotangents of any size the arithmetic holds give the gradient of weights of one times that size (numbers that
     become subnormal on the way lose what they lose there)."""
     _gradients_scale(precision, sizes, *((1e-12, 5e-324) if precision == "fp64" else (3e-5, 1.4e-45)))
+
+
+# ---- FP64 numbers below the format's smallest exponents (2^-900, 2^-450 where two exponents add up)
+@pytest.mark.parametrize("size", [1e-265, 1e-275, 1e-285, 1e-295])
+def test_the_thinnest_slices_keep_their_digits(oracle, size):
+    N = (4, 5, 24)
+    f = O.random_fields(N, 101, link_amp=0.2, e_amp=0.1, j_amp=0.05)
+    far = slice(10, N[2] + 2)
+    f["U"][far] = O.new_fields(N)["U"][far]
+    f["UOld"] = f["U"].copy()
+    for k in ("E", "Jp", "Jm", "JpStat", "JmStat"):
+        f[k][far] *= size
+    ref = O.copy_fields(f)
+    oracle.update(ref, N, A, DT, 2)
+    with Lattice(N, A) as lat:
+        lat.upload_fields(f)
+        lat.step(DT, 2)
+        out = lat.download_fields()
+        lat.upload("G", _random_gauge(N, 102))
+        g = O.links_as_matrices(lat.download("G"))
+        lat.coulomb_fix(0.08, 0)
+        EG = lat.download("EG")
+    want = _rotated(g[..., None, :, :], out["E"])
+    for z in range(16, N[2] + 1):  # out of reach of the strong half
+        for k in ("E", "Jp", "Jm", "JpStat", "JmStat"):
+            assert np.max(np.abs(out[k][z] - ref[k][z])) <= 1e-12 * np.max(np.abs(ref[k][z])), (k, z)
+        top = np.max(np.abs(ref["U"][z].imag))
+        assert 0 < top < size and np.max(np.abs(out["U"][z].imag - ref["U"][z].imag)) <= 1e-12 * top, z
+        assert np.max(np.abs(EG[z] - want[z])) <= 1e-12 * np.max(np.abs(want[z])), z
+
+
+def test_adjoint_of_the_smallest_weights():
+    _gradients_scale("fp64", [1e-130, 1e-145, 1e-160, 1e-250, 1e-290, 1e-306], 1e-12, 5e-324)
