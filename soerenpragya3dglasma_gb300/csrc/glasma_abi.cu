@@ -1,5 +1,6 @@
 // glasma_abi.cu -- the C ABI (include/glasma_gb300.h): handle, device memory, host copies
 // and the orchestration of the kernels for each reference entry point.
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -10,6 +11,7 @@
 #include <vector>
 
 #include "../../include/glasma_gb300.h"
+#include "extent.h"
 #include "handle.h"
 
 using glasma::cx;
@@ -509,15 +511,35 @@ static void* mapped_host(const void* p) {
   return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// Whether p is memory of the handle's own GPU: the layout kernels then read or write it in place, where other device
-// memory goes through the staging buffer and a copy (two more passes over the field).
-static bool own_device(const glasma_lattice* h, const void* p) {
+// The allocation that holds the device address p, by cuMemGetAddressRange (asked of the driver, so that the library needs no
+// libcuda to link); false when the driver does not tell.
+static bool allocation_of(const void* p, uintptr_t* base, size_t* size) {
+  static const PFN_cuMemGetAddressRange_v3020 range = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 3020, cudaEnableDefault, &found);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(fn)
+                                                                    : nullptr;
+  }();
+  CUdeviceptr b = 0;
+  if (!range || range(&b, size, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return false;
+  *base = static_cast<uintptr_t>(b);
+  return true;
+}
+// Whether `bytes` at p are memory of the handle's own GPU: the layout kernels then read or write it in place, where other
+// device memory, and a buffer that may run past its allocation, goes through the staging buffer and a copy (two more passes
+// over the field), which refuses what it cannot reach.
+static bool own_device(const glasma_lattice* h, const void* p, size_t bytes) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == h->device && reinterpret_cast<size_t>(p) % sizeof(double) == 0;
+  if (a.type != cudaMemoryTypeDevice || a.device != h->device || reinterpret_cast<uintptr_t>(p) % sizeof(double)) return false;
+  uintptr_t base;
+  size_t size;
+  return allocation_of(p, &base, &size) && glasma::extent_holds(base, size, reinterpret_cast<uintptr_t>(p), bytes);
 }
 
 static int upload_common(glasma_lattice* h, int field, const double* src, cudaMemcpyKind kind) {
@@ -536,7 +558,7 @@ static int upload_common(glasma_lattice* h, int field, const double* src, cudaMe
       return e == cudaSuccess ? GLASMA_OK : cuda_fail(e, "aos_to_soa from host");
     }
   }
-  if (kind == cudaMemcpyDeviceToDevice && own_device(h, src)) {
+  if (kind == cudaMemcpyDeviceToDevice && own_device(h, src, bytes)) {
     cudaError_t e = h->precision == GLASMA_FP64
                         ? glasma::launch_aos_to_soa<double>(src, static_cast<double*>(h->f[field]), h->g.S, P, h->stream)
                         : glasma::launch_aos_to_soa<float>(src, static_cast<float*>(h->f[field]), h->g.S, P, h->stream);
@@ -570,7 +592,7 @@ static int download_common(glasma_lattice* h, int field, double* dst, cudaMemcpy
       return GLASMA_OK;
     }
   }
-  if (kind == cudaMemcpyDeviceToDevice && own_device(h, dst)) {
+  if (kind == cudaMemcpyDeviceToDevice && own_device(h, dst, bytes)) {
     cudaError_t e = h->precision == GLASMA_FP64
                         ? glasma::launch_soa_to_aos<double>(static_cast<const double*>(h->f[field]), dst, h->g.S, P, h->stream)
                         : glasma::launch_soa_to_aos<float>(static_cast<const float*>(h->f[field]), dst, h->g.S, P, h->stream);

@@ -316,3 +316,27 @@ def test_the_thinnest_slices_keep_their_digits(oracle, size):
 
 def test_adjoint_of_the_smallest_weights():
     _gradients_scale("fp64", [1e-130, 1e-145, 1e-160, 1e-250, 1e-290, 1e-306], 1e-12, 5e-324)
+
+
+# ---- device buffers of the caller, in the middle of an allocation and up to its end
+def test_device_buffers_inside_an_allocation():
+    torch = pytest.importorskip("torch")
+    N = (32, 32, 64)
+    f = O.random_fields(N, 103)
+    with Lattice(N) as lat:
+        n = lat.field_doubles("U")
+        block = torch.zeros(n + 1024, dtype=torch.float64, device="cuda")
+        lat.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for at in (0, 512, 1024):
+            part = block[at:at + n]
+            part.copy_(torch.from_numpy(f["U"].view(np.float64).ravel()))
+            torch.cuda.synchronize()
+            lat.upload_device("U", part.data_ptr())
+            lat.synchronize()
+            block.zero_()
+            torch.cuda.synchronize()
+            lat.download_device("U", part.data_ptr())
+            assert np.array_equal(part.cpu().numpy(), f["U"].view(np.float64).ravel())
+            assert not block[:at].any() and not block[at + n:].any()
+        assert before - torch.cuda.mem_get_info()[0] < 8 << 20  # read and written in place: no staging buffer (30 MB)
