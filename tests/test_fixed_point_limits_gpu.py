@@ -340,3 +340,41 @@ def test_device_buffers_inside_an_allocation():
             assert np.array_equal(part.cpu().numpy(), f["U"].view(np.float64).ravel())
             assert not block[:at].any() and not block[at + n:].any()
         assert before - torch.cuda.mem_get_info()[0] < 8 << 20  # read and written in place: no staging buffer (30 MB)
+
+
+# ---- gradient arrays: nothing is written to them by the host before the copy that fills or refuses them
+DEVICE_GRADIENT = """
+import ctypes, sys
+import numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+from oracle import oracle as O
+from soerenpragya3dglasma_gb300 import Lattice, _lib
+N = (4, 5, 6)
+f = O.random_fields(N, 104, link_amp=0.25, e_amp=0.3, j_amp=0.05)
+with Lattice(N) as lat:
+    lat.upload_fields(f)
+    value, want = lat.adjoint(0.1, 2, 1, 5, Lattice.ENERGY, checkpoint_every=1)
+    out = torch.zeros(want["E"].size, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    num, den = (ctypes.c_double * 6)(*Lattice.ENERGY[0]), (ctypes.c_double * 6)(*Lattice.ENERGY[1])
+    v = ctypes.c_double()
+    st = lat.lib.glasma_adjoint(lat.h, 0.1, 2, 1, 1, 5, num, den, ctypes.byref(v),
+                                ctypes.cast(out.data_ptr(), _lib._D), None, None, None, None)
+    print("status", st)  # refused, or filled
+    if st == 0:
+        assert np.allclose(out.cpu().numpy(), want["E"].ravel(), rtol=1e-9, atol=1e-12)
+    again, _ = lat.adjoint(0.1, 2, 1, 5, Lattice.ENERGY, checkpoint_every=1)
+    assert abs(again - value) <= 1e-12 * abs(value)
+print("done")
+"""
+
+
+def test_a_device_gradient_array_does_not_end_the_process():
+    import os
+    import subprocess
+    import sys
+
+    pytest.importorskip("torch")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", DEVICE_GRADIENT, root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "done" in r.stdout, (r.returncode, r.stdout, r.stderr[-2000:])
