@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 inline bool make_plan(int n, Plan& p) {
   p = Plan{};
   p.n = n;
+  if (n < 2 || n >= (1 << 16)) return false;  // at most ten stages (3^10)
   int twos = 0, m = n;
   while (m % 2 == 0) m /= 2, twos++;
   auto push = [&](int r) { p.radix[p.nstages++] = r; };
@@ -299,7 +300,7 @@ inline bool make_plan(int n, Plan& p) {
   }
   while (m % 5 == 0) m /= 5, push(5);
   while (m % 3 == 0) m /= 3, push(3);
-  if (m != 1 || n < 2 || n >= (1 << 16)) return false;
+  if (m != 1) return false;
   unsigned ns = 1;
   for (int s = 0; s < p.nstages; s++) {
     p.magic[s] = ns == 1 ? 0u : (unsigned)((0x100000000ULL + ns - 1) / ns);
