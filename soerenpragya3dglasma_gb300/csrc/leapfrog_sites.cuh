@@ -317,7 +317,7 @@ __device__ __forceinline__ void efield_site(const Geometry& g, const FieldPtrs<T
 // InverseAdjointMultiplication.  The same terms as the staple form (K1), regrouped: three plaquettes
 // (three products each) and six adjoint rotations per site instead of twelve staples (two products
 // each, three shared) and three final products: ~18 instead of ~24 matrix products per site.
-// K1' (plaquette_site) runs one thread per plaquette owner y, slices -1 .. Nz-1 (the ghost slice owns
+// K1' (plaquette_site_direct, or plaquette_site_fx in FP64) runs one thread per plaquette owner y, slices -1 .. Nz-1 (the ghost slice owns
 // the plaquettes whose lower-staple terms reach slice 0): it adds the first two terms and the current
 // source to E at y and stores the rotated vectors of the last two, without their weights, in a contribution
 // buffer at y.  K2' (links_site with kGather) adds the two each link receives, from y = x-q and x-p, times
@@ -530,7 +530,7 @@ __device__ __forceinline__ void plaquette_site_direct(const Geometry& g, const F
   }
 }
 
-// plaquette_site for FP64 fields with the products on the integer pipe (fx.cuh).  Bound by FP64, the direct form
+// plaquette_site_direct for FP64 fields with the products on the integer pipe (fx.cuh).  Bound by FP64, the direct form
 // runs ~2000 FP64 operations per site; here they are ~5,000 mad.wide and ~15,000 other integer operations, with ~300
 // FP64 ones beside them (the sums into E, conversions): 128x128x512 30.7 ms in FP64, 10.9 here.  One copy of the plaquette and of the rotation in the code, so
 // that it stays inside the instruction cache; the three anti-Hermitian parts wait in shared memory for their rotations.
@@ -852,7 +852,7 @@ __device__ __forceinline__ void transport_currents(const FieldPtrs<T>& f, const 
 
 // K2's body for link mu of one site: the link to t+dt (two applications of one exp), UOld, J transport (mu = 2).
 // kGather (the plaquette method): first E_mu += the two contributions link mu receives from the plaquette owners
-// x-nu (see plaquette_site), stored with its ghost copy.
+// x-nu (see plaquette_site_direct), stored with its ghost copy.
 template <typename T, typename I, int R = 3, bool kGather = false>
 __device__ __forceinline__ void link_site(const Geometry& g, const FieldPtrs<T>& f, const LParams<T>& p, I idx,
                                            const int mu, const T* __restrict__ C = nullptr) {

@@ -1,7 +1,7 @@
 // march.cuh -- the whole leapfrog step in one launch by the plaquette method, each block marching
 // along z through a column of the lattice.
 //
-// The plaquette method (leapfrog_sites.cuh: plaquette_site, links_site<kGather>) computes each
+// The plaquette method (leapfrog_sites.cuh: plaquette_site_direct, links_site<kGather>) computes each
 // plaquette once, at its owner site y, and hands the two rotated force terms that belong to other
 // links (U_p(y+q), U_q(y+p)) to the link kernel through a contribution buffer in HBM: 48 reals per
 // site written and read back, and E, U and the currents read by both kernels.  Here one block owns a
@@ -67,7 +67,7 @@ __device__ __forceinline__ void march_get(const T* csm, int slot, int c, Alg<T>&
   for (int a = 0; a < 8; a++) v.a[a] = csm[(slot * 8 + a) * kMarchThreads + c];
 }
 
-// UpdateJStat at slice site sz from the state of t (as plaquette_site forms it): uzm = U_z one slice down.
+// UpdateJStat at slice site sz from the state of t (as plaquette_site_direct forms it): uzm = U_z one slice down.
 template <typename T, typename I>
 __device__ __forceinline__ void march_jstat(const FieldPtrs<T>& in, I S, I plane, I sz, const Mat<T>& uzm, T cj,
                                             Alg<T>& stp, Alg<T>& stm) {
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kMarchThreads, MarchOccupancy<T>::kMinBlocks)
       }
 #pragma unroll 1
       for (int mu = 0; mu < 3; mu++) {
-        // E_mu + the direct terms (as plaquette_site sums them) + the two rotated terms (as links_site
+        // E_mu + the direct terms (as plaquette_site_direct sums them) + the two rotated terms (as links_site
         // adds them)
         Alg<T> e, a1, a2, alA, alB;
         load_alg(in.E, S, mu * 8, s, e);
