@@ -370,10 +370,14 @@ def run_ours(args):
         key = "%s_%s" % (name, prec)
         tr = traffic.get(key)
         # what limits the kernel, from the ncu capture of the same kernel: the FP64 staple kernels keep
-        # GB300's FP64 pipe >90 % busy (hence their small HBM fraction), the fixed-point ones are bound by
-        # latency and the integer multiplier, the FP32 ones by HBM traffic and issue
+        # GB300's FP64 pipe >90 % busy (hence their small HBM fraction), the FP32 ones move half and more
+        # of what HBM can, and the fixed-point ones (integer multiplier half busy) are bound by neither
         pa = traffic.get("pipe_active", {}).get(key)
-        bound = "fp64_pipe" if pa and pa.get("pipe") == "fp64" and pa.get("frac", 0) > 0.8 else "hbm"
+        moved = (tr or alg) / (ms * 1e-3) / 1e9
+        if pa and pa.get("pipe") == "fp64" and pa.get("frac", 0) > 0.8:
+            bound = "fp64_pipe"
+        else:
+            bound = "hbm" if moved > peak / 3 else "latency"
         out = {"bound": bound, "kernel": name, "achieved": ach, "peak": peak, "unit": "GB/s",
                "frac": ach / peak, "peak_kind": peak_kind, "traffic": tr,
                "algorithmic_bytes_per_launch": alg, "launch_ms": ms,

@@ -86,8 +86,12 @@ enum glasma_field {
                                             until the maximum deviation is <= 1e-5 or stops falling, then
                                             G is widened, projected onto SU(3) in FP64, and the FP64
                                             sweeps finish to the stopping rule; log rows and the count
-                                            cover both phases.  The FP32 update's unitarity guard is
-                                            1e-5.  GLASMA_ERR_UNSUPPORTED on FP32 handles */
+                                            cover both phases.  Rows of the FP32 phase leave the ghost
+                                            z links below slice 0 out of the two functional columns: the
+                                            functional per volume is (a_scale/a_z)^2 3/Nz below the FP64
+                                            rows', which count their trace of 3 as the reference does.
+                                            The FP32 update's unitarity guard is 1e-5.
+                                            GLASMA_ERR_UNSUPPORTED on FP32 handles */
 
 /* Create a lattice (replaces Lattice::Init, S/LATTICE/SUNcVariables.cpp:71-90, and the
  * container constructors, S/LATTICE/GaugeLinks.cpp:110-127): links set to the identity,

@@ -19,7 +19,7 @@
 //   y = InvAdj(V, e)   -> l_V += e x Adj(V, l_y),  l_e += Adj(V, l_y)
 //   X = exp(i c t.e)   -> l_e += c sum_n (c e x)^n l_X / (n + 1)!, or the Cayley-Hamilton form's derivative for |c e| >= 1
 // FP64 does this in fixed point on the integer pipe (fx.cuh), since one FP64 instruction costs GB300 as much as 60 FP32 ones.
-// 32x32x64, 20 steps, FP64: 47.1 ms with matrix cotangents in FP64, 40.9 with algebra vectors, 21.4 in fixed point.
+// 32x32x64, 20 steps, FP64: 47.1 ms with matrix cotangents in FP64, 40.9 with algebra vectors, 20.9 in fixed point.
 // Ghost slices are copies of the boundary slices, so cotangents that land on a ghost are added to
 // the slice it copies.
 #include <cuda_runtime.h>

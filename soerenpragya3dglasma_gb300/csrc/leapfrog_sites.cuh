@@ -100,8 +100,8 @@ struct LinkStep<double> {
 // Blocks per SM the register allocation must leave room for (the register cap is 64K / (128 * n)),
 // chosen by measurement on GB300; overridable at build time for tuning sweeps.
 // (GB300 sweep, 128x128x512: FP32 K1 fastest at 5 blocks/SM, K2 at 8; the staple kernels in FP64 are FP64-ALU bound.
-// The fixed-point kernels: force 10.7 ms at 3 blocks/SM, 12.3 at 2, 11.9 at 4; links 11.4 ms at 2 and at 3, 14 at 4, and
-// on 32x32x64 0.106 ms at 2, 0.130 at 3.)
+// The fixed-point kernels: force 10.9 ms at 3 blocks/SM, 12.4 at 2, 12.6 at 4; links 8.9 ms at 2, 8.8 at 3 and at 4, and
+// on 32x32x64 0.097 ms at 2, 0.115 at 3, 0.086 at 4.)
 #ifndef GLASMA_FP64_MIN_BLOCKS
 #define GLASMA_FP64_MIN_BLOCKS 2
 #endif
@@ -317,8 +317,8 @@ __device__ __forceinline__ void efield_site(const Geometry& g, const FieldPtrs<T
 // InverseAdjointMultiplication.  The same terms as the staple form (K1), regrouped: three plaquettes
 // (three products each) and six adjoint rotations per site instead of twelve staples (two products
 // each, three shared) and three final products: ~18 instead of ~24 matrix products per site.
-// K1' (plaquette_site_direct, or plaquette_site_fx in FP64) runs one thread per plaquette owner y, slices -1 .. Nz-1 (the ghost slice owns
-// the plaquettes whose lower-staple terms reach slice 0): it adds the first two terms and the current
+// K1' (plaquette_site_direct, or plaquette_site_fx in FP64) runs one thread per plaquette owner y, slices -1 .. Nz-1
+// (the ghost slice owns the plaquettes whose lower-staple terms reach slice 0): it adds the first two terms and the current
 // source to E at y and stores the rotated vectors of the last two, without their weights, in a contribution
 // buffer at y.  K2' (links_site with kGather) adds the two each link receives, from y = x-q and x-p, times
 // their weights (LParams wa, wb: an fma where a weighted contribution would take an add) to E before it
@@ -532,8 +532,9 @@ __device__ __forceinline__ void plaquette_site_direct(const Geometry& g, const F
 
 // plaquette_site_direct for FP64 fields with the products on the integer pipe (fx.cuh).  Bound by FP64, the direct form
 // runs ~2000 FP64 operations per site; here they are ~5,000 mad.wide and ~15,000 other integer operations, with ~300
-// FP64 ones beside them (the sums into E, conversions): 128x128x512 30.7 ms in FP64, 10.9 here.  One copy of the plaquette and of the rotation in the code, so
-// that it stays inside the instruction cache; the three anti-Hermitian parts wait in shared memory for their rotations.
+// FP64 ones beside them (the sums into E, conversions): 128x128x512 30.7 ms in FP64, 10.9 here.  One copy of the plaquette
+// and of the rotation in the code, so that it stays inside the instruction cache; the three anti-Hermitian parts wait in
+// shared memory for their rotations.
 // kRoles = 1: a thread does its site's three plaquettes and four rotation pairs in turn.  kRoles = 4: a block of four
 // warps does 32 sites, warp r plaquette r, rotation r and the sum into E_r (warp 3 the currents' rotation and JStat):
 // a third of the serial chain and four times the blocks, for lattices that do not fill the GPU (launch_plaquette_rows).
@@ -888,7 +889,7 @@ __device__ __forceinline__ void link_site(const Geometry& g, const FieldPtrs<T>&
   if constexpr (std::is_same<T, double>::value) {
     // One copy of the product and of the current transport in the code, run once or twice per link: written out
     // (three products, two exponentials) the fixed-point body overflowed the instruction cache (5.6 fetch stalls
-    // per issue, 14.3 ms at 128x128x512; 10.6 like this, 21.9 in FP64).
+    // per issue, 14.3 ms at 128x128x512 where the other form took 10.6; 8.9 now, 21.9 in FP64).
     const bool doubled = p.do_second && !p.save_uold && !(mu == 2 && p.do_j);
     LinkStep<double> X;
     X.set(doubled ? 2.0 * pick3(p.cU, mu) : pick3(p.cU, mu), e);
