@@ -11,8 +11,8 @@
 //             time-reversed integration (the step is an exact composition of shears: the forward
 //             kernels run with -dt, the links are rotated back by X^dagger), or reload the checkpoint
 //             at t; then pull the cotangents back through the step's sub-steps in reverse order.
-// Cotangent convention: links are in SU(3), so a link's cotangent is the algebra vector l with dL = l.d for U -> exp(i t.d) U
-// (eight numbers; what a matrix cotangent has normal to the group no E or current gradient sees).  With c = a x b for
+// Cotangent convention: the steps multiply links by elements of SU(3) from the left, so a link's cotangent is the algebra vector l
+// with dL = l.d for U -> exp(i t.d) U (eight numbers; no E or current gradient sees what else a matrix cotangent has).  With c = a x b for
 // c^k = f^klm a_l b_m:
 //   W = A B            -> l_A += l_W,  l_B += InvAdj(A, l_W)
 //   y = Adj(V, e)      -> l_V += y x l_y,  l_e += InvAdj(V, l_y)

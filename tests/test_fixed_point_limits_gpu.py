@@ -410,3 +410,50 @@ def test_a_slice_with_infinities_stays_one(bad):
         profile = lat.gauss(profile=True)[2]
     assert np.array_equal(np.isfinite(profile), np.arange(N[2]) != 2)
     assert np.isnan(profile[2]) if np.isnan(bad) else profile[2] == np.inf
+
+
+# ---- adjoint on links that are not unitary: a link's variations stay those of the group, whatever the link
+@pytest.mark.parametrize("factor", [1.0, 1 + 1e-12, 1 + 1e-6, 1.01, 0.8])
+@pytest.mark.parametrize("key", ["E", "Jp"])
+def test_adjoint_of_links_off_the_group(factor, key):
+    """A fifth of the links scaled: the gradient along a random direction against fourth-order central differences.
+    eps = 1e-3 of fields of order one: truncation eps^4 = 1e-12 and rounding 1e-15 / eps = 1e-12 of the objective, which
+    is up to a thousand times the derivative: 1e-8 with a margin of ten."""
+    N, steps, eps = (4, 5, 10), 3, 1e-3
+    rng = np.random.default_rng(106)
+    f = O.random_fields(N, 107, link_amp=0.3, e_amp=0.2, j_amp=0.1)
+    f["U"][rng.random(f["U"].shape[:3]) < 0.2] *= factor
+    O.sync_ghosts(f["U"])
+    d = _synced(rng.standard_normal(f[key].shape))
+
+    def value(x):
+        with Lattice(N, A) as lat:
+            lat.upload_fields(dict(f, **{key: x}))
+            lat.step(DT, steps, save_uold=False)
+            return lat.objective(2, 8, Lattice.ENERGY)
+
+    with Lattice(N, A) as lat:
+        lat.upload_fields(f)
+        _, g = lat.adjoint(DT, steps, 2, 8, Lattice.ENERGY, checkpoint_every=1)
+    v = [value(f[key] + s * eps * d) for s in (2, 1, -1, -2)]
+    fd = (8 * (v[1] - v[2]) - (v[0] - v[3])) / (12 * eps)
+    assert abs(fd - float(np.sum(g[key][1:-1] * d[1:-1]))) <= 1e-8 * abs(fd)
+
+
+def test_fp32_adjoint_of_links_off_the_group():
+    """The same links on an FP32 handle: its gradient against the FP64 one of the numbers it holds.  FP32 rounding on hot fields
+    is 5e-6 of the gradient after forty steps; three steps stay below 1e-5."""
+    N, steps = (4, 5, 10), 3
+    rng = np.random.default_rng(108)
+    f = O.random_fields(N, 109, link_amp=0.3, e_amp=0.2, j_amp=0.1)
+    f["U"][rng.random(f["U"].shape[:3]) < 0.2] *= 0.9
+    O.sync_ghosts(f["U"])
+    with Lattice(N, A, precision="fp32") as lat:
+        lat.upload_fields(f)
+        held = lat.download_fields()
+        _, g = lat.adjoint(DT, steps, 2, 8, Lattice.ENERGY, checkpoint_every=1)
+    with Lattice(N, A) as lat:
+        lat.upload_fields(held)
+        _, want = lat.adjoint(DT, steps, 2, 8, Lattice.ENERGY, checkpoint_every=1)
+    for k in g:
+        assert np.max(np.abs(g[k] - want[k])) <= 1e-5 * np.max(np.abs(want[k])), k
