@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from soerenpragya3dglasma_gb300 import Lattice, build
+from soerenpragya3dglasma_gb300 import GlasmaError, Lattice, build
 
 pytestmark = pytest.mark.gpu
 
@@ -457,3 +457,32 @@ def test_fp32_adjoint_of_links_off_the_group():
         _, want = lat.adjoint(DT, steps, 2, 8, Lattice.ENERGY, checkpoint_every=1)
     for k in g:
         assert np.max(np.abs(g[k] - want[k])) <= 1e-5 * np.max(np.abs(want[k])), k
+
+
+@pytest.mark.parametrize("precision,mixed", [("fp64", False), ("fp64", True), ("fp32", False)])
+def test_gauge_fields_where_the_guard_ends_the_sweeps(precision, mixed):
+    """A NaN link trips the guard: E is left as EG, and UG, whose memory the sweeps use, holds links again: G U G^dagger of the
+    transformation the call ends with (mixed: the FP32 sweeps' copy is dropped, so the links themselves)."""
+    N = (4, 5, 6)
+    f = O.random_fields(N, 110, link_amp=0.1, e_amp=0.1)
+    f["U"][2, 1, 2, 0, 0, 0] = np.nan
+    with Lattice(N, precision=precision) as lat:
+        lat.upload("U", f["U"])
+        lat.upload("E", f["E"])
+        held = {k: lat.download(k) for k in ("U", "E")}
+        with pytest.raises(GlasmaError):
+            lat.coulomb_fix(0.08, 5, mixed=mixed)
+        got = {k: lat.download(k) for k in ("G", "UG", "EG")}
+    assert np.array_equal(got["EG"][1:-1], held["E"][1:-1])
+    assert np.array_equal(got["UG"][[0, -1]], O.identity_links(N)[[0, -1]])
+    g, u = O.links_as_matrices(got["G"]), O.links_as_matrices(held["U"])
+    forward = [np.roll(g, -1, axis=2), np.roll(g, -1, axis=1), np.roll(g, -1, axis=0)]
+    for mu in range(3):
+        want = g @ u[..., mu, :, :] @ np.swapaxes(forward[mu].conj(), -1, -2)
+        if mixed:
+            want = u[..., mu, :, :]
+        have = O.links_as_matrices(got["UG"])[..., mu, :, :]
+        inside = np.s_[1:-2]  # the top slice's z links look at G's ghost
+        ok = np.isfinite(want[inside])
+        assert np.array_equal(np.isfinite(have[inside]), ok), mu
+        assert np.max(np.abs(have - want)[inside][ok], initial=0) <= (1e-13 if precision == "fp64" else 2e-7), mu
